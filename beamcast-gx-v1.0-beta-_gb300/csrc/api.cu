@@ -150,7 +150,7 @@ void bc_destroy(bc_context* ctx) {
   destroy_photon_state(ctx);
   for (DevBuf* b : {&ctx->d_nodes, &ctx->d_tri, &ctx->d_slot64, &ctx->d_snorm, &ctx->d_slot_prim, &ctx->d_mats,
                     &ctx->d_lights, &ctx->d_lpdf, &ctx->d_bin, &ctx->d_rays, &ctx->d_t, &ctx->d_prim, &ctx->d_occ,
-                    &ctx->d_kids8, &ctx->d_geom, &ctx->d_build, &ctx->d_build_out, &ctx->d_order[0],
+                    &ctx->d_kids8, &ctx->d_geom, &ctx->d_build, &ctx->d_order[0],
                     &ctx->d_order[1], &ctx->d_order[2], &ctx->d_rec[0], &ctx->d_rec[1], &ctx->d_rec[2],
                     &ctx->d_rec_any})
     b->release();

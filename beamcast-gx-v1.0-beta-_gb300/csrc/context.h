@@ -78,7 +78,7 @@ struct bc_context {
   bool is_set = false;                    // resident scenes came from bc_scene_set_upload
   bcgx::GeomInfo geom;                    // geometry-only updates (refit.cu)
   bcgx::DevBuf d_kids8, d_geom;           // Node8 -> binary child map; fp64 geometry staging
-  bcgx::DevBuf d_build, d_build_out;      // device SAH build (build.cu)
+  bcgx::DevBuf d_build;                   // device SAH build (build.cu)
   bcgx::DevBuf d_post_stack, d_post_hist; // bc_post_stack buffers and temporal history (post.cu)
   struct PostHistory* post_hist = nullptr;
   std::vector<int8_t> mat_kind;           // host copy of the resident materials' kinds

@@ -69,3 +69,23 @@ def test_device_built_scene_renders_and_casts(gpu_ctx, orc):
     t_ref, p_ref, _ = orc.OracleScene.from_spec(spec).hit_f32(rays)
     assert np.array_equal(p, p_ref)
     assert np.array_equal(t[p >= 0], t_ref[p >= 0].astype(np.float32))
+
+
+# Edges of the two phases (32 elements: one warp finishes the range; 256: one
+# chunk of the level-wise kernels) and of the bin and leaf limits.
+@pytest.mark.parametrize("n", [31, 32, 33, 64, 65, 255, 256, 257, 511, 513, 1025, 8191])
+@pytest.mark.parametrize("bins,leaf", [(32, 1), (4, 4), (31, 16)])
+def test_phase_and_chunk_edges(gpu_ctx, n, bins, leaf):
+    _same_tree(scenes.random_triangles(n, seed=0xBEAC0300 + n), gpu_ctx, bins, leaf)
+
+
+def test_equal_centroids_make_one_large_leaf_or_chains(gpu_ctx):
+    """Ranges without extent end as leaves in the level-wise phase too; uneven
+    splits give tasks of very different sizes in one level."""
+    base = scenes.random_triangle_verts(1, seed=3)
+    one = np.repeat(base, 700, axis=0)              # all centroids equal: 700 elements in one leaf
+    tail = np.concatenate([base * (1.0 + 10.0 ** k) for k in range(0, 12)])
+    spec = scenes.SceneSpec(name="chain", bvh_mode="SAH", bvh_bins=32, bvh_leaf=4)
+    m = spec.material(scenes.Material(0, (0.5, 0.5, 0.5)))
+    spec.triangles(np.concatenate([one, tail, np.repeat(tail, 40, axis=0)]), m)
+    _same_tree(spec, gpu_ctx)
