@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(1024) k_photon_scan(const int* __restrict__ co
 
 // Sorts the photons by (cell key, append index) (bitonic sort of the padded
 // power of two), lists the distinct keys with their runs, gathers the photons
-// into sorted order, fills the lookup table and writes the dense table's box
-// (the photons' cells and two more each side; no dense table when it would
-// hold more than max_cells cells). One block.
+// into sorted order, fills the lookup table and writes the neighbour lists' box
+// (the photons' cells and two more each side; no lists when it would hold more
+// than max_cells cells). One block.
 __global__ void __launch_bounds__(1024) k_photon_grid(const int* __restrict__ header, int p2max,
                                                       const unsigned long long* __restrict__ key,
                                                       const float4* __restrict__ pos_u, const float4* __restrict__ nrm_u,
@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(1024) k_photon_grid(const int* __restrict__ he
   __syncthreads();
   if (t == 0) {
     bool ok = n > 0 && max_cells > 0;
+    grid->used = 0;
     double cells = 1.0;
     for (int a = 0; a < 3 && ok; a++) {
       const long long d = cmax[a] - cmin[a] + 5;
@@ -324,16 +325,56 @@ __global__ void __launch_bounds__(1024) k_photon_grid(const int* __restrict__ he
 
 namespace bcgx {
 
-// The dense table: the run of every cell of the box, looked up in the hash
-// table exactly as a gather would look the cell up.
-__global__ void k_photon_dense(PhotonView pm, const PhotonGrid* __restrict__ grid, int* __restrict__ dense) {
+// The neighbour lists, a thread per cell of the box: the photons of the 27
+// cells around it, each cell's run looked up in the hash table exactly as a
+// gather would look it up, in the gather's order. `runs` holds the lookups (run
+// index or -1, written by k_photon_runs). A cell whose list would not fit in
+// the remaining entries gets none, and gathers there use the hash. Every photon
+// is in the lists of at most 27 cells (more only where cell keys collide).
+__global__ void k_photon_runs(PhotonView pm, const PhotonGrid* __restrict__ grid, int* __restrict__ runs) {
   const int gx = grid->dim[0];
   if (gx == 0) return;
   const int gy = grid->dim[1], gz = grid->dim[2];
   const long long total = (long long)gx * gy * gz;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long x = i % gx, y = (i / gx) % gy, z = i / ((long long)gx * gy);
-    dense[i] = photon_cell_lookup(pm, photon_cell_key(grid->g0[0] + x, grid->g0[1] + y, grid->g0[2] + z));
+    runs[i] = photon_cell_lookup(pm, photon_cell_key(grid->g0[0] + x, grid->g0[1] + y, grid->g0[2] + z));
+  }
+}
+
+__global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, const int* __restrict__ runs,
+                               int2* __restrict__ list, float4* __restrict__ lpos, int cap) {
+  const int gx = grid->dim[0];
+  if (gx == 0) return;
+  const int gy = grid->dim[1], gz = grid->dim[2];
+  const long long total = (long long)gx * gy * gz;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int x = (int)(i % gx), y = (int)((i / gx) % gy), z = (int)(i / ((long long)gx * gy));
+    if (x < 1 || y < 1 || z < 1 || x > gx - 2 || y > gy - 2 || z > gz - 2) {
+      list[i] = make_int2(-1, 0);  // a gather there is zero without a lookup
+      continue;
+    }
+    int n = 0;
+    for (int c = 0; c < 27; c++) {
+      const int u = runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
+      if (u >= 0) n += pm.span[u].y;
+    }
+    int at = 0;
+    if (n > 0) {
+      at = atomicAdd(&grid->used, n);
+      if (at < 0 || at > cap - n) at = -1;
+    }
+    list[i] = make_int2(at, n);
+    if (at < 0) continue;
+    for (int c = 0; c < 27 && n > 0; c++) {
+      const int u = runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
+      if (u < 0) continue;
+      const int2 sp = pm.span[u];
+      for (int k = sp.x; k < sp.x + sp.y; k++) {
+        const float4 P = pm.pos[k];
+        lpos[at++] = make_float4(P.x, P.y, P.z, __int_as_float(k));
+      }
+    }
   }
 }
 
@@ -410,8 +451,8 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   if (radius <= 1e-4) radius = 0.25;
   p.attempts = budget * 6;
   p.np = budget + p.max_bounces;  // the last emission may overshoot the budget by max_bounces - 1
-  // dense table: photons lie in the scene bounds (a cell of slack per side for
-  // fp32 hit points); larger than 2^22 cells, the hash serves alone
+  // neighbour lists: photons lie in the scene bounds (a cell of slack per side
+  // for fp32 hit points); with more than 2^22 cells the hash serves alone
   double cells = 1.0;
   for (int a = 0; a < 3; a++)
     cells *= std::floor(sr.hi[a] / radius) - std::floor(sr.lo[a] / radius) + 7.0;
@@ -419,11 +460,13 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   int p2max = 2;
   while (p2max < p.np) p2max <<= 1;
   const int tsize = 2 * p2max;
+  const int list_cap = 32 * p.np;
   const size_t a = (size_t)p.attempts, np = (size_t)p.np, p2 = (size_t)p2max;
   const size_t bytes = 4 * 256 + ((a * 4 + 255) / 256) * 256 * 2 + ((np * 16 + 255) / 256) * 256 * 6 +
                        ((np * 8 + 255) / 256) * 256 * 2 + ((p2 * 8 + 255) / 256) * 256 +
                        ((p2 * 4 + 255) / 256) * 256 + ((np * 8 + 255) / 256) * 256 + ((tsize * 4 + 255) / 256) * 256 +
-                       256 + (((size_t)max_cells * 4 + 255) / 256) * 256;
+                       256 + (((size_t)max_cells * 4 + 255) / 256) * 256 + (((size_t)max_cells * 8 + 255) / 256) * 256 +
+                       (max_cells ? ((size_t)list_cap * 16 + 255) / 256 * 256 : 0);
   cudaError_t e = cudaMalloc(&p.mem, bytes);
   if (e) {
     p.mem = nullptr;
@@ -447,7 +490,9 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   float4* flux = take<float4>(c, np);
   int* table = take<int>(c, tsize);
   PhotonGrid* grid = take<PhotonGrid>(c, 1);
-  int* dense = max_cells ? take<int>(c, (size_t)max_cells) : nullptr;
+  int* runs = max_cells ? take<int>(c, (size_t)max_cells) : nullptr;
+  int2* list = max_cells ? take<int2>(c, (size_t)max_cells) : nullptr;
+  float4* lpos = max_cells ? take<float4>(c, (size_t)list_cap) : nullptr;
   p.pos_u = pos_u;
   p.nrm_u = nrm_u;
   p.flux_u = flux_u;
@@ -489,12 +534,16 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
     e = cudaGetLastError();
   }
   PhotonView hv{};
+  hv.pos = pos;
   hv.ukey = ukey;
+  hv.span = span;
   hv.table = table;
   hv.mask = tsize - 1;
-  if (!e && dense) {
+  if (!e && list) {
     const int blocks = (int)std::min<long long>(1024, (max_cells + 255) / 256);
-    k_photon_dense<<<blocks, 256, 0, st>>>(hv, grid, dense);
+    k_photon_runs<<<blocks, 256, 0, st>>>(hv, grid, runs);
+    k_photon_lists<<<(int)std::min<long long>(4096, (max_cells + 63) / 64), 64, 0, st>>>(hv, grid, runs, list, lpos,
+                                                                                        list_cap);
     e = cudaGetLastError();
   }
   if (e) {
@@ -511,8 +560,9 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   p.view.cell = (float)radius;
   p.view.r2 = (float)(radius * radius);
   p.view.pir2 = (float)(M_PI * radius * radius);
-  p.view.grid = dense ? grid : nullptr;
-  p.view.dense = dense;
+  p.view.grid = list ? grid : nullptr;
+  p.view.list = list;
+  p.view.lpos = lpos;
   return BC_OK;
 }
 
@@ -572,7 +622,7 @@ bc_status photon_map_for(bc_context* ctx, int scene, const bc_settings& s, uint6
   *view = p->view;  // an empty map has a null table
   if (!ctx->photon_grid) {
     view->grid = nullptr;
-    view->dense = nullptr;
+    view->list = nullptr;
   }
   return BC_OK;
 }
