@@ -48,6 +48,11 @@ double photon_radius(double diag, int level) {  // renderer.go:1163-1182
   }
 }
 
+// A photon is in the lists of 27 cells, more only where cell keys collide.
+int photon_list_entries(const bc_settings& s) {
+  return 32 * (photon_budget(s.photon_mapping) + std::max(2, s.bounces));
+}
+
 struct PhotonTraceArgs {
   SceneView sv;
   const MatGPU* __restrict__ mats;
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(128) k_photon_trace(PhotonTraceArgs a, unsigne
       const int li = draw_index(rng, a.n_lights);  // rng.Intn
       const LightGPU Lg = a.lights[a.light_off + li];
       const float3 surf = rand_unit_vector(rng);
-      float3 o = f3(Lg.cx, Lg.cy, Lg.cz) + surf * (Lg.r + 2e-4f);
+      float3 o = fma3(surf, Lg.r + 2e-4f, f3(Lg.cx, Lg.cy, Lg.cz));
       float3 d = rand_cos_hemisphere(surf, rng);
       float3 tp = f3(Lg.er, Lg.eg, Lg.eb) * ((4.0f * kPhotonPi * Lg.r * Lg.r) / (float)a.budget);
       FastWalker<STACK, kLeafVote> w;
@@ -117,25 +122,27 @@ __global__ void __launch_bounds__(128) k_photon_trace(PhotonTraceArgs a, unsigne
           }
           out++;
           d = rand_cos_hemisphere(S.N, rng);
-          o = S.p + S.N * 2e-4f;
+          o = fma3(S.N, 2e-4f, S.p);
         } else if (kind == BC_MAT_METAL) {
           const float rough = fminf(fmaxf(M.rough, 0.0f), 1.0f);
-          const float3 nd = unit3(reflect3(unit3(d), S.N) + rand_in_unit_sphere(rng) * rough);
+          const float3 refl = reflect3(unit_of(d, dot3_xyz(d, d)), S.N);
+          const float3 nd = unit3(fma3(rand_in_unit_sphere(rng), rough, refl));
           if (dot3(nd, S.N) <= 0.0f) break;
           tp = had(tp, col);
-          o = S.p + S.N * 2e-4f;
+          o = fma3(S.N, 2e-4f, S.p);
           d = nd;
         } else {  // glass and any other kind (renderer.go:1695-1710)
           float eta = M.ior;
           if (eta <= 1.0f) eta = 1.5f;
           const float ratio = S.front ? 1.0f / eta : eta;
-          const float3 un = unit3(d);
-          const float cosT = fminf(dot3(un * -1.0f, S.N), 1.0f);
-          const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
-          const float3 nd = (ratio * sinT > 1.0f || schlick(cosT, ratio) > rng.uniform()) ? reflect3(un, S.N)
-                                                                                          : refract3(un, S.N, ratio);
+          const float3 un = unit_of(d, dot3_xyz(d, d));
+          const float udn = glass_dot(un, S.N);
+          const float cosT = fminf(-udn, 1.0f);
+          const float sinT = sqrtf(fmaxf(0.0f, __fmaf_rn(-cosT, cosT, 1.0f)));
+          const float3 nd = (ratio * sinT > 1.0f || schlick(cosT, ratio) > rng.uniform()) ? glass_reflect(un, S.N, udn)
+                                                                                          : glass_refract(un, S.N, udn, ratio);
           tp = had(tp, col);
-          o = S.p + nd * 2e-4f;
+          o = fma3(nd, 2e-4f, S.p);
           d = nd;
         }
         if (b >= 2) {  // renderer.go:1711-1717
@@ -460,7 +467,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   int p2max = 2;
   while (p2max < p.np) p2max <<= 1;
   const int tsize = 2 * p2max;
-  const int list_cap = 32 * p.np;
+  const int list_cap = photon_list_entries(s);
   const size_t a = (size_t)p.attempts, np = (size_t)p.np, p2 = (size_t)p2max;
   const size_t bytes = 4 * 256 + ((a * 4 + 255) / 256) * 256 * 2 + ((np * 16 + 255) / 256) * 256 * 6 +
                        ((np * 8 + 255) / 256) * 256 * 2 + ((p2 * 8 + 255) / 256) * 256 +

@@ -67,13 +67,13 @@ __device__ __forceinline__ int photon_cell_lookup(const PhotonView& pm, unsigned
 // the radius of p and faces n; true once kGatherMax photons are counted.
 __device__ __forceinline__ bool gather_photon(const PhotonView& pm, float4 P, int i, float3 p, float3 n, float3& sum,
                                               int& count) {
-  const float3 d = f3(P.x - p.x, P.y - p.y, P.z - p.z);
+  const float3 d = f3(P.x, P.y, P.z) - p;
   if (dot3(d, d) > pm.r2) return false;
   const float4 N = __ldg(pm.nrm + i);
-  const float nd = N.x * n.x + N.y * n.y + N.z * n.z;
+  const float nd = dot3(f3(N.x, N.y, N.z), n);
   if (nd <= 0.05f) return false;
   const float4 F = __ldg(pm.flux + i);
-  sum = sum + f3(F.x, F.y, F.z) * nd;
+  sum = fma3(f3(F.x, F.y, F.z), nd, sum);
   return ++count >= kGatherMax;
 }
 
@@ -81,29 +81,30 @@ __device__ __forceinline__ bool gather_photon(const PhotonView& pm, float4 P, in
 // (dz, dy, dx) order, each cell's photons in append order; a key shared by two
 // of the cells is visited twice, as the reference's map lookups do.
 // A cell's neighbour list holds exactly those photons in exactly that order, so
-// a gather is one lookup and one contiguous run, and only the candidates within
-// the radius read their normal and flux (about a third). The gather is bound by
-// dependent loads of divergent lanes: with 27 cell lookups, a span per non-empty
-// cell and two loads per candidate it took 10.6 of a 12.4 ms photon frame
-// (1280 x 720, 16 spp, 8 bounces, 8,192 photons). A point more than one cell
-// outside the photons' cells has no photon within the radius (cells are one
-// radius wide), so its gather is zero, as the loop would find.
-__device__ __forceinline__ float3 photon_gather(const PhotonView& pm, float3 p, float3 n) {
-  if (!pm.table) return f3(0.0f, 0.0f, 0.0f);
-  const long long cx = (long long)floorf(p.x / pm.cell);
-  const long long cy = (long long)floorf(p.y / pm.cell);
-  const long long cz = (long long)floorf(p.z / pm.cell);
-  float3 sum = f3(0.0f, 0.0f, 0.0f);
-  int count = 0;
+// a gather is one lookup (gather_run) and one contiguous run (gather_sum), and
+// only the candidates within the radius read their normal and flux (about a
+// third).
+
+// The run of p's cell: (first entry, entries), entries 0 where the gather is
+// zero; first < 0: no list, the hash serves. A point more than one cell outside
+// the photons' cells has no photon within the radius (cells are one radius
+// wide), so its gather is zero, as the loop would find.
+__device__ __forceinline__ int2 gather_run(const PhotonView& pm, float3 p) {
+  if (!pm.table) return make_int2(0, 0);
   const PhotonGrid* G = pm.list ? pm.grid : nullptr;
   const int gx = G ? __ldg(&G->dim[0]) : 0;
-  int2 run = make_int2(-1, 0);
-  if (gx > 0) {
-    const int gy = __ldg(&G->dim[1]), gz = __ldg(&G->dim[2]);
-    const long long lx = cx - __ldg(&G->g0[0]), ly = cy - __ldg(&G->g0[1]), lz = cz - __ldg(&G->g0[2]);
-    if (lx < 1 || ly < 1 || lz < 1 || lx > gx - 2 || ly > gy - 2 || lz > gz - 2) return f3(0.0f, 0.0f, 0.0f);
-    run = __ldg(pm.list + (lz * gy + ly) * (long long)gx + lx);
-  }
+  if (gx == 0) return make_int2(-1, 0);
+  const int gy = __ldg(&G->dim[1]), gz = __ldg(&G->dim[2]);
+  const long long lx = (long long)floorf(p.x / pm.cell) - __ldg(&G->g0[0]);
+  const long long ly = (long long)floorf(p.y / pm.cell) - __ldg(&G->g0[1]);
+  const long long lz = (long long)floorf(p.z / pm.cell) - __ldg(&G->g0[2]);
+  if (lx < 1 || ly < 1 || lz < 1 || lx > gx - 2 || ly > gy - 2 || lz > gz - 2) return make_int2(0, 0);
+  return __ldg(pm.list + (lz * gy + ly) * (long long)gx + lx);
+}
+
+__device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, float3 p, float3 n) {
+  float3 sum = f3(0.0f, 0.0f, 0.0f);
+  int count = 0;
   if (run.x >= 0) {
     const float4* e = pm.lpos + run.x;
     for (int i = 0; i < run.y; i += 4) {  // four positions in flight; the last group reads the last entry again
@@ -117,6 +118,9 @@ __device__ __forceinline__ float3 photon_gather(const PhotonView& pm, float3 p, 
       if (full) break;
     }
   } else {
+    const long long cx = (long long)floorf(p.x / pm.cell);
+    const long long cy = (long long)floorf(p.y / pm.cell);
+    const long long cz = (long long)floorf(p.z / pm.cell);
     bool full = false;
     for (int dz = -1; dz <= 1 && !full; dz++)
       for (int dy = -1; dy <= 1 && !full; dy++)
@@ -132,6 +136,12 @@ __device__ __forceinline__ float3 photon_gather(const PhotonView& pm, float3 p, 
   return sum * (1.0f / (pm.pir2 * (float)count));
 }
 
+__device__ __forceinline__ float3 photon_gather(const PhotonView& pm, float3 p, float3 n) {
+  const int2 run = gather_run(pm, p);
+  if (run.x >= 0 && run.y == 0) return f3(0.0f, 0.0f, 0.0f);
+  return gather_sum(pm, run, p, n);
+}
+
 // Hit point and facing normal of a closest hit at fp32 distance t: the
 // sphereHitAccel normal (renderer.go:670-677) or the triangle's unit normal,
 // flipped to face the ray (triHit, renderer.go:704-710). `nrm` is the slot's snorm word.
@@ -142,7 +152,7 @@ struct Surface {
 };
 __device__ __forceinline__ Surface hit_surface(const SceneView& sv, int slot, float4 nrm, float3 o, float3 d, float t) {
   Surface S;
-  S.p = o + d * t;
+  S.p = fma3(d, t, o);
   const float4 r2 = __ldg(sv.tri + 3 * slot + 2);
   S.sphere = r2.w < 0.0f;
   S.radius = 0.0f;

@@ -13,6 +13,8 @@
 //                bounce) / metal / glass, Russian roulette; survivors are pushed
 //                with block-level compaction (one atomic per block), shadow rays
 //                with warp-ballot compaction (one atomic per warp)
+//   gather    -> (photon integrator) the photon density at the bounce's diffuse
+//                vertices, sorted by photon cell
 //   connect   -> any hit for the shadow queue; unoccluded contributions are added
 //   accumulate-> per pixel, the firefly-clamped sample radiance of the wave,
 //                summed in sample order (no atomics: one thread per pixel)
@@ -87,13 +89,30 @@ struct RecurRec {
   int cap;
 };
 
+// Photon gathers of one bounce. The shading step lists the diffuse vertices of
+// photon views whose cell has photons; k_gather adds their photon radiance.
+// Sorted by the photon run, the lanes of a warp read the same candidates.
+constexpr int kGatherBins = 1 << 16;
+constexpr int kGatherSortPaths = 1 << 20;  // waves of at least this many paths sort their gathers
+struct GatherSoA {
+  float4* p;       // point, first list entry
+  float4* n;       // facing normal, list entries
+  float4* w;       // throughput at the vertex, path slot
+  uint32_t* key;   // sort bin (kGatherBins of them)
+  uint32_t* rank;  // rank within the bin
+  int32_t* perm;   // sorted order
+  int* bins;       // [kGatherBins] zero between bounces
+  int* base;       // [kGatherBins] first place of each bin
+};
+
 // Device counters of a wave. cur/next alternate between [0] and [1].
 struct WaveCounters {
   int q[2];
   int shadow;
   int work_ext;
   int work_con;
-  int pad[3];
+  int gather;
+  int pad[2];
   unsigned long long rays;
   unsigned long long shadow_rays;
 };
@@ -375,6 +394,7 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
     atomicAdd(&cnt->rays, (unsigned long long)n);
     cnt->q[cur ^ 1] = 0;  // the queue and shadow list this bounce's shade fills
     cnt->shadow = 0;
+    cnt->gather = 0;
   }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
@@ -454,7 +474,7 @@ __device__ __forceinline__ float light_dir_pdf(const ShadeScene& sc, int n_light
   float dist2 = dot3(to, to);
   if (dist2 <= 1e-12f) return 0.0f;
   float3 ld = unit3(to);
-  float cosL = fmaxf(0.0f, dot3(ln, ld * -1.0f));
+  float cosL = fmaxf(0.0f, neg_dot3(ln, ld));
   if (cosL <= 1e-12f) return 0.0f;
   float area = 4.0f * kPi * radius * radius;
   float sel = n_lights == 0 ? 0.0f : (power ? __ldg(sc.lpdf_by_prim + prim) : 1.0f / (float)n_lights);
@@ -495,6 +515,10 @@ struct SoAPath {
     L = get_L() + v;
     l_added = true;
   }
+  __device__ __forceinline__ void add_L(float3 a, float3 b) {  // a b, component-wise
+    L = fma3(a, b, get_L());
+    l_added = true;
+  }
   __device__ __forceinline__ void flush_L() {
     if (!LAZY || l_added) {
       sst(ps.lx + path, L.x); sst(ps.ly + path, L.y); sst(ps.lz + path, L.z);
@@ -529,6 +553,7 @@ struct RegPath {
   float ppdf;
   __device__ __forceinline__ float3 get_L() const { return L; }
   __device__ __forceinline__ void add_L(float3 v) { L = L + v; }
+  __device__ __forceinline__ void add_L(float3 a, float3 b) { L = fma3(a, b, L); }
   __device__ __forceinline__ void load_vertex() {}
   __device__ __forceinline__ float3 prev() const { return pv; }
   __device__ __forceinline__ void set_prev(float3 p) { pv = p; }
@@ -545,6 +570,9 @@ struct VertexOut {
   float4 so, sd, scon;  // shadow ray: origin + tmax, direction + scene root, contribution
   int rec_m;
   float3 rec_v;
+  bool gather;         // photon gather to do (DEFER), at point gp with normal gn, weight gw
+  float3 gp, gn, gw;
+  int2 grun;
 };
 
 // Guide outputs of a path's first vertex (sample 0 only).
@@ -568,8 +596,8 @@ __device__ __forceinline__ void write_guides(const GuideOut& gd, float3 N, float
     px = copysignf(ax, q.x);
     py = copysignf(ay, q.y);
   }
-  px = fminf(fmaxf(px * 0.5f + 0.5f, 0.0f), 1.0f);
-  py = fminf(fmaxf(py * 0.5f + 0.5f, 0.0f), 1.0f);
+  px = fminf(fmaxf(__fmaf_rn(px, 0.5f, 0.5f), 0.0f), 1.0f);
+  py = fminf(fmaxf(__fmaf_rn(py, 0.5f, 0.5f), 0.0f), 1.0f);
   const uint32_t qx = (uint32_t)rintf(px * 1023.0f), qy = (uint32_t)rintf(py * 1023.0f);
   const uint32_t mm = (uint32_t)min(max(m, 0), 2047);
   uint32_t* g = gd.c + 3 * (size_t)gd.px;
@@ -603,13 +631,13 @@ __device__ __forceinline__ int sample_direct(const ViewGPU& wp, const ShadeScene
   }
   const LightGPU Lg = sc.lights[wp.light_off + li];
   const float3 ln = sel > 0.0f ? rand_unit_vector(rng) : f3(0, 0, 1);
-  const float3 q = f3(Lg.cx, Lg.cy, Lg.cz) + ln * Lg.r;
+  const float3 q = fma3(ln, Lg.r, f3(Lg.cx, Lg.cy, Lg.cz));
   const float3 to = q - p;
   const float dist2 = dot3(to, to);
   if (!(dist2 >= 1e-8f && sel > 0.0f)) return 0;
   const float3 ld = unit3(to);
   const float ndl = fmaxf(0.0f, dot3(N, ld));
-  const float cosL = fmaxf(0.0f, dot3(ln * -1.0f, ld));
+  const float cosL = fmaxf(0.0f, neg_dot3(ln, ld));
   if (!(ndl > 0.0f && cosL > 0.0f)) return 0;
   const float area = 4.0f * kPi * Lg.r * Lg.r;
   const float lightPDF = sel * dist2 / (cosL * area);
@@ -618,7 +646,7 @@ __device__ __forceinline__ int sample_direct(const ViewGPU& wp, const ShadeScene
   const float w = wp.mis ? power_heuristic(lightPDF, bsdfPDF) : 1.0f;
   const float3 f = f3(M.cr, M.cg, M.cb) * (1.0f / kPi);
   *contrib = had(weight, had(f, f3(Lg.er, Lg.eg, Lg.eb)) * (ndl * w / lightPDF));
-  const float3 from = p + N * 2e-4f;  // visible (renderer.go:1333-1341)
+  const float3 from = fma3(N, 2e-4f, p);  // visible (renderer.go:1333-1341)
   const float3 sdv = q - from;
   const float sd2 = dot3(sdv, sdv);
   if (sd2 < 1e-12f) return 1;
@@ -634,8 +662,9 @@ __device__ __forceinline__ int sample_direct(const ViewGPU& wp, const ShadeScene
 // weight), for a path whose extension ray hit `slot` at fp32 distance t
 // (slot < 0: miss). Updates s.L / s.tp and, when the path continues, its next
 // ray (store_continuation). ALT: the batch has views of the other integrators
-// (the path-only kernels compile without their code).
-template <bool ALT, class P>
+// (the path-only kernels compile without their code). DEFER: photon gathers are
+// left to the caller (VertexOut.gather).
+template <bool ALT, bool DEFER, class P>
 __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, const ShadeScene& sc, P& s, float t,
                                              int slot, int bounce, const GuideOut& gd, VertexOut& out,
                                              bool want_rec) {
@@ -643,11 +672,12 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
   out.shadow = false;
   out.rec_m = -1;
   out.rec_v = f3(0, 0, 0);
+  out.gather = false;
   const int rr_depth = wp.rr_depth < 1 ? 4 : wp.rr_depth;
   const float3 o = s.o, d = s.d;
   float3 tp = s.tp;
   if (slot < 0) {
-    s.add_L(had(tp, background(d)));
+    s.add_L(tp, background(d));
   } else {
     const float4 nrm = __ldg(sc.sv.snorm + slot);
     const int m = __float_as_int(nrm.w);
@@ -671,7 +701,7 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
           }
           w = power_heuristic(ppdf, lpdf);
         }
-        s.add_L(had(tp, f3(M.er, M.eg, M.eb)) * w);
+        s.add_L(had(tp, f3(M.er, M.eg, M.eb)), f3(w, w, w));
         out.rec_m = m | kEmitTag;
         out.rec_v = tp * w;
       } else {
@@ -680,7 +710,17 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
         if (kind == BC_MAT_DIFFUSE) {
           out.rec_m = m;
           if (want_rec) out.rec_v = s.get_L();  // everything added from here on carries this albedo once more
-          if (ALT && wp.integrator == BC_INTEGRATOR_PHOTON) s.add_L(had(tp, photon_gather(wp.pm, p, N)));
+          if (ALT && wp.integrator == BC_INTEGRATOR_PHOTON) {
+            if (DEFER) {
+              out.grun = gather_run(wp.pm, p);
+              out.gather = out.grun.x < 0 || out.grun.y > 0;  // else nothing to add
+              out.gp = p;
+              out.gn = N;
+              out.gw = tp;
+            } else {
+              s.add_L(tp, photon_gather(wp.pm, p, N));
+            }
+          }
           float3 contrib;
           const int k = sample_direct(wp, sc, rng, p, N, M, tp, &out.so, &out.sd, &contrib);
           if (k == 1) {
@@ -696,31 +736,32 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
           // prevPoint feeds only lightDirectionalPDF of a sphere light hit,
           // which is 0 for a view without sphere lights
           if (wp.n_lights > 0) s.set_prev(p);
-          no = p + N * 2e-4f;
+          no = fma3(N, 2e-4f, p);
         } else if (kind == BC_MAT_METAL) {
           const float rough = fminf(fmaxf(M.rough, 0.0f), 1.0f);
-          nd_dir = unit3(reflect3(unit3(d), N) + rand_in_unit_sphere(rng) * rough);
+          nd_dir = unit3(fma3(rand_in_unit_sphere(rng), rough, reflect3(unit3(d), N)));
           if (dot3(nd_dir, N) <= 0.0f) {
             cont = false;
           } else {
             flags &= ~1u;
             tp = had(tp, f3(M.cr, M.cg, M.cb));
-            no = p + N * 2e-4f;
+            no = fma3(N, 2e-4f, p);
           }
         } else {  // glass
           float eta = M.ior;
           if (eta <= 1.0f) eta = 1.5f;
           const float ratio = S.front ? 1.0f / eta : eta;
           const float3 un = unit3(d);
-          const float cosT = fminf(dot3(un * -1.0f, N), 1.0f);
-          const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
+          const float udn = glass_dot(un, N);
+          const float cosT = fminf(-udn, 1.0f);
+          const float sinT = sqrtf(fmaxf(0.0f, __fmaf_rn(-cosT, cosT, 1.0f)));
           if (ratio * sinT > 1.0f || schlick(cosT, ratio) > rng.uniform())
-            nd_dir = reflect3(un, N);
+            nd_dir = glass_reflect(un, N, udn);
           else
-            nd_dir = refract3(un, N, ratio);
+            nd_dir = glass_refract(un, N, udn, ratio);
           flags &= ~1u;
           tp = had(tp, f3(M.cr, M.cg, M.cb));
-          no = p + nd_dir * 2e-4f;
+          no = fma3(nd_dir, 2e-4f, p);
         }
         if (cont && bounce >= rr_depth) {  // Russian roulette (renderer.go:1550-1560)
           const float pr = fminf(fmaxf(maxcomp(tp), 0.08f), 0.95f);
@@ -759,7 +800,7 @@ __device__ __forceinline__ bool shade_recursive(const ViewGPU& wp, int n_mats, c
   float4 rec = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
   const size_t r = (size_t)bounce * rr.cap + path;
   if (slot < 0) {
-    s.add_L(had(W, background(d)));
+    s.add_L(W, background(d));
   } else {
     const float4 nrm = __ldg(sc.sv.snorm + slot);
     const int m = __float_as_int(nrm.w);
@@ -771,7 +812,7 @@ __device__ __forceinline__ bool shade_recursive(const ViewGPU& wp, int n_mats, c
       const float3 col = f3(M.cr, M.cg, M.cb);
       if (gd.px >= 0) write_guides(gd, N, t, d, m);
       if (kind == BC_MAT_EMISSIVE) {
-        s.add_L(had(W, f3(M.er, M.eg, M.eb)));
+        s.add_L(W, f3(M.er, M.eg, M.eb));
       } else if (kind == BC_MAT_DIFFUSE) {
         const float scale = (wp.bounces - bounce < 8) ? 1.0f / fminf(fmaxf(maxcomp(col), 0.1f), 0.95f) : 1.0f;
         const float3 Wv = W * scale;
@@ -780,14 +821,14 @@ __device__ __forceinline__ bool shade_recursive(const ViewGPU& wp, int n_mats, c
         rr.w[r] = make_float4(Wv.x, Wv.y, Wv.z, 0.0f);
         W = had(Wv, col);
         nd_dir = rand_cos_hemisphere(N, rng);
-        no = p + N * 2e-4f;
+        no = fma3(N, 2e-4f, p);
         cont = true;
       } else if (kind == BC_MAT_METAL) {
         const float rough = fminf(fmaxf(M.rough, 0.0f), 1.0f);
-        nd_dir = unit3(reflect3(unit3(d), N) + rand_in_unit_sphere(rng) * rough);
+        nd_dir = unit3(fma3(rand_in_unit_sphere(rng), rough, reflect3(unit3(d), N)));
         if (dot3(nd_dir, N) > 0.0f) {
           W = had(W, col);
-          no = p + N * 2e-4f;
+          no = fma3(N, 2e-4f, p);
           cont = true;
         }
       } else {  // glass and any other kind
@@ -795,14 +836,15 @@ __device__ __forceinline__ bool shade_recursive(const ViewGPU& wp, int n_mats, c
         if (eta <= 1.0f) eta = 1.5f;
         const float ratio = S.front ? 1.0f / eta : eta;
         const float3 un = unit3(d);
-        const float cosT = fminf(dot3(un * -1.0f, N), 1.0f);
-        const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
+        const float udn = glass_dot(un, N);
+        const float cosT = fminf(-udn, 1.0f);
+        const float sinT = sqrtf(fmaxf(0.0f, __fmaf_rn(-cosT, cosT, 1.0f)));
         if (ratio * sinT > 1.0f || schlick(cosT, ratio) > rng.uniform())
-          nd_dir = reflect3(un, N);
+          nd_dir = glass_reflect(un, N, udn);
         else
-          nd_dir = refract3(un, N, ratio);
+          nd_dir = glass_refract(un, N, udn, ratio);
         W = had(W, col);
-        no = p + nd_dir * 2e-4f;
+        no = fma3(nd_dir, 2e-4f, p);
         cont = true;
       }
     }
@@ -862,7 +904,7 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
                                                ShadowSoA sh, WaveCounters* cnt, int cur, int bounce,
                                                float4* __restrict__ guide_nd, uint32_t* __restrict__ guide_c,
                                                const uint32_t* __restrict__ guide_jit, GradRec rec, RecurRec rr,
-                                               long long sh_cap, unsigned* status) {
+                                               GatherSoA ga, int gshift, long long sh_cap, unsigned* status) {
   const int n = *((volatile int*)&cnt->q[cur]);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     cnt->work_ext = 0;  // the next bounce's extend and this bounce's connect start from zero
@@ -875,6 +917,7 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
     VertexOut out;
     out.alive = false;
     out.shadow = false;
+    out.gather = false;
     if (path >= 0) {
       const ViewGPU& wp = views[sld(ps.view + path)];
       SoAPath<!ALT> s(ps, path);
@@ -887,7 +930,7 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
         out.alive = !ended;
         if (ended) unwind_recursive(wp, sc, s.rng, rr, path, bounce, sh, cnt, sh_cap, status);
       } else {
-        shade_vertex<ALT>(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, out, rec.m != nullptr);
+        shade_vertex<ALT, true>(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, out, rec.m != nullptr);
       }
       s.flush_L();
       if (rec.m) {
@@ -910,6 +953,15 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
         atomicOr(status, kStatusCapacity);
       }
     }
+    if (ALT) {  // at most one gather per path and bounce: the queue has a slot for each
+      const int qg = warp_reserve(&cnt->gather, out.gather);
+      if (out.gather) {
+        ga.p[qg] = make_float4(out.gp.x, out.gp.y, out.gp.z, __int_as_float(out.grun.x));
+        ga.n[qg] = make_float4(out.gn.x, out.gn.y, out.gn.z, __int_as_float(out.grun.y));
+        ga.w[qg] = make_float4(out.gw.x, out.gw.y, out.gw.z, __int_as_float(path));
+        ga.key[qg] = out.grun.x < 0 ? kGatherBins - 1u : min((uint32_t)out.grun.x >> gshift, kGatherBins - 1u);
+      }
+    }
   }
 }
 
@@ -921,14 +973,103 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
   const ViewGPU *__restrict__ views, int n_mats, ShadeScene sc, PathSoA ps, const int *__restrict__ qcur,  \
       int *__restrict__ qnext, ShadowSoA sh, WaveCounters *cnt, int cur, int bounce,                       \
       float4 *__restrict__ guide_nd, uint32_t *__restrict__ guide_c, const uint32_t *__restrict__ guide_jit, \
-      GradRec rec, RecurRec rr, long long sh_cap, unsigned *status
-#define BC_SHADE_PASS views, n_mats, sc, ps, qcur, qnext, sh, cnt, cur, bounce, guide_nd, guide_c, guide_jit, rec, rr, sh_cap, status
+      GradRec rec, RecurRec rr, GatherSoA ga, int gshift, long long sh_cap, unsigned *status
+#define BC_SHADE_PASS views, n_mats, sc, ps, qcur, qnext, sh, cnt, cur, bounce, guide_nd, guide_c, guide_jit, rec, rr, ga, gshift, sh_cap, status
 template <bool ALT>
 __global__ void __launch_bounds__(256, 4) k_shade(BC_SHADE_ARGS) { shade_body<ALT, 256>(BC_SHADE_PASS); }
 template <bool ALT>
 __global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_body<ALT, 128>(BC_SHADE_PASS); }
 #undef BC_SHADE_ARGS
 #undef BC_SHADE_PASS
+
+// ---- gather --------------------------------------------------------------------
+// The photon gathers of a bounce. In the shading kernel, at 64 registers and
+// with its block barriers, they took 7.6 of a 9.5 ms photon frame: the barrier
+// waits for the block's longest run on the first bounce, and later bounces run
+// 7 of 32 lanes, each on its own candidates. Here the vertices are listed,
+// counting-sorted by their run (k_gather_count, k_gather_scan, k_gather_scatter)
+// and gathered with the lanes of a warp on the same run.
+__global__ void __launch_bounds__(256) k_gather_count(GatherSoA ga, const WaveCounters* cnt) {
+  const int n = cnt->gather;
+  const int lane = threadIdx.x & 31;
+  const int stride = gridDim.x * blockDim.x;
+  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+    const int i = base + threadIdx.x;
+    const uint32_t key = i < n ? ga.key[i] : 0xffffffffu;
+    // one atomic per distinct bin of the warp: neighbouring vertices share cells
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if (lane == leader && i < n) at = atomicAdd(&ga.bins[key], __popc(peers));
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (i < n) ga.rank[i] = (uint32_t)(at + __popc(peers & ((1u << lane) - 1u)));
+  }
+}
+
+// Exclusive scan of the bins (one block), which are cleared for the next bounce.
+__global__ void __launch_bounds__(1024) k_gather_scan(GatherSoA ga) {
+  __shared__ int wsum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int carry = 0;
+  for (int b0 = 0; b0 < kGatherBins; b0 += 8192) {
+    int v[8], s = 0;
+    int4* src = reinterpret_cast<int4*>(ga.bins + b0) + 2 * threadIdx.x;
+    const int4 x = src[0], y = src[1];
+    src[0] = make_int4(0, 0, 0, 0);
+    src[1] = make_int4(0, 0, 0, 0);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int c = v[k];
+      v[k] = s;
+      s += c;
+    }
+    int inc = s;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int z = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += z;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    int below = carry, all = 0;
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+      const int c = wsum[k];
+      if (k < w) below += c;
+      all += c;
+    }
+    below += inc - s;
+    int4* dst = reinterpret_cast<int4*>(ga.base + b0) + 2 * threadIdx.x;
+    dst[0] = make_int4(below + v[0], below + v[1], below + v[2], below + v[3]);
+    dst[1] = make_int4(below + v[4], below + v[5], below + v[6], below + v[7]);
+    carry += all;
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) k_gather_scatter(GatherSoA ga, const WaveCounters* cnt) {
+  const int n = cnt->gather;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    ga.perm[ga.base[ga.key[i]] + (int)ga.rank[i]] = i;
+}
+
+__global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ views, PathSoA ps, GatherSoA ga,
+                                                const WaveCounters* cnt, int sorted) {
+  const int n = cnt->gather;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const int i = sorted ? ga.perm[j] : j;
+    const float4 P = ga.p[i], N = ga.n[i], W = ga.w[i];
+    const int path = __float_as_int(W.w);
+    const PhotonView& pm = views[ps.view[path]].pm;
+    const float3 g = gather_sum(pm, make_int2(__float_as_int(P.w), __float_as_int(N.w)), f3(P.x, P.y, P.z),
+                                f3(N.x, N.y, N.z));
+    const float3 L = fma3(f3(W.x, W.y, W.z), g, f3(ps.lx[path], ps.ly[path], ps.lz[path]));
+    ps.lx[path] = L.x;
+    ps.ly[path] = L.y;
+    ps.lz[path] = L.z;
+  }
+}
 
 // ---- connect -----------------------------------------------------------------
 template <int STACK, bool SPH>
@@ -1040,7 +1181,7 @@ __global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* _
           }
         const float3 c = clamp_sample(L, V.clamp);
         acc = acc + c;
-        acc2 = acc2 + had(c, c);
+        acc2 = fma3(c, c, acc2);
         if (V.adaptive) stop = adaptive_step(V, c, &an, &sl, &ssl);
       }
       if (V.adaptive) {
@@ -1195,7 +1336,7 @@ __global__ void __launch_bounds__(128) k_render_plain(const ViewGPU* __restrict_
         segs++;
         const GuideOut gd{guide_nd, guide_c, guide_jit, (b == 0 && guide) ? V.pix_off + p : -1};
         VertexOut out;
-        shade_vertex<ALT>(V, n_mats, sc, st, leaf.best_t, leaf.best_slot, b, gd, out, false);
+        shade_vertex<ALT, false>(V, n_mats, sc, st, leaf.best_t, leaf.best_slot, b, gd, out, false);
         if (out.shadow) {
           shadows++;
           const Ray32 sr = make_ray(out.so.x, out.so.y, out.so.z, out.sd.x, out.sd.y, out.sd.z, 1e-4f);
@@ -1209,7 +1350,7 @@ __global__ void __launch_bounds__(128) k_render_plain(const ViewGPU* __restrict_
       }
       const float3 c = clamp_sample(st.L, V.clamp);
       acc = acc + c;
-      acc2 = acc2 + had(c, c);
+      acc2 = fma3(c, c, acc2);
       if (V.adaptive && adaptive_step(V, c, &an, &sl, &ssl)) {
         an |= kPixDone;
         break;
@@ -1285,6 +1426,10 @@ struct RenderBuffers {
   bcgx::DevBuf rrec;
   bcgx::RecurRec rr{};
   int rr_bounces = 0, rr_cap = 0;
+  // photon gathers of a bounce
+  bcgx::DevBuf gather;
+  bcgx::GatherSoA ga{};
+  int gather_cap = 0;
   // one wave as an instantiated CUDA graph, and the launch arguments it was captured with
   cudaGraphExec_t graph = nullptr;
   std::vector<uintptr_t> graph_key;
@@ -1333,6 +1478,7 @@ void destroy_render_buffers(bc_context* ctx) {
   rb->staging.release();
   rb->rec.release();
   rb->rrec.release();
+  rb->gather.release();
   delete rb;
   ctx->rb = nullptr;
 }
@@ -1563,6 +1709,9 @@ struct WaveShape {
   const GradArgs* grad;  // non-null: gradient render
   bool recursive;        // the batch has views of the recursive integrator
   bool alt;              // the batch has views of the recursive or photon integrator
+  bool photon;           // the batch has views of the photon integrator
+  bool gather_sort;      // their gathers are sorted
+  int gshift;            // list entry -> sort bin
 };
 
 template <int STACK, bool SPH>
@@ -1595,6 +1744,8 @@ static WaveShape wave_shape(int cap, int bounces, bool lights, const GradArgs* g
   w.grad = grad;
   w.recursive = false;
   w.alt = false;
+  w.photon = w.gather_sort = false;
+  w.gshift = 0;
   return w;
 }
 
@@ -1623,8 +1774,8 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
     rb->mark(st, kTimeShade);
 #define BC_SHADE_LAUNCH(KERNEL, BLOCK)                                                                         \
   KERNEL<<<w.shade_grid, BLOCK, 0, st>>>(rb->views, ctx->ds.n_mats, sc, rb->ps, rb->q[cur], rb->q[cur ^ 1], rb->sh, \
-                                        c, cur, b, rb->guide_nd, rb->guide_c, rb->guide_jit, rec, rr, rb->sh_cap,   \
-                                        ctx->d_status)
+                                        c, cur, b, rb->guide_nd, rb->guide_c, rb->guide_jit, rec, rr, rb->ga,       \
+                                        w.gshift, rb->sh_cap, ctx->d_status)
     if (w.shade_block == 128) {
       if (w.alt) BC_SHADE_LAUNCH(k_shade_128<true>, 128);
       else BC_SHADE_LAUNCH(k_shade_128<false>, 128);
@@ -1633,6 +1784,14 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
       else BC_SHADE_LAUNCH(k_shade<false>, 256);
     }
 #undef BC_SHADE_LAUNCH
+    if (w.photon) {
+      if (w.gather_sort) {
+        k_gather_count<<<w.acc_grid * 2, 256, 0, st>>>(rb->ga, c);
+        k_gather_scan<<<1, 1024, 0, st>>>(rb->ga);
+        k_gather_scatter<<<w.acc_grid * 2, 256, 0, st>>>(rb->ga, c);
+      }
+      k_gather<<<w.acc_grid * 4, 128, 0, st>>>(rb->views, rb->ps, rb->ga, c, w.gather_sort ? 1 : 0);
+    }
     if (w.lights) rb->mark(st, kTimeConnect);
     if (w.lights)
       k_connect<STACK, SPH><<<w.con_grid, 128, 0, st>>>(sc.sv, rb->ps, rb->sh, c, rr, rb->sh_cap, ctx->d_status);
@@ -1653,7 +1812,7 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
 // Runs `n_waves` waves, through one captured CUDA graph when the option allows.
 template <int STACK, bool SPH>
 static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const ShadeScene& sc, int64_t n_waves,
-                           int wave_paths, const GradArgs* grad, bool recursive, bool alt) {
+                           int wave_paths, const GradArgs* grad, bool recursive, bool alt, int photon_entries) {
   RenderBuffers* rb = ctx->rb;
   cudaStream_t st = ctx->stream;
   // generate's grid covers this render's wave, not the slots a larger earlier
@@ -1661,11 +1820,15 @@ static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const Shad
   WaveShape w = wave_shape<STACK, SPH>(wave_paths, bounces, lights, grad, ctx->render_extend, ctx->render_shade_block);
   w.recursive = recursive;
   w.alt = alt;
+  w.photon = photon_entries > 0;
+  w.gather_sort = w.photon && wave_paths >= kGatherSortPaths;
+  while ((photon_entries >> w.gshift) >= kGatherBins) w.gshift++;
   // A wave graph pays for its capture when a render has several waves, or when
   // a single-wave render repeats with the same launches (a frame loop at fixed
   // settings): such a render is captured the second time its key is seen.
   bool use_graph = ctx->render_graph != 0 && !rb->ktiming;  // per-launch events need direct launches
-  rb->launches += n_waves * (3 + (int64_t)bounces * (2 + (lights ? 1 : 0)) + (grad ? 1 : 0));
+  rb->launches += n_waves * (3 + (int64_t)bounces * (2 + (lights ? 1 : 0) + (w.photon ? (w.gather_sort ? 4 : 1) : 0)) +
+                             (grad ? 1 : 0));
   rb->extend_launches += n_waves * (int64_t)bounces;
   if (use_graph) {
     // every value the captured launches were given
@@ -1689,6 +1852,9 @@ static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const Shad
     key.push_back((uintptr_t)recursive);
     key.push_back((uintptr_t)alt);
     if (recursive) add_bytes(&rb->rr, sizeof(rb->rr));
+    key.push_back((uintptr_t)(w.photon ? 1 + w.gather_sort : 0));
+    key.push_back((uintptr_t)w.gshift);
+    if (w.photon) add_bytes(&rb->ga, sizeof(rb->ga));
     add_bytes(&sc, sizeof(sc));
     key.push_back((uintptr_t)(grad != nullptr));
     if (grad) {
@@ -1787,7 +1953,7 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
   std::vector<ViewGPU> views(n);
   std::vector<double> X, Y;
   long long total = 0;
-  int max_bounces = 0, rec_bounces = 0;
+  int max_bounces = 0, rec_bounces = 0, photon_entries = 0;
   bool lights = false, alt = false;
   std::vector<const unsigned long long*> photon_rays;  // ray counters of photon maps built for this call
   const uint64_t photon_pin = photon_clock(ctx);
@@ -1827,6 +1993,7 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
       const unsigned long long* built = nullptr;
       if ((bst = photon_map_for(ctx, r.scene, r.s, photon_pin, &V.pm, &built))) return bst;
       if (built) photon_rays.push_back(built);
+      photon_entries = std::max(photon_entries, photon_list_entries(r.s));
     }
     camera_basis(r.cam, (double)V.W / (double)V.H, V.origin, V.lower, V.horiz, V.vert);
     for (int k = 0; k < 3; k++) {
@@ -1866,6 +2033,25 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     rb->rr.cap = cap;
     rb->rr_bounces = rec_bounces;
     rb->rr_cap = cap;
+  }
+  if (photon_entries && rb->gather_cap < cap) {
+    cudaError_t e = rb->gather.ensure((size_t)cap * (3 * sizeof(float4) + 3 * sizeof(int32_t)) +
+                                      2 * kGatherBins * sizeof(int) + 8 * 256);
+    if (e) {
+      rb->gather_cap = 0;
+      return cuda_status(ctx, e, "photon gather queue");
+    }
+    char* p = (char*)rb->gather.p;
+    GatherSoA& g = rb->ga;
+    g.bins = carve<int>(p, kGatherBins);
+    g.base = carve<int>(p, kGatherBins);
+    g.p = carve<float4>(p, cap);
+    g.n = carve<float4>(p, cap);
+    g.w = carve<float4>(p, cap);
+    g.key = carve<uint32_t>(p, cap);
+    g.rank = carve<uint32_t>(p, cap);
+    g.perm = carve<int32_t>(p, cap);
+    rb->gather_cap = cap;
   }
   if (grad) {  // path replay records: one per path and bounce
     if (max_bounces > kMaxGradBounces) return set_error(ctx, BC_ERR_INVALID_ARG, "gradient renders allow 64 bounces");
@@ -1918,6 +2104,7 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
   e = cudaMemcpyAsync(rb->table.p, hs, tbytes, cudaMemcpyHostToDevice, ctx->stream);
   if (!e && !X.empty())
     e = cudaMemcpyAsync(rb->seq.p, hq, X.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream);
+  if (!e && photon_entries) e = cudaMemsetAsync(rb->ga.bins, 0, kGatherBins * sizeof(int), ctx->stream);
   for (int v = 0; v < n && !e; v++) {
     const ViewGPU& V = views[v];
     e = cudaMemsetAsync(rb->sum + 3 * (size_t)V.pix_off, 0, 3 * sizeof(float) * (size_t)V.npix, ctx->stream);
@@ -1952,14 +2139,20 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     else if (stack == 128) bst = sph ? run_plain<128, true>(ctx, sc, views, alt) : run_plain<128, false>(ctx, sc, views, alt);
     else bst = sph ? run_plain<256, true>(ctx, sc, views, alt) : run_plain<256, false>(ctx, sc, views, alt);
   } else if (stack == 64)
-    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt)
-              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt);
+    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries)
+              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries);
   else if (stack == 128)
-    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt)
-              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt);
+    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries)
+              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries);
   else
-    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt)
-              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt);
+    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries)
+              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
+                                photon_entries);
   if (bst) return bst;
   rb->mark(ctx->stream, kTimeOther);
   k_finish_views<<<sm_count() * 8, 256, 0, ctx->stream>>>(rb->views, n, rb->sum, rb->out, rb->adapt.n);

@@ -41,6 +41,7 @@ struct PhotonView;
 uint64_t photon_clock(bc_context* ctx);
 bc_status photon_map_for(bc_context* ctx, int scene, const bc_settings& s, uint64_t pin, PhotonView* view,
                          const unsigned long long** built_rays);
+int photon_list_entries(const bc_settings& s);  // neighbour-list entries of the map's capacity
 int gradient_grid();
 int effective_spp(const bc_settings& s);
 
