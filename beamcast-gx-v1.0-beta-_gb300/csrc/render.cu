@@ -40,19 +40,18 @@
 
 namespace bcgx {
 
-struct PathSoA {
-  float *ox, *oy, *oz, *dx, *dy, *dz;
-  float *tx, *ty, *tz;     // throughput
-  float *lx, *ly, *lz;     // radiance of the path so far
-  float *px, *py, *pz;     // prevPoint
-  uint32_t* prev;          // prevBSDFPDF (fp32, >= 0) in bits 0-30, prevWasDiffuse in bit 31
-  uint64_t *rs, *ri;       // PCG32 state and increment
-  float* hit_t;
-  int32_t* hit_slot;
-  int32_t* view;           // view of the path
-  int32_t* pix;            // pixel within the view's rows
-  int32_t* samp;           // sample index
+// Path state in 32-byte records. The queue of a bounce is in path order but
+// thins out, and a lane that reads 4 bytes of every array pulls a 32-byte
+// sector for each once its neighbours' paths have ended; a record is one full
+// sector whatever the density, and two 128-bit accesses.
+struct PathState {
+  float4* ray;    // [2i] = (origin, view bits), [2i + 1] = (direction, scene root bits)
+  float4* st;     // [2i] = (throughput, prev word), [2i + 1] = PCG32 (state, inc) bits
+  float4* L;      // radiance of the path so far; w unused
+  float4* prevp;  // prevPoint; w unused
+  float2* hit;    // (t, slot bits) of the bounce's queue entries, by queue position
 };
+// prev word: prevBSDFPDF (fp32, >= 0) in bits 0-30, prevWasDiffuse in bit 31.
 
 struct ShadowSoA {
   float4* o;  // origin, tmax
@@ -183,17 +182,18 @@ constexpr int kMaxBounces = 1024;  // a wave is one launch sequence of max(bounc
 // gigabytes per wave), so its loads and stores are marked evict-first
 // (ld.global.cs / st.global.cs): L2 stays with the BVH nodes and triangle
 // records the walks reuse.
-__device__ __forceinline__ float sld(const float* p) { return __ldcs(p); }
-__device__ __forceinline__ int32_t sld(const int32_t* p) { return __ldcs(p); }
-__device__ __forceinline__ uint32_t sld(const uint32_t* p) { return __ldcs(p); }
-__device__ __forceinline__ uint64_t sld(const uint64_t* p) {
-  return __ldcs(reinterpret_cast<const unsigned long long*>(p));
+__device__ __forceinline__ float4 sld(const float4* p) { return __ldcs(p); }
+__device__ __forceinline__ void sst(float4* p, float4 v) { __stcs(p, v); }
+__device__ __forceinline__ float4 with_bits(float3 v, uint32_t w) { return make_float4(v.x, v.y, v.z, __uint_as_float(w)); }
+__device__ __forceinline__ float4 rng_bits(const Pcg32& r) {
+  return make_float4(__uint_as_float((uint32_t)r.state), __uint_as_float((uint32_t)(r.state >> 32)),
+                     __uint_as_float((uint32_t)r.inc), __uint_as_float((uint32_t)(r.inc >> 32)));
 }
-__device__ __forceinline__ void sst(float* p, float v) { __stcs(p, v); }
-__device__ __forceinline__ void sst(int32_t* p, int32_t v) { __stcs(p, v); }
-__device__ __forceinline__ void sst(uint32_t* p, uint32_t v) { __stcs(p, v); }
-__device__ __forceinline__ void sst(uint64_t* p, uint64_t v) {
-  __stcs(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
+__device__ __forceinline__ Pcg32 rng_of(float4 b) {
+  Pcg32 r;
+  r.state = (uint64_t)__float_as_uint(b.x) | (uint64_t)__float_as_uint(b.y) << 32;
+  r.inc = (uint64_t)__float_as_uint(b.z) | (uint64_t)__float_as_uint(b.w) << 32;
+  return r;
 }
 
 __device__ __forceinline__ int warp_reserve(int* counter, bool pred) {
@@ -332,7 +332,7 @@ __device__ __forceinline__ uint32_t jitter_word(float jx, float jy) {
 // seq: the views' sample tables, (x, y) pairs
 // The wave's paths of pixels that have not stopped (adaptive sampling) enter
 // the first queue (warp-aggregated append; cnt->q[0] is zero on entry).
-__global__ void k_generate(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views, PathSoA ps,
+__global__ void k_generate(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views, PathState ps,
                            int* __restrict__ queue, const float4* __restrict__ seq,
                            uint32_t* __restrict__ guide_jit, WaveCounters* cnt, AdaptState ad) {
   const long long w0 = bs->w0;
@@ -357,16 +357,11 @@ __global__ void k_generate(const BatchState* __restrict__ bs, const ViewGPU* __r
   Pcg32 rng;
   float jx, jy;
   primary_ray(V, x, y, s, seq, &o, &d, &rng, &jx, &jy);
-  sst(ps.ox + i, o.x); sst(ps.oy + i, o.y); sst(ps.oz + i, o.z);
-  sst(ps.dx + i, d.x); sst(ps.dy + i, d.y); sst(ps.dz + i, d.z);
-  sst(ps.tx + i, 1.0f); sst(ps.ty + i, 1.0f); sst(ps.tz + i, 1.0f);
-  sst(ps.lx + i, 0.0f); sst(ps.ly + i, 0.0f); sst(ps.lz + i, 0.0f);
-  sst(ps.prev + i, 0u);
-  sst(ps.rs + i, rng.state);
-  sst(ps.ri + i, rng.inc);
-  sst(ps.view + i, (int32_t)v);
-  sst(ps.pix + i, (int32_t)p);
-  sst(ps.samp + i, (int32_t)s);
+  sst(ps.ray + 2 * (size_t)i, with_bits(o, (uint32_t)v));
+  sst(ps.ray + 2 * (size_t)i + 1, with_bits(d, (uint32_t)V.root));
+  sst(ps.st + 2 * (size_t)i, make_float4(1.0f, 1.0f, 1.0f, 0.0f));
+  sst(ps.st + 2 * (size_t)i + 1, rng_bits(rng));
+  sst(ps.L + i, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
   queue[slot] = i;
   if (s == 0 && V.want_guides) guide_jit[V.pix_off + p] = jitter_word(jx, jy);
 }
@@ -386,7 +381,7 @@ __global__ void k_generate(const BatchState* __restrict__ bs, const ViewGPU* __r
 constexpr int kExtendVariants = 3;
 
 template <int STACK, bool SPH, int VAR>
-__device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restrict__ views, PathSoA ps,
+__device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restrict__ views, PathState ps,
                                             const int* __restrict__ queue, WaveCounters* cnt, int cur,
                                             unsigned* status) {
   const int n = *((volatile int*)&cnt->q[cur]);
@@ -398,7 +393,7 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
   }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned below = (1u << lane) - 1u;
-  int path = -1;
+  int at = -1;  // queue position of the lane's path
   bool exhausted = false;
   __shared__ Ray32 ray_sh[VAR == 2 ? 128 : 1];
   Ray32 ray_reg;
@@ -408,9 +403,9 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
   FastWalker<STACK, kLeafVote> w;
   w.reset(r);
   for (;;) {
-    const bool need = path < 0 && !exhausted;
+    const bool need = at < 0 && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, need);
-    if (m && (__popc(m) >= kRefillLanes || !__any_sync(0xffffffffu, path >= 0))) {
+    if (m && (__popc(m) >= kRefillLanes || !__any_sync(0xffffffffu, at >= 0))) {
       const int leader = __ffs(m) - 1;
       int base = 0;
       if ((int)lane == leader) base = atomicAdd(&cnt->work_ext, __popc(m));
@@ -418,21 +413,21 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
       if (need) {
         const int my = base + __popc(m & below);
         if (my < n) {
-          path = queue[my];
-          r = make_ray(sld(ps.ox + path), sld(ps.oy + path), sld(ps.oz + path), sld(ps.dx + path),
-                       sld(ps.dy + path), sld(ps.dz + path), 1e-4f);
+          at = my;
+          const size_t path = (size_t)queue[my];
+          const float4 o = sld(ps.ray + 2 * path), d = sld(ps.ray + 2 * path + 1);
+          r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, 1e-4f);
           leaf.reset(1e30f);
-          w.reset(r, views[sld(ps.view + path)].root);
+          w.reset(r, __float_as_uint(d.w));
         } else {
           exhausted = true;
         }
       }
     }
-    if (!__any_sync(0xffffffffu, path >= 0)) break;
-    if (path >= 0 && w.step(sv, r, leaf, status)) {
-      sst(ps.hit_t + path, leaf.best_t);
-      sst(ps.hit_slot + path, (int32_t)leaf.best_slot);
-      path = -1;
+    if (!__any_sync(0xffffffffu, at >= 0)) break;
+    if (at >= 0 && w.step(sv, r, leaf, status)) {
+      __stcs(ps.hit + at, make_float2(leaf.best_t, __int_as_float(leaf.best_slot)));
+      at = -1;
     }
   }
 }
@@ -440,19 +435,19 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
 // The variants differ only in their launch bounds (variant 0 leaves the
 // register count to the compiler's default heuristic).
 template <int STACK, bool SPH>
-__global__ void __launch_bounds__(128) k_extend(SceneView sv, const ViewGPU* __restrict__ views, PathSoA ps,
+__global__ void __launch_bounds__(128) k_extend(SceneView sv, const ViewGPU* __restrict__ views, PathState ps,
                                                 const int* __restrict__ queue, WaveCounters* cnt, int cur,
                                                 unsigned* status) {
   extend_body<STACK, SPH, 0>(sv, views, ps, queue, cnt, cur, status);
 }
 template <int STACK, bool SPH>
-__global__ void __launch_bounds__(128, 10) k_extend_10(SceneView sv, const ViewGPU* __restrict__ views, PathSoA ps,
+__global__ void __launch_bounds__(128, 10) k_extend_10(SceneView sv, const ViewGPU* __restrict__ views, PathState ps,
                                                        const int* __restrict__ queue, WaveCounters* cnt, int cur,
                                                        unsigned* status) {
   extend_body<STACK, SPH, 1>(sv, views, ps, queue, cnt, cur, status);
 }
 template <int STACK, bool SPH>
-__global__ void __launch_bounds__(128, 12) k_extend_12(SceneView sv, const ViewGPU* __restrict__ views, PathSoA ps,
+__global__ void __launch_bounds__(128, 12) k_extend_12(SceneView sv, const ViewGPU* __restrict__ views, PathState ps,
                                                        const int* __restrict__ queue, WaveCounters* cnt, int cur,
                                                        unsigned* status) {
   extend_body<STACK, SPH, 2>(sv, views, ps, queue, cnt, cur, status);
@@ -482,31 +477,37 @@ __device__ __forceinline__ float light_dir_pdf(const ShadeScene& sc, int n_light
 }
 
 // Path state between bounces as the shading step sees it. The wavefront
-// kernels keep it in the SoA arrays (SoAPath loads what a vertex needs and
-// stores what changes); the one-kernel renderer keeps it in registers (RegPath).
+// kernels keep it in records (RecPath loads what a vertex needs and stores what
+// changes); the one-kernel renderer keeps it in registers (RegPath).
 // LAZY: the path's radiance L is read on its first addition at a vertex and
 // written back only if something was added; most vertices (a diffuse or metal
 // bounce without a light sample) leave it as it was, and the additions keep
 // their order. The kernel with the other integrators' code keeps L in
 // registers from the start: at its register budget the lazy form spills.
 template <bool LAZY>
-struct SoAPath {
-  const PathSoA& ps;
-  int path;
+struct RecPath {
+  const PathState& ps;
+  size_t path;
   float3 o, d, tp, L;
   bool l_read, l_added;
   Pcg32 rng;
+  uint32_t view, root, prev_word;
   uint32_t flags;
   float ppdf;
-  __device__ SoAPath(const PathSoA& p, int i) : ps(p), path(i), l_read(false), l_added(false) {
-    o = f3(sld(ps.ox + i), sld(ps.oy + i), sld(ps.oz + i));
-    d = f3(sld(ps.dx + i), sld(ps.dy + i), sld(ps.dz + i));
-    tp = f3(sld(ps.tx + i), sld(ps.ty + i), sld(ps.tz + i));
+  __device__ RecPath(const PathState& p, int i) : ps(p), path(i), l_read(false), l_added(false) {
+    const float4 a = sld(ps.ray + 2 * path), b = sld(ps.ray + 2 * path + 1), c = sld(ps.st + 2 * path);
+    o = f3(a.x, a.y, a.z);
+    d = f3(b.x, b.y, b.z);
+    tp = f3(c.x, c.y, c.z);
+    view = __float_as_uint(a.w);
+    root = __float_as_uint(b.w);
+    prev_word = __float_as_uint(c.w);
     if (!LAZY) get_L();
   }
   __device__ __forceinline__ float3 get_L() {
     if (!l_read) {
-      L = f3(sld(ps.lx + path), sld(ps.ly + path), sld(ps.lz + path));
+      const float4 v = sld(ps.L + path);
+      L = f3(v.x, v.y, v.z);
       l_read = true;
     }
     return L;
@@ -520,29 +521,24 @@ struct SoAPath {
     l_added = true;
   }
   __device__ __forceinline__ void flush_L() {
-    if (!LAZY || l_added) {
-      sst(ps.lx + path, L.x); sst(ps.ly + path, L.y); sst(ps.lz + path, L.z);
-    }
+    if (!LAZY || l_added) sst(ps.L + path, with_bits(L, 0u));
   }
   __device__ __forceinline__ void load_vertex() {  // only a path that hit a valid material needs these
-    rng.state = sld(ps.rs + path);
-    rng.inc = sld(ps.ri + path);
-    const uint32_t w = sld(ps.prev + path);
-    flags = w >> 31;
-    ppdf = __uint_as_float(w & 0x7fffffffu);
+    rng = rng_of(sld(ps.st + 2 * path + 1));
+    flags = prev_word >> 31;
+    ppdf = __uint_as_float(prev_word & 0x7fffffffu);
   }
   __device__ __forceinline__ float3 prev() const {
-    return f3(sld(ps.px + path), sld(ps.py + path), sld(ps.pz + path));
+    const float4 v = sld(ps.prevp + path);
+    return f3(v.x, v.y, v.z);
   }
-  __device__ __forceinline__ void set_prev(float3 p) {
-    sst(ps.px + path, p.x); sst(ps.py + path, p.y); sst(ps.pz + path, p.z);
-  }
+  __device__ __forceinline__ void set_prev(float3 p) { sst(ps.prevp + path, with_bits(p, 0u)); }
   __device__ __forceinline__ void store_continuation(float3 no, float3 nd) {
-    sst(ps.ox + path, no.x); sst(ps.oy + path, no.y); sst(ps.oz + path, no.z);
-    sst(ps.dx + path, nd.x); sst(ps.dy + path, nd.y); sst(ps.dz + path, nd.z);
-    sst(ps.tx + path, tp.x); sst(ps.ty + path, tp.y); sst(ps.tz + path, tp.z);
-    sst(ps.prev + path, (__float_as_uint(ppdf) & 0x7fffffffu) | (flags & 1u) << 31);  // ppdf >= 0 (or -0)
-    sst(ps.rs + path, rng.state);
+    sst(ps.ray + 2 * path, with_bits(no, view));
+    sst(ps.ray + 2 * path + 1, with_bits(nd, root));
+    // ppdf >= 0 (or -0)
+    sst(ps.st + 2 * path, with_bits(tp, (__float_as_uint(ppdf) & 0x7fffffffu) | (flags & 1u) << 31));
+    sst(ps.st + 2 * path + 1, rng_bits(rng));
   }
 };
 
@@ -899,8 +895,9 @@ __device__ __forceinline__ void unwind_recursive(const ViewGPU& wp, const ShadeS
 }
 
 template <bool ALT, int BLOCK>
-__device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, int n_mats, ShadeScene sc,
-                                               PathSoA ps, const int* __restrict__ qcur, int* __restrict__ qnext,
+__device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
+                                               const ViewGPU* __restrict__ views, int n_mats, ShadeScene sc,
+                                               PathState ps, const int* __restrict__ qcur, int* __restrict__ qnext,
                                                ShadowSoA sh, WaveCounters* cnt, int cur, int bounce,
                                                float4* __restrict__ guide_nd, uint32_t* __restrict__ guide_c,
                                                const uint32_t* __restrict__ guide_jit, GradRec rec, RecurRec rr,
@@ -919,12 +916,16 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
     out.shadow = false;
     out.gather = false;
     if (path >= 0) {
-      const ViewGPU& wp = views[sld(ps.view + path)];
-      SoAPath<!ALT> s(ps, path);
+      RecPath<!ALT> s(ps, path);
+      const ViewGPU& wp = views[s.view];
       GuideOut gd{guide_nd, guide_c, guide_jit, -1};
-      if (bounce == 0 && wp.want_guides && ps.samp[path] == 0) gd.px = wp.pix_off + ps.pix[path];
-      const float hit_t = sld(ps.hit_t + path);
-      const int hit_slot = sld(ps.hit_slot + path);
+      if (bounce == 0 && wp.want_guides) {
+        const long long local = bs->w0 + path - wp.path_off;  // sample-major: sample 0 comes first
+        if (local < wp.npix) gd.px = wp.pix_off + local;
+      }
+      const float2 hit = __ldcs(ps.hit + idx);
+      const float hit_t = hit.x;
+      const int hit_slot = __float_as_int(hit.y);
       if (ALT && wp.integrator == BC_INTEGRATOR_RECURSIVE) {
         const bool ended = shade_recursive(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, rr, path);
         out.alive = !ended;
@@ -970,11 +971,11 @@ __device__ __forceinline__ void shade_body(const ViewGPU* __restrict__ views, in
 // 128 threads at eight; the same 64-register budget and resident threads, a
 // different scheduling granularity of the grid-stride loop.
 #define BC_SHADE_ARGS                                                                                       \
-  const ViewGPU *__restrict__ views, int n_mats, ShadeScene sc, PathSoA ps, const int *__restrict__ qcur,  \
-      int *__restrict__ qnext, ShadowSoA sh, WaveCounters *cnt, int cur, int bounce,                       \
+  const BatchState *__restrict__ bs, const ViewGPU *__restrict__ views, int n_mats, ShadeScene sc,         \
+      PathState ps, const int *__restrict__ qcur, int *__restrict__ qnext, ShadowSoA sh, WaveCounters *cnt, int cur, int bounce,                       \
       float4 *__restrict__ guide_nd, uint32_t *__restrict__ guide_c, const uint32_t *__restrict__ guide_jit, \
       GradRec rec, RecurRec rr, GatherSoA ga, int gshift, long long sh_cap, unsigned *status
-#define BC_SHADE_PASS views, n_mats, sc, ps, qcur, qnext, sh, cnt, cur, bounce, guide_nd, guide_c, guide_jit, rec, rr, ga, gshift, sh_cap, status
+#define BC_SHADE_PASS bs, views, n_mats, sc, ps, qcur, qnext, sh, cnt, cur, bounce, guide_nd, guide_c, guide_jit, rec, rr, ga, gshift, sh_cap, status
 template <bool ALT>
 __global__ void __launch_bounds__(256, 4) k_shade(BC_SHADE_ARGS) { shade_body<ALT, 256>(BC_SHADE_PASS); }
 template <bool ALT>
@@ -1054,26 +1055,24 @@ __global__ void __launch_bounds__(256) k_gather_scatter(GatherSoA ga, const Wave
     ga.perm[ga.base[ga.key[i]] + (int)ga.rank[i]] = i;
 }
 
-__global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ views, PathSoA ps, GatherSoA ga,
+__global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ views, PathState ps, GatherSoA ga,
                                                 const WaveCounters* cnt, int sorted) {
   const int n = cnt->gather;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const int i = sorted ? ga.perm[j] : j;
     const float4 P = ga.p[i], N = ga.n[i], W = ga.w[i];
     const int path = __float_as_int(W.w);
-    const PhotonView& pm = views[ps.view[path]].pm;
+    const PhotonView& pm = views[__float_as_uint(ps.ray[2 * (size_t)path].w)].pm;
     const float3 g = gather_sum(pm, make_int2(__float_as_int(P.w), __float_as_int(N.w)), f3(P.x, P.y, P.z),
                                 f3(N.x, N.y, N.z));
-    const float3 L = fma3(f3(W.x, W.y, W.z), g, f3(ps.lx[path], ps.ly[path], ps.lz[path]));
-    ps.lx[path] = L.x;
-    ps.ly[path] = L.y;
-    ps.lz[path] = L.z;
+    const float4 L = ps.L[path];
+    ps.L[path] = with_bits(fma3(f3(W.x, W.y, W.z), g, f3(L.x, L.y, L.z)), 0u);
   }
 }
 
 // ---- connect -----------------------------------------------------------------
 template <int STACK, bool SPH>
-__global__ void __launch_bounds__(128) k_connect(SceneView sv, PathSoA ps, ShadowSoA sh, WaveCounters* cnt,
+__global__ void __launch_bounds__(128) k_connect(SceneView sv, PathState ps, ShadowSoA sh, WaveCounters* cnt,
                                                  RecurRec rr, long long sh_cap, unsigned* status) {
   // entries past the queue were never written (the shading step flagged them)
   const int n = (int)min((long long)*((volatile int*)&cnt->shadow), sh_cap);
@@ -1114,9 +1113,8 @@ __global__ void __launch_bounds__(128) k_connect(SceneView sv, PathSoA ps, Shado
         const float4 c = sh.c[i];
         const int tag = __float_as_int(c.w);  // 0, or the recursive record's bounce + 1
         if (tag == 0) {
-          ps.lx[path] += c.x;
-          ps.ly[path] += c.y;
-          ps.lz[path] += c.z;
+          const float4 L = ps.L[path];
+          ps.L[path] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0.0f);
         } else {
           rr.a[(size_t)(tag - 1) * rr.cap + path].w = 1.0f;
         }
@@ -1139,7 +1137,7 @@ __device__ __forceinline__ float3 clamp_sample(float3 c, float limit) {
 // For every view the wave touches, each pixel adds its samples of the wave in
 // sample order (path = view.path_off + s * npix + p): no atomics, and the sum
 // does not depend on thread scheduling.
-__global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views, PathSoA ps,
+__global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views, PathState ps,
                              float* __restrict__ sum, float* __restrict__ sumsq, AdaptState ad, RecurRec rr) {
   const long long w0 = bs->w0;
   const long long w1 = min(bs->total, w0 + (long long)bs->cap);
@@ -1173,7 +1171,8 @@ __global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* _
       bool stop = false;
       for (int s = s_lo; s < s_hi && !stop; s++) {
         const long long i = V.path_off + (long long)s * V.npix + p - w0;
-        float3 L = f3(sld(ps.lx + i), sld(ps.ly + i), sld(ps.lz + i));
+        const float4 Lw = sld(ps.L + i);
+        float3 L = f3(Lw.x, Lw.y, Lw.z);
         if (V.integrator == BC_INTEGRATOR_RECURSIVE)  // the visible light samples, deepest vertex first
           for (int b = rr.nb[i] - 1; b >= 0; b--) {
             const float4 A = rr.a[(size_t)b * rr.cap + i];
@@ -1209,7 +1208,7 @@ __global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* _
 // linear in that albedo; Russian roulette probabilities are held fixed).
 // Per block sums in fp64 shared memory, one row of `partial` per block.
 __global__ void __launch_bounds__(256) k_gradient(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views,
-                                                  PathSoA ps, GradRec rec, GradArgs ga,
+                                                  PathState ps, GradRec rec, GradArgs ga,
                                                   const MatGPU* __restrict__ mats) {
   extern __shared__ double sg[];
   const int np3 = 3 * ga.n_params;
@@ -1218,12 +1217,14 @@ __global__ void __launch_bounds__(256) k_gradient(const BatchState* __restrict__
   const long long w0 = bs->w0;
   const int n = (int)min((long long)bs->cap, bs->total - w0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const ViewGPU& V = views[ps.view[i]];
-    const float* dp = ga.dimg + 3 * (size_t)(V.pix_off + ps.pix[i]);
+    const ViewGPU& V = views[__float_as_uint(ps.ray[2 * (size_t)i].w)];
+    const long long pix = (w0 + i - V.path_off) % V.npix;
+    const float* dp = ga.dimg + 3 * (size_t)(V.pix_off + pix);
     const float inv = 1.0f / (float)V.spp;
     const float3 dl = f3(dp[0] * inv, dp[1] * inv, dp[2] * inv);
     if (dl.x == 0.0f && dl.y == 0.0f && dl.z == 0.0f) continue;
-    const float3 Lf = f3(ps.lx[i], ps.ly[i], ps.lz[i]);
+    const float4 Lw = ps.L[i];
+    const float3 Lf = f3(Lw.x, Lw.y, Lw.z);
     const int nb = rec.nb[i];
     for (int b = 0; b < nb; b++) {
       const size_t r = (size_t)b * rec.cap + i;
@@ -1400,7 +1401,7 @@ struct RenderBuffers {
   size_t frame_px = 0;  // pixels of the frame buffers
   bcgx::DevBuf paths, shadow, queues, counters, seq, frame, table;
   bcgx::HostBuf staging;
-  bcgx::PathSoA ps{};
+  bcgx::PathState ps{};
   bcgx::ShadowSoA sh{};
   int* q[2] = {nullptr, nullptr};
   bcgx::WaveCounters* cnt = nullptr;
@@ -1539,25 +1540,20 @@ static void timing_collect(bc_context* ctx) {
 static bc_status ensure_paths(bc_context* ctx, int cap, long long sh_cap) {
   RenderBuffers* rb = ctx->rb;
   if (rb->cap < cap) {
-    size_t per = 15 * sizeof(float) + sizeof(uint32_t) + 2 * sizeof(uint64_t) + sizeof(float) + 4 * sizeof(int32_t);
-    cudaError_t e = rb->paths.ensure((size_t)cap * per + 64 * 256);
+    const size_t per = 6 * sizeof(float4) + sizeof(float2);
+    cudaError_t e = rb->paths.ensure((size_t)cap * per + 8 * 256);
     if (e == cudaSuccess) e = rb->queues.ensure((size_t)cap * 2 * sizeof(int) + 4 * 256);
     if (e != cudaSuccess) {
       rb->cap = 0;
       return cuda_status(ctx, e, "path buffers");
     }
     char* p = (char*)rb->paths.p;
-    PathSoA& s = rb->ps;
-    float** fl[] = {&s.ox, &s.oy, &s.oz, &s.dx, &s.dy, &s.dz, &s.tx, &s.ty, &s.tz, &s.lx, &s.ly, &s.lz, &s.px, &s.py, &s.pz};
-    for (float** f : fl) *f = carve<float>(p, cap);
-    s.prev = carve<uint32_t>(p, cap);
-    s.rs = carve<uint64_t>(p, cap);
-    s.ri = carve<uint64_t>(p, cap);
-    s.hit_t = carve<float>(p, cap);
-    s.hit_slot = carve<int32_t>(p, cap);
-    s.view = carve<int32_t>(p, cap);
-    s.pix = carve<int32_t>(p, cap);
-    s.samp = carve<int32_t>(p, cap);
+    PathState& s = rb->ps;
+    s.ray = carve<float4>(p, 2 * (size_t)cap);
+    s.st = carve<float4>(p, 2 * (size_t)cap);
+    s.L = carve<float4>(p, cap);
+    s.prevp = carve<float4>(p, cap);
+    s.hit = carve<float2>(p, cap);
     char* qq = (char*)rb->queues.p;
     rb->q[0] = carve<int>(qq, cap);
     rb->q[1] = carve<int>(qq, cap);
@@ -1773,7 +1769,7 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
     const GradRec rec = w.grad ? rb->grec : GradRec{nullptr, nullptr, nullptr, 0};
     rb->mark(st, kTimeShade);
 #define BC_SHADE_LAUNCH(KERNEL, BLOCK)                                                                         \
-  KERNEL<<<w.shade_grid, BLOCK, 0, st>>>(rb->views, ctx->ds.n_mats, sc, rb->ps, rb->q[cur], rb->q[cur ^ 1], rb->sh, \
+  KERNEL<<<w.shade_grid, BLOCK, 0, st>>>(rb->bs, rb->views, ctx->ds.n_mats, sc, rb->ps, rb->q[cur], rb->q[cur ^ 1], rb->sh, \
                                         c, cur, b, rb->guide_nd, rb->guide_c, rb->guide_jit, rec, rr, rb->ga,       \
                                         w.gshift, rb->sh_cap, ctx->d_status)
     if (w.shade_block == 128) {
