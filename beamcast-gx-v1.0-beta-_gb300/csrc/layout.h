@@ -30,7 +30,7 @@ constexpr unsigned kStatusTimeout = 2u;
 constexpr unsigned kStatusCapacity = 4u;
 constexpr unsigned kStatusBound = 8u;  // an fp32 hit classified as certain failed its fp64 test
 
-// Wide node with quantized child boxes (96 bytes, six 128-bit loads). Each
+// Wide node with quantized child boxes (96 bytes, three 32-byte sectors). Each
 // axis has a power-of-two grid anchored at (px, py, pz): a child's box on that
 // axis is [p + qlo * 2^(e-127), p + qhi * 2^(e-127)], decoded on the device with
 // round-down / round-up FMAs. The packer picks p, e and q so that every decoded

@@ -33,6 +33,10 @@ constexpr float kFarSlack = 8.0e-7f;  // > 2*gamma_3 + rounding of the scaling i
 // lane is slower than letting a few lanes wait.
 constexpr int kRefillLanes = 6;
 
+// The traversal stacks hold this many entries past STACK: a node visit checks
+// once for room, then pushes up to seven children without a branch each.
+constexpr int kStackSlack = 8;
+
 struct Ray32 {
   float ox, oy, oz;
   float dx, dy, dz;
@@ -59,6 +63,19 @@ __device__ __forceinline__ Ray32 make_ray(float ox, float oy, float oz, float dx
 // reject the box; fma(|t|, slack, t) would turn -inf into NaN, which fminf
 // ignores, and the box would be entered.
 __device__ __forceinline__ float widen(float t) { return t * (t >= 0.0f ? 1.0f + kFarSlack : 1.0f - kFarSlack); }
+
+// 32 bytes in one load (32-byte aligned). The lanes of a walk read different
+// records, so an access costs the L1 a pass per lane and line whatever its width.
+struct Word8 {
+  uint32_t v[8];
+};
+__device__ __forceinline__ Word8 ldg256(const void* p) {
+  Word8 r;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+      : "l"(p));
+  return r;
+}
 
 // 1 + b 2^-15 for byte j of word (bit pattern 0x3f80bb00, exact).
 __device__ __forceinline__ float byte_v(uint32_t word, int j) {
@@ -341,13 +358,30 @@ __device__ __forceinline__ RayPre ray_pre(const Ray32& r) {
 template <bool CONS>
 __device__ __forceinline__ void node_children_fused(const Node8* __restrict__ node, const RayPre& rp, float tmin,
                                                     float tlim, float near[8], uint32_t child[8]) {
-  const float4* p = reinterpret_cast<const float4*>(node);
-  const float4 w0 = __ldg(p + 0);
-  const uint4 c0 = __ldg(reinterpret_cast<const uint4*>(p + 1));
-  const uint4 c1 = __ldg(reinterpret_cast<const uint4*>(p + 2));
-  const uint4 qx = __ldg(reinterpret_cast<const uint4*>(p + 3));
-  const uint4 qy = __ldg(reinterpret_cast<const uint4*>(p + 4));
-  const uint4 qz = __ldg(reinterpret_cast<const uint4*>(p + 5));
+  // The render walk reads the record with three 256-bit loads instead of six
+  // 128-bit ones (512 x 512 adjoint step: k_extend 32.7 -> 32.0 ms). The exact
+  // walk keeps the narrow loads: at its 40 registers the wide ones spill
+  // (million-triangle ray cast 6.50 -> 6.89 ms).
+  float4 w0;
+  uint4 c0, c1, qx, qy, qz;
+  if (CONS) {
+    const float4* p = reinterpret_cast<const float4*>(node);
+    w0 = __ldg(p + 0);
+    c0 = __ldg(reinterpret_cast<const uint4*>(p + 1));
+    c1 = __ldg(reinterpret_cast<const uint4*>(p + 2));
+    qx = __ldg(reinterpret_cast<const uint4*>(p + 3));
+    qy = __ldg(reinterpret_cast<const uint4*>(p + 4));
+    qz = __ldg(reinterpret_cast<const uint4*>(p + 5));
+  } else {
+    const Word8 r0 = ldg256(node), r1 = ldg256(reinterpret_cast<const char*>(node) + 32),
+                r2 = ldg256(reinterpret_cast<const char*>(node) + 64);
+    w0 = make_float4(__uint_as_float(r0.v[0]), __uint_as_float(r0.v[1]), __uint_as_float(r0.v[2]), __uint_as_float(r0.v[3]));
+    c0 = make_uint4(r0.v[4], r0.v[5], r0.v[6], r0.v[7]);
+    c1 = make_uint4(r1.v[0], r1.v[1], r1.v[2], r1.v[3]);
+    qx = make_uint4(r1.v[4], r1.v[5], r1.v[6], r1.v[7]);
+    qy = make_uint4(r2.v[0], r2.v[1], r2.v[2], r2.v[3]);
+    qz = make_uint4(r2.v[4], r2.v[5], r2.v[6], r2.v[7]);
+  }
   const uint32_t meta = __float_as_uint(w0.w);
   const int nchild = (int)(meta >> 24);
   const float bx = __uint_as_float((meta & 0xffu) << 23) * rp.ivx * 32768.0f;
@@ -496,6 +530,7 @@ __device__ __forceinline__ uint32_t order_children(float nr[8], uint32_t ch[8], 
       }
     }
     if (hits == 0) return walker.pop(tlim);
+    walker.room(status);
     cswap(n0, c0, n1, c1);
     cswap(n2, c2, n3, c3);
     cswap(n0, c0, n2, c2);
@@ -506,19 +541,18 @@ __device__ __forceinline__ uint32_t order_children(float nr[8], uint32_t ch[8], 
       const float nk = k == 3 ? n3 : (k == 2 ? n2 : n1);
       const uint32_t ck = k == 3 ? c3 : (k == 2 ? c2 : c1);
       if (nk != kInf) {
-        if (sp < STACK) st[sp++] = make_uint2(ck, __float_as_uint(nk));
-        else atomicOr(status, kStatusStackOverflow);
+        walker.push(ck, nk);
       }
     }
     return c0;
   }
   sort8(nr, ch);
   if (nr[0] == kInf) return walker.pop(tlim);
+  walker.room(status);
 #pragma unroll
   for (int k = 7; k >= 1; k--) {
     if (nr[k] != kInf) {
-      if (sp < STACK) st[sp++] = make_uint2(ch[k], __float_as_uint(nr[k]));
-      else atomicOr(status, kStatusStackOverflow);
+      walker.push(ch[k], nr[k]);
     }
   }
   return ch[0];
@@ -549,7 +583,7 @@ __device__ __forceinline__ bool leaf_phase_now(uint32_t pending) {
 // current ray has finished (stack empty, or leaf.done).
 template <int STACK, int VOTE = 8>
 struct Walker {
-  uint2 st[STACK];
+  uint2 st[STACK + kStackSlack];
   int sp;
   uint32_t ref;
   uint32_t pending;
@@ -566,6 +600,15 @@ struct Walker {
       if (__uint_as_float(e.y) <= tlim) return e.x;
     }
     return kEnd;
+  }
+  __device__ __forceinline__ void push(uint32_t c, float n) {
+    st[sp++] = make_uint2(c, __float_as_uint(n));
+  }
+  __device__ __forceinline__ void room(unsigned* status) {
+    if (sp > STACK) {
+      sp = STACK;
+      atomicOr(status, kStatusStackOverflow);
+    }
   }
   template <class Leaf>
   __device__ __forceinline__ bool step(const SceneView& sv, const Ray32& r, Leaf& leaf, unsigned* status) {
@@ -600,7 +643,7 @@ struct Walker {
 // fine for rendering, not for the exact ray cast.
 template <int STACK, int VOTE = 8>
 struct FastWalker {
-  uint2 st[STACK];
+  uint2 st[STACK + kStackSlack];
   int sp;
   uint32_t ref;
   uint32_t pending;
@@ -617,6 +660,15 @@ struct FastWalker {
       if (__uint_as_float(e.y) <= tlim) return e.x;
     }
     return kEnd;
+  }
+  __device__ __forceinline__ void push(uint32_t c, float n) {
+    st[sp++] = make_uint2(c, __float_as_uint(n));
+  }
+  __device__ __forceinline__ void room(unsigned* status) {
+    if (sp > STACK) {
+      sp = STACK;
+      atomicOr(status, kStatusStackOverflow);
+    }
   }
   template <class Leaf>
   __device__ __forceinline__ bool step(const SceneView& sv, const Ray32& r, Leaf& leaf, unsigned* status) {
