@@ -366,13 +366,13 @@ bc_status bc_raycast_device(bc_context* ctx, const float* d_rays, int64_t n, flo
     order = ctx->d_order[2].p;
   }
   void* rec = nullptr;
-  if (ctx->raycast_split && ctx->raycast_exact && n > 0) {
+  if (ctx->raycast_split && ctx->raycast_exact && !cast_in_groups(ctx->ds, n, false)) {
     cudaError_t e = ctx->d_rec[2].ensure(exact_record_bytes(n));
     if (e) return cuda_status(ctx, e, "ray-cast record buffers");
     rec = ctx->d_rec[2].p;
   }
   cudaError_t e = launch_raycast_closest(ctx->ds, (const float4*)d_rays, n, d_t_out, d_prim_out,
-                                         ctx->d_status_async, ctx->d_work + 2, ctx->raycast_variant, order, rec, st);
+                                         ctx->d_status_async, ctx->d_work + 2, ctx->raycast_variant, ctx->raycast_split != 0, order, rec, st);
   if (e == cudaSuccess) e = raise_test_status(ctx, st);
   return cuda_status(ctx, e, "ray-cast launch");
 }
@@ -403,7 +403,7 @@ bc_status bc_raycast(bc_context* ctx, const float* rays, int64_t n, float* t_out
       order[k] = ctx->d_order[k].p;
     }
   void* rec[2] = {nullptr, nullptr};
-  if (ctx->raycast_split && ctx->raycast_exact)
+  if (ctx->raycast_split && ctx->raycast_exact && !cast_in_groups(ctx->ds, n, false))
     for (int k = 0; k < 2; k++) {
       if ((e = ctx->d_rec[k].ensure(exact_record_bytes(std::min(chunk, n))))) return cuda_status(ctx, e, "ray-cast record buffers");
       rec[k] = ctx->d_rec[k].p;
@@ -415,8 +415,8 @@ bc_status bc_raycast(bc_context* ctx, const float* rays, int64_t n, float* t_out
     e = cudaMemcpyAsync(dr, rays + 8 * off, (size_t)m * 32, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
       e = launch_raycast_closest(ctx->ds, dr, m, ctx->d_t.as<float>() + off, ctx->d_prim.as<int32_t>() + off,
-                                 ctx->d_status, ctx->d_work + (c & 1), ctx->raycast_variant, order[c & 1], rec[c & 1],
-                                 st);
+                                 ctx->d_status, ctx->d_work + (c & 1), ctx->raycast_variant, ctx->raycast_split != 0, order[c & 1],
+                                 rec[c & 1], st);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(t_out + off, ctx->d_t.as<float>() + off, (size_t)m * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
@@ -438,7 +438,7 @@ bc_status bc_occluded_device(bc_context* ctx, const float* d_rays, int64_t n, ui
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   void* rec = nullptr;
   void* order = nullptr;
-  if (ctx->raycast_split && n > 0) {
+  if (ctx->raycast_split && !cast_in_groups(ctx->ds, n, true)) {
     cudaError_t e = ctx->d_rec_any.ensure(any_record_bytes(n));
     if (e) return cuda_status(ctx, e, "any-hit record buffers");
     rec = ctx->d_rec_any.p;
@@ -448,7 +448,7 @@ bc_status bc_occluded_device(bc_context* ctx, const float* d_rays, int64_t n, ui
     }
   }
   cudaError_t e = launch_raycast_any(ctx->ds, (const float4*)d_rays, n, d_out, ctx->d_status_async,
-                                     ctx->raycast_variant, ctx->d_work + 3, rec, order, st);
+                                     ctx->raycast_variant, ctx->raycast_split != 0, ctx->d_work + 3, rec, order, st);
   if (e == cudaSuccess) e = raise_test_status(ctx, st);
   return cuda_status(ctx, e, "any-hit launch");
 }
@@ -470,7 +470,7 @@ bc_status bc_occluded(bc_context* ctx, const float* rays, int64_t n, uint8_t* ou
     return cuda_status(ctx, e, "any-hit buffers");
   void* rec = nullptr;
   void* order = nullptr;
-  if (ctx->raycast_split) {
+  if (ctx->raycast_split && !cast_in_groups(ctx->ds, n, true)) {
     if ((e = ctx->d_rec_any.ensure(any_record_bytes(n)))) return cuda_status(ctx, e, "any-hit record buffers");
     rec = ctx->d_rec_any.p;
     if (ctx->raycast_sort && n >= kMinOrderedRays && n < (int64_t(1) << 31)) {
@@ -481,7 +481,7 @@ bc_status bc_occluded(bc_context* ctx, const float* rays, int64_t n, uint8_t* ou
   e = cudaMemcpyAsync(ctx->d_rays.p, rays, (size_t)n * 32, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess)
     e = launch_raycast_any(ctx->ds, ctx->d_rays.as<float4>(), n, ctx->d_occ.as<uint8_t>(), ctx->d_status, ctx->raycast_variant,
-                           ctx->d_work + 3, rec, order, ctx->stream);
+                           ctx->raycast_split != 0, ctx->d_work + 3, rec, order, ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, ctx->d_occ.p, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_status(ctx, e, "any hit");

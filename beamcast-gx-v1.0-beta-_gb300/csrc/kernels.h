@@ -33,18 +33,22 @@ int stack_variant(int need);
 // spatially coherent order (batches of at least kMinOrderedRays rays).
 // rec_scratch (exact_record_bytes(n) bytes, or NULL): the exact closest hit of
 // a triangle-only scene runs as separate walk and fp64 settlement passes.
-constexpr int64_t kMinOrderedRays = 65536;
+constexpr int64_t kMinOrderedRays = 1 << 20;
+// Small batches of a triangle-only scene are cast by groups of eight lanes in
+// one launch without scratch, where `split` (bc_set_option "raycast_split") allows.
+constexpr int64_t kGroupRaysClosest = 32768, kGroupRaysAny = 65536;
+bool cast_in_groups(const DeviceScene& s, int64_t n, bool any);
 size_t ray_order_bytes(int64_t n);
 size_t exact_record_bytes(int64_t n);
 cudaError_t launch_raycast_closest(const DeviceScene& s, const float4* rays, int64_t n, float* t_out,
                                    int32_t* prim_out, unsigned* status, unsigned long long* work, int variant,
-                                   void* order_scratch, void* rec_scratch, cudaStream_t st);
+                                   bool split, void* order_scratch, void* rec_scratch, cudaStream_t st);
 // Exact any hit. rec_scratch (any_record_bytes(n) bytes) and `work` (as for the
 // closest hit), or NULL: a triangle-only scene runs as walk and fp64 passes,
 // in the coherent ray order when order_scratch (ray_order_bytes(n)) is given.
 size_t any_record_bytes(int64_t n);
 cudaError_t launch_raycast_any(const DeviceScene& s, const float4* rays, int64_t n, uint8_t* out, unsigned* status,
-                               int variant, unsigned long long* work, void* rec_scratch, void* order_scratch,
-                               cudaStream_t st);
+                               int variant, bool split, unsigned long long* work, void* rec_scratch,
+                               void* order_scratch, cudaStream_t st);
 
 }  // namespace bcgx

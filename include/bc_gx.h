@@ -429,16 +429,20 @@ bc_status bc_post_process_noalloc(int32_t width, int32_t height, const float* d_
  *                        then fp64 tests of the undecided triangles of the rays
  *                        the walk could not decide (28 bytes per ray). 0: one
  *                        kernel walks and settles. Both give the same results.
+ *                        With 1, small batches of a triangle-only scene (closest
+ *                        hit up to 32,768 rays, any hit up to 65,536) are cast by
+ *                        eight lanes per ray in one launch without scratch.
  *   "raycast_minblocks"  1, 6 or 8: register budget of the one-kernel ray-cast
  *                        kernels (resident 128-thread blocks per SM the allocation
  *                        must allow).
  *   "raycast_exact"      1 (default): bc_raycast is exact as documented there;
  *                        0: plain fp32 closest hit, t = the fp32 distance, with no
  *                        exactness contract near edges and ties.
- *   "raycast_sort"       1 (default): batches of at least 65,536 rays are traced
- *                        in a spatially coherent order (origin Morton code on a
- *                        64^3 grid over the scene bounds, then direction octant);
- *                        results are returned in the caller's order either way.
+ *   "raycast_sort"       1 (default): batches of at least 1,048,576 rays that come
+ *                        in no spatial order of their own are traced in one (origin
+ *                        Morton code on a 64^3 grid over the scene bounds, then
+ *                        direction octant); results are returned in the caller's
+ *                        order either way.
  *   "photon_grid"        1 (default): a photon gather reads its cell's neighbour
  *                        list, built with the map; 0: 27 hash lookups.
  *                        Both give the same photons in the same order.

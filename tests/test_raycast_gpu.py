@@ -322,3 +322,53 @@ def test_merged_leaves_parity(gpu_ctx, orc, which):
     assert np.array_equal(merged[1], plain[1]) and np.array_equal(merged[0], plain[0])
     occ_ref, _ = ref.occluded_f32(rays)
     assert np.array_equal(occ, occ_ref)
+
+
+# Small batches are cast by groups of eight lanes per ray (one, two or four groups
+# to a warp by size); the sizes are the edges of those rules and of the walk's.
+@pytest.mark.parametrize("which", ["random", "stacked", "edge"])
+@pytest.mark.parametrize("n", [1, 9, 4096, 4097, 6145, 8193, 32768, 32769, 65536, 65537])
+def test_small_batches_parity(gpu_ctx, orc, which, n):
+    if which == "random":
+        spec = scenes.random_triangles(20_000, seed=scenes.SEED_TRIS + 9)
+        rays = scenes.random_rays(n, seed=18)
+    elif which == "stacked":  # more contenders than a group's lanes hold, and thousands of exact ties
+        spec = _stacked_triangles()
+        rays = scenes.random_rays(n, seed=19)
+    else:
+        spec, _, _ = scenes.cornell_box()
+        rng = np.random.default_rng(4)
+        rays = scenes.random_rays(n, seed=20)
+        rays[:, 0:3] = rng.uniform(-1, 1, (n, 3))
+        rays[::3, 4 + rng.integers(3)] = 0.0
+        rays[1::7, 1] = -1.0
+        rays[2::11, 7] = 0.4  # short rays
+    gpu_ctx.upload(scenes.to_scene(spec))
+    ref = orc.OracleScene.from_spec(spec)
+    _check(gpu_ctx, ref, rays)
+    occ_ref, _ = ref.occluded_f32(rays)
+    assert np.array_equal(gpu_ctx.occluded(rays), occ_ref)
+
+
+@pytest.mark.parametrize("order", ["random", "one origin", "by place", "mixed"])
+def test_ray_order_probe_changes_no_result(gpu_ctx, order):
+    """Batches of 2^20 rays and more are ordered when their own order is incoherent;
+    either way each ray gets its answer."""
+    n = (1 << 20) + 77
+    rays = scenes.random_rays(n, seed=21)
+    if order == "one origin":
+        rays[:, 0:3] = 0.5
+    elif order == "by place":
+        rays[:, 0:3] = rays[np.lexsort(np.floor(rays[:, 0:3] * 48).T), 0:3]
+    elif order == "mixed":
+        rays[: n // 2, 0:3] = 0.25
+    gpu_ctx.upload(scenes.to_scene(scenes.random_triangles(20_000, seed=scenes.SEED_TRIS + 10)))
+    t1, p1 = gpu_ctx.raycast(rays)
+    o1 = gpu_ctx.occluded(rays)
+    try:
+        gpu_ctx.set_option("raycast_sort", 0)
+        t0, p0 = gpu_ctx.raycast(rays)
+        o0 = gpu_ctx.occluded(rays)
+    finally:
+        gpu_ctx.set_option("raycast_sort", 1)
+    assert np.array_equal(p0, p1) and np.array_equal(t0, t1) and np.array_equal(o0, o1)
