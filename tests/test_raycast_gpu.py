@@ -372,3 +372,36 @@ def test_ray_order_probe_changes_no_result(gpu_ctx, order):
     finally:
         gpu_ctx.set_option("raycast_sort", 1)
     assert np.array_equal(p0, p1) and np.array_equal(t0, t1) and np.array_equal(o0, o1)
+
+
+@pytest.mark.parametrize("offset", [0.0, 300.0])
+def test_sphere_edges_parity(gpu_ctx, orc, offset):
+    """Spheres of very different sizes, overlapping, far from the origin: rays that graze
+    them, start inside or on them, or end between their two roots."""
+    rng = np.random.default_rng(17)
+    n, k = 400, 24_000
+    centers = rng.uniform(-4, 4, (n, 3)) + offset
+    radii = 10.0 ** rng.uniform(-3, 0.3, n)
+    spec = scenes.SceneSpec(name="spheres", bvh_mode="SAH", bvh_bins=16, bvh_leaf=4)
+    m = spec.material(scenes.Material(scenes.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    for c, r in zip(centers, radii):
+        spec.sphere(c, r, m)
+    spec.sphere((offset, offset - 1002.0, offset), 1000.0, m)
+    i = rng.integers(0, n, k)
+    d = rng.normal(size=(k, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    side = np.cross(d, rng.normal(size=(k, 3)))
+    side /= np.linalg.norm(side, axis=1, keepdims=True)
+    back = rng.uniform(0.0, 6.0, (k, 1))
+    miss = radii[i] * rng.choice([1.0, 1.0 - 1e-6, 1.0 + 1e-6, 0.3, 0.999], k)  # tangent and near-tangent rays
+    o = centers[i] + side * miss[:, None] - d * back
+    o[::5] = centers[i[::5]] + d[::5] * radii[i[::5], None] * rng.choice([1.0, 0.5, 0.0], (len(o[::5]), 1))
+    rays = np.empty((k, 8), np.float32)
+    rays[:, 0:3], rays[:, 3], rays[:, 4:7], rays[:, 7] = o, 1e-4, d * rng.choice([1.0, 0.01, 30.0], (k, 1)), 1e30
+    rays[::7, 7] = rng.uniform(0.0, 6.0, len(rays[::7]))
+    rays[3::7, 3] = rng.uniform(0.0, 6.0, len(rays[3::7]))
+    gpu_ctx.upload(scenes.to_scene(spec))
+    ref = orc.OracleScene.from_spec(spec)
+    _check(gpu_ctx, ref, rays)
+    occ_ref, _ = ref.occluded_f32(rays)
+    assert np.array_equal(gpu_ctx.occluded(rays), occ_ref)
