@@ -350,7 +350,7 @@ __global__ void k_photon_runs(PhotonView pm, const PhotonGrid* __restrict__ grid
 }
 
 __global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, const int* __restrict__ runs,
-                               int2* __restrict__ list, float4* __restrict__ lpos, int cap) {
+                               int2* __restrict__ list, float4* __restrict__ lent, int cap) {
   const int gx = grid->dim[0];
   if (gx == 0) return;
   const int gy = grid->dim[1], gz = grid->dim[2];
@@ -378,8 +378,11 @@ __global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, con
       if (u < 0) continue;
       const int2 sp = pm.span[u];
       for (int k = sp.x; k < sp.x + sp.y; k++) {
-        const float4 P = pm.pos[k];
-        lpos[at++] = make_float4(P.x, P.y, P.z, __int_as_float(k));
+        const float4 P = pm.pos[k], N = pm.nrm[k], F = pm.flux[k];
+        float4* e = lent + 3 * (size_t)at++;
+        e[0] = make_float4(P.x, P.y, P.z, N.x);
+        e[1] = make_float4(N.y, N.z, F.x, F.y);
+        e[2] = make_float4(F.z, 0.0f, 0.0f, 0.0f);
       }
     }
   }
@@ -473,7 +476,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
                        ((np * 8 + 255) / 256) * 256 * 2 + ((p2 * 8 + 255) / 256) * 256 +
                        ((p2 * 4 + 255) / 256) * 256 + ((np * 8 + 255) / 256) * 256 + ((tsize * 4 + 255) / 256) * 256 +
                        256 + (((size_t)max_cells * 4 + 255) / 256) * 256 + (((size_t)max_cells * 8 + 255) / 256) * 256 +
-                       (max_cells ? ((size_t)list_cap * 16 + 255) / 256 * 256 : 0);
+                       (max_cells ? ((size_t)list_cap * 48 + 255) / 256 * 256 : 0);
   cudaError_t e = cudaMalloc(&p.mem, bytes);
   if (e) {
     p.mem = nullptr;
@@ -499,7 +502,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   PhotonGrid* grid = take<PhotonGrid>(c, 1);
   int* runs = max_cells ? take<int>(c, (size_t)max_cells) : nullptr;
   int2* list = max_cells ? take<int2>(c, (size_t)max_cells) : nullptr;
-  float4* lpos = max_cells ? take<float4>(c, (size_t)list_cap) : nullptr;
+  float4* lent = max_cells ? take<float4>(c, 3 * (size_t)list_cap) : nullptr;
   p.pos_u = pos_u;
   p.nrm_u = nrm_u;
   p.flux_u = flux_u;
@@ -542,6 +545,8 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   }
   PhotonView hv{};
   hv.pos = pos;
+  hv.nrm = nrm;
+  hv.flux = flux;
   hv.ukey = ukey;
   hv.span = span;
   hv.table = table;
@@ -549,7 +554,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   if (!e && list) {
     const int blocks = (int)std::min<long long>(1024, (max_cells + 255) / 256);
     k_photon_runs<<<blocks, 256, 0, st>>>(hv, grid, runs);
-    k_photon_lists<<<(int)std::min<long long>(4096, (max_cells + 63) / 64), 64, 0, st>>>(hv, grid, runs, list, lpos,
+    k_photon_lists<<<(int)std::min<long long>(4096, (max_cells + 63) / 64), 64, 0, st>>>(hv, grid, runs, list, lent,
                                                                                         list_cap);
     e = cudaGetLastError();
   }
@@ -569,7 +574,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   p.view.pir2 = (float)(M_PI * radius * radius);
   p.view.grid = list ? grid : nullptr;
   p.view.list = list;
-  p.view.lpos = lpos;
+  p.view.lent = lent;
   return BC_OK;
 }
 

@@ -38,7 +38,7 @@ struct PhotonView {
   float cell, r2, pir2;             // cell size (= radius), radius^2, pi radius^2
   const PhotonGrid* grid;           // null: no neighbour lists
   const int2* list;                 // per cell of the box: (first entry, entries); first < 0: none, use the hash
-  const float4* lpos;               // list entries: position, sorted photon index bits
+  const float4* lent;               // list entries, three float4 each: (position, normal x) (normal y z, flux x y) (flux z)
 };
 
 // photonCellKey (renderer.go:1636-1639): the int64 products wrap, as unsigned products do.
@@ -65,15 +65,13 @@ __device__ __forceinline__ int photon_cell_lookup(const PhotonView& pm, unsigned
 
 // One candidate of a gather (renderer.go:1745-1752): counted when it is within
 // the radius of p and faces n; true once kGatherMax photons are counted.
-__device__ __forceinline__ bool gather_photon(const PhotonView& pm, float4 P, int i, float3 p, float3 n, float3& sum,
+__device__ __forceinline__ bool gather_photon(float r2, float3 P, float3 N, float3 F, float3 p, float3 n, float3& sum,
                                               int& count) {
-  const float3 d = f3(P.x, P.y, P.z) - p;
-  if (dot3(d, d) > pm.r2) return false;
-  const float4 N = __ldg(pm.nrm + i);
-  const float nd = dot3(f3(N.x, N.y, N.z), n);
+  const float3 d = P - p;
+  if (dot3(d, d) > r2) return false;
+  const float nd = dot3(N, n);
   if (nd <= 0.05f) return false;
-  const float4 F = __ldg(pm.flux + i);
-  sum = fma3(f3(F.x, F.y, F.z), nd, sum);
+  sum = fma3(F, nd, sum);
   return ++count >= kGatherMax;
 }
 
@@ -81,9 +79,8 @@ __device__ __forceinline__ bool gather_photon(const PhotonView& pm, float4 P, in
 // (dz, dy, dx) order, each cell's photons in append order; a key shared by two
 // of the cells is visited twice, as the reference's map lookups do.
 // A cell's neighbour list holds exactly those photons in exactly that order, so
-// a gather is one lookup (gather_run) and one contiguous run (gather_sum), and
-// only the candidates within the radius read their normal and flux (about a
-// third).
+// a gather is one lookup (gather_run) and one contiguous run (gather_sum) whose
+// loads do not depend on what the candidates before them gave.
 
 // The run of p's cell: (first entry, entries), entries 0 where the gather is
 // zero; first < 0: no list, the hash serves. A point more than one cell outside
@@ -106,16 +103,15 @@ __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, flo
   float3 sum = f3(0.0f, 0.0f, 0.0f);
   int count = 0;
   if (run.x >= 0) {
-    const float4* e = pm.lpos + run.x;
-    for (int i = 0; i < run.y; i += 4) {  // four positions in flight; the last group reads the last entry again
-      float4 P[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) P[k] = __ldg(e + min(i + k, run.y - 1));
-      bool full = false;
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (!full && i + k < run.y) full = gather_photon(pm, P[k], __float_as_int(P[k].w), p, n, sum, count);
-      if (full) break;
+    const float4* e = pm.lent + 3 * (size_t)run.x;
+    for (int i = 0; i < run.y; i += 2) {  // two candidates in flight; the last pair may read the last entry twice
+      const float4* e1 = e + 3 * (size_t)min(i + 1, run.y - 1);
+      const float4 a0 = __ldg(e + 3 * (size_t)i), a1 = __ldg(e + 3 * (size_t)i + 1), a2 = __ldg(e + 3 * (size_t)i + 2);
+      const float4 b0 = __ldg(e1), b1 = __ldg(e1 + 1), b2 = __ldg(e1 + 2);
+      if (gather_photon(pm.r2, f3(a0.x, a0.y, a0.z), f3(a0.w, a1.x, a1.y), f3(a1.z, a1.w, a2.x), p, n, sum, count)) break;
+      if (i + 1 < run.y &&
+          gather_photon(pm.r2, f3(b0.x, b0.y, b0.z), f3(b0.w, b1.x, b1.y), f3(b1.z, b1.w, b2.x), p, n, sum, count))
+        break;
     }
   } else {
     const long long cx = (long long)floorf(p.x / pm.cell);
@@ -128,8 +124,10 @@ __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, flo
           const int u = photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
           if (u < 0) continue;
           const int2 sp = __ldg(pm.span + u);
-          for (int i = sp.x; i < sp.x + sp.y && !full; i++)
-            full = gather_photon(pm, __ldg(pm.pos + i), i, p, n, sum, count);
+          for (int i = sp.x; i < sp.x + sp.y && !full; i++) {
+            const float4 P = __ldg(pm.pos + i), N = __ldg(pm.nrm + i), F = __ldg(pm.flux + i);
+            full = gather_photon(pm.r2, f3(P.x, P.y, P.z), f3(N.x, N.y, N.z), f3(F.x, F.y, F.z), p, n, sum, count);
+          }
         }
   }
   if (count == 0) return f3(0.0f, 0.0f, 0.0f);

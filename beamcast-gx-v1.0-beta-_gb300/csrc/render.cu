@@ -88,20 +88,23 @@ struct RecurRec {
   int cap;
 };
 
-// Photon gathers of one bounce. The shading step lists the diffuse vertices of
-// photon views whose cell has photons; k_gather adds their photon radiance.
-// Sorted by the photon run, the lanes of a warp read the same candidates.
-constexpr int kGatherBins = 1 << 16;
+// Photon gathers of one bounce. The shading step records the diffuse vertices of
+// photon views whose cell has photons (by queue position) and lists them;
+// k_gather adds their photon radiance. Sorted by the photon run, the lanes of a
+// warp read the same candidates.
+constexpr int kGatherBins = 1 << 16, kGatherScan = 1024;  // bins, bins per scan block
 constexpr int kGatherSortPaths = 1 << 20;  // waves of at least this many paths sort their gathers
 struct GatherSoA {
-  float4* p;       // point, first list entry
+  float4* p;       // by queue position: point, first list entry
   float4* n;       // facing normal, list entries
   float4* w;       // throughput at the vertex, path slot
-  uint32_t* key;   // sort bin (kGatherBins of them)
-  uint32_t* rank;  // rank within the bin
-  int32_t* perm;   // sorted order
+  int32_t* list;   // queue positions with a gather
+  uint32_t* key;   // their sort bins
+  uint32_t* rank;  // and ranks within the bin
+  int32_t* perm;   // queue positions in sorted order
   int* bins;       // [kGatherBins] zero between bounces
-  int* base;       // [kGatherBins] first place of each bin
+  int* base;       // [kGatherBins] first place of each bin within its scan block
+  int* totals;     // [kGatherBins / kGatherScan] entries of each scan block
 };
 
 // Device counters of a wave. cur/next alternate between [0] and [1].
@@ -566,9 +569,14 @@ struct VertexOut {
   float4 so, sd, scon;  // shadow ray: origin + tmax, direction + scene root, contribution
   int rec_m;
   float3 rec_v;
-  bool gather;         // photon gather to do (DEFER), at point gp with normal gn, weight gw
-  float3 gp, gn, gw;
-  int2 grun;
+  bool gather;         // photon gather to do (recorded at the vertex's queue position), its sort key
+  uint32_t gkey;
+};
+
+// Where a vertex records its photon gather.
+struct GatherOut {
+  const GatherSoA& ga;
+  int idx, path, shift;
 };
 
 // Guide outputs of a path's first vertex (sample 0 only).
@@ -657,13 +665,14 @@ __device__ __forceinline__ int sample_direct(const ViewGPU& wp, const ShadeScene
 // (1763-1831: a photon gather at diffuse vertices, emitters without an MIS
 // weight), for a path whose extension ray hit `slot` at fp32 distance t
 // (slot < 0: miss). Updates s.L / s.tp and, when the path continues, its next
-// ray (store_continuation). ALT: the batch has views of the other integrators
-// (the path-only kernels compile without their code). DEFER: photon gathers are
-// left to the caller (VertexOut.gather).
-template <bool ALT, bool DEFER, class P>
+// ray (store_continuation). MODE: the integrators the batch's views use, so that
+// a kernel carries no other's code. `go`: where a photon
+// gather is recorded (null: done in place).
+constexpr int kModePath = 0, kModePhoton = 1, kModeAll = 2;
+template <int MODE, class P>
 __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, const ShadeScene& sc, P& s, float t,
                                              int slot, int bounce, const GuideOut& gd, VertexOut& out,
-                                             bool want_rec) {
+                                             bool want_rec, const GatherOut* go) {
   out.alive = false;
   out.shadow = false;
   out.rec_m = -1;
@@ -689,7 +698,7 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
       if (gd.px >= 0) write_guides(gd, N, t, d, m);
       if (kind == BC_MAT_EMISSIVE) {
         float w = 1.0f;
-        if ((!ALT || wp.integrator == BC_INTEGRATOR_PATH) && wp.mis && (flags & 1u)) {  // 0 for triangles
+        if ((MODE == kModePath || wp.integrator == BC_INTEGRATOR_PATH) && wp.mis && (flags & 1u)) {  // 0 for triangles
           float lpdf = 0.0f;
           if (S.sphere) {
             const int prim = __ldg(sc.sv.slot_prim + slot);
@@ -706,13 +715,16 @@ __device__ __forceinline__ void shade_vertex(const ViewGPU& wp, int n_mats, cons
         if (kind == BC_MAT_DIFFUSE) {
           out.rec_m = m;
           if (want_rec) out.rec_v = s.get_L();  // everything added from here on carries this albedo once more
-          if (ALT && wp.integrator == BC_INTEGRATOR_PHOTON) {
-            if (DEFER) {
-              out.grun = gather_run(wp.pm, p);
-              out.gather = out.grun.x < 0 || out.grun.y > 0;  // else nothing to add
-              out.gp = p;
-              out.gn = N;
-              out.gw = tp;
+          if (MODE != kModePath && wp.integrator == BC_INTEGRATOR_PHOTON) {
+            if (go) {
+              const int2 run = gather_run(wp.pm, p);
+              if (run.x < 0 || run.y > 0) {  // else nothing to add
+                out.gather = true;
+                out.gkey = run.x < 0 ? kGatherBins - 1u : min((uint32_t)run.x >> go->shift, kGatherBins - 1u);
+                go->ga.p[go->idx] = with_bits(p, (uint32_t)run.x);
+                go->ga.n[go->idx] = with_bits(N, (uint32_t)run.y);
+                go->ga.w[go->idx] = with_bits(tp, (uint32_t)go->path);
+              }
             } else {
               s.add_L(tp, photon_gather(wp.pm, p, N));
             }
@@ -894,7 +906,7 @@ __device__ __forceinline__ void unwind_recursive(const ViewGPU& wp, const ShadeS
   rr.nb[path] = last + 1;
 }
 
-template <bool ALT, int BLOCK>
+template <int MODE, int BLOCK>
 __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
                                                const ViewGPU* __restrict__ views, int n_mats, ShadeScene sc,
                                                PathState ps, const int* __restrict__ qcur, int* __restrict__ qnext,
@@ -916,7 +928,7 @@ __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
     out.shadow = false;
     out.gather = false;
     if (path >= 0) {
-      RecPath<!ALT> s(ps, path);
+      RecPath<MODE != kModeAll> s(ps, path);
       const ViewGPU& wp = views[s.view];
       GuideOut gd{guide_nd, guide_c, guide_jit, -1};
       if (bounce == 0 && wp.want_guides) {
@@ -926,12 +938,13 @@ __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
       const float2 hit = __ldcs(ps.hit + idx);
       const float hit_t = hit.x;
       const int hit_slot = __float_as_int(hit.y);
-      if (ALT && wp.integrator == BC_INTEGRATOR_RECURSIVE) {
+      if (MODE == kModeAll && wp.integrator == BC_INTEGRATOR_RECURSIVE) {
         const bool ended = shade_recursive(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, rr, path);
         out.alive = !ended;
         if (ended) unwind_recursive(wp, sc, s.rng, rr, path, bounce, sh, cnt, sh_cap, status);
       } else {
-        shade_vertex<ALT, true>(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, out, rec.m != nullptr);
+        const GatherOut go{ga, idx, path, gshift};
+        shade_vertex<MODE>(wp, n_mats, sc, s, hit_t, hit_slot, bounce, gd, out, rec.m != nullptr, &go);
       }
       s.flush_L();
       if (rec.m) {
@@ -954,13 +967,11 @@ __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
         atomicOr(status, kStatusCapacity);
       }
     }
-    if (ALT) {  // at most one gather per path and bounce: the queue has a slot for each
+    if (MODE != kModePath) {  // at most one gather per path and bounce: the list has a place for each
       const int qg = warp_reserve(&cnt->gather, out.gather);
       if (out.gather) {
-        ga.p[qg] = make_float4(out.gp.x, out.gp.y, out.gp.z, __int_as_float(out.grun.x));
-        ga.n[qg] = make_float4(out.gn.x, out.gn.y, out.gn.z, __int_as_float(out.grun.y));
-        ga.w[qg] = make_float4(out.gw.x, out.gw.y, out.gw.z, __int_as_float(path));
-        ga.key[qg] = out.grun.x < 0 ? kGatherBins - 1u : min((uint32_t)out.grun.x >> gshift, kGatherBins - 1u);
+        ga.list[qg] = idx;
+        ga.key[qg] = out.gkey;
       }
     }
   }
@@ -976,10 +987,10 @@ __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
       float4 *__restrict__ guide_nd, uint32_t *__restrict__ guide_c, const uint32_t *__restrict__ guide_jit, \
       GradRec rec, RecurRec rr, GatherSoA ga, int gshift, long long sh_cap, unsigned *status
 #define BC_SHADE_PASS bs, views, n_mats, sc, ps, qcur, qnext, sh, cnt, cur, bounce, guide_nd, guide_c, guide_jit, rec, rr, ga, gshift, sh_cap, status
-template <bool ALT>
-__global__ void __launch_bounds__(256, 4) k_shade(BC_SHADE_ARGS) { shade_body<ALT, 256>(BC_SHADE_PASS); }
-template <bool ALT>
-__global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_body<ALT, 128>(BC_SHADE_PASS); }
+template <int MODE>
+__global__ void __launch_bounds__(256, 4) k_shade(BC_SHADE_ARGS) { shade_body<MODE, 256>(BC_SHADE_PASS); }
+template <int MODE>
+__global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_body<MODE, 128>(BC_SHADE_PASS); }
 #undef BC_SHADE_ARGS
 #undef BC_SHADE_PASS
 
@@ -1007,59 +1018,60 @@ __global__ void __launch_bounds__(256) k_gather_count(GatherSoA ga, const WaveCo
   }
 }
 
-// Exclusive scan of the bins (one block), which are cleared for the next bounce.
-__global__ void __launch_bounds__(1024) k_gather_scan(GatherSoA ga) {
-  __shared__ int wsum[32];
+// Exclusive scan of kGatherScan bins per block; the bins are cleared for the next bounce.
+__global__ void __launch_bounds__(256) k_gather_scan(GatherSoA ga) {
+  __shared__ int wsum[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int carry = 0;
-  for (int b0 = 0; b0 < kGatherBins; b0 += 8192) {
-    int v[8], s = 0;
-    int4* src = reinterpret_cast<int4*>(ga.bins + b0) + 2 * threadIdx.x;
-    const int4 x = src[0], y = src[1];
-    src[0] = make_int4(0, 0, 0, 0);
-    src[1] = make_int4(0, 0, 0, 0);
-    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int c = v[k];
-      v[k] = s;
-      s += c;
-    }
-    int inc = s;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int z = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += z;
-    }
-    if (lane == 31) wsum[w] = inc;
-    __syncthreads();
-    int below = carry, all = 0;
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-      const int c = wsum[k];
-      if (k < w) below += c;
-      all += c;
-    }
-    below += inc - s;
-    int4* dst = reinterpret_cast<int4*>(ga.base + b0) + 2 * threadIdx.x;
-    dst[0] = make_int4(below + v[0], below + v[1], below + v[2], below + v[3]);
-    dst[1] = make_int4(below + v[4], below + v[5], below + v[6], below + v[7]);
-    carry += all;
-    __syncthreads();
+  int4* src = reinterpret_cast<int4*>(ga.bins + kGatherScan * blockIdx.x) + threadIdx.x;
+  const int4 x = *src;
+  *src = make_int4(0, 0, 0, 0);
+  const int s = x.x + x.y + x.z + x.w;
+  int inc = s;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int z = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += z;
   }
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  int below = inc - s, all = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int c = wsum[k];
+    if (k < w) below += c;
+    all += c;
+  }
+  reinterpret_cast<int4*>(ga.base + kGatherScan * blockIdx.x)[threadIdx.x] =
+      make_int4(below, below + x.x, below + x.x + x.y, below + x.x + x.y + x.z);
+  if (threadIdx.x == 0) ga.totals[blockIdx.x] = all;
 }
 
 __global__ void __launch_bounds__(256) k_gather_scatter(GatherSoA ga, const WaveCounters* cnt) {
+  constexpr int kBlocks = kGatherBins / kGatherScan;
+  static_assert(kBlocks == 64, "two scan blocks per lane");
+  __shared__ int first[kBlocks];  // entries before each scan block
+  if (threadIdx.x < 32) {
+    const int a = ga.totals[2 * threadIdx.x], b = ga.totals[2 * threadIdx.x + 1];
+    int inc = a + b;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int z = __shfl_up_sync(0xffffffffu, inc, o);
+      if ((int)threadIdx.x >= o) inc += z;
+    }
+    first[2 * threadIdx.x] = inc - a - b;
+    first[2 * threadIdx.x + 1] = inc - b;
+  }
+  __syncthreads();
   const int n = cnt->gather;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    ga.perm[ga.base[ga.key[i]] + (int)ga.rank[i]] = i;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t k = ga.key[i];
+    ga.perm[first[k / kGatherScan] + ga.base[k] + (int)ga.rank[i]] = ga.list[i];
+  }
 }
 
 __global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ views, PathState ps, GatherSoA ga,
-                                                const WaveCounters* cnt, int sorted) {
+                                                const WaveCounters* cnt, const int32_t* __restrict__ order) {
   const int n = cnt->gather;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const int i = sorted ? ga.perm[j] : j;
+    const int i = order[j];
     const float4 P = ga.p[i], N = ga.n[i], W = ga.w[i];
     const int path = __float_as_int(W.w);
     const PhotonView& pm = views[__float_as_uint(ps.ray[2 * (size_t)path].w)].pm;
@@ -1169,19 +1181,28 @@ __global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* _
       float3 acc = f3(sp[0], sp[1], sp[2]);
       float3 acc2 = qp ? f3(qp[0], qp[1], qp[2]) : f3(0, 0, 0);
       bool stop = false;
-      for (int s = s_lo; s < s_hi && !stop; s++) {
-        const long long i = V.path_off + (long long)s * V.npix + p - w0;
-        const float4 Lw = sld(ps.L + i);
-        float3 L = f3(Lw.x, Lw.y, Lw.z);
-        if (V.integrator == BC_INTEGRATOR_RECURSIVE)  // the visible light samples, deepest vertex first
-          for (int b = rr.nb[i] - 1; b >= 0; b--) {
-            const float4 A = rr.a[(size_t)b * rr.cap + i];
-            if (A.w == 1.0f) L = L + f3(A.x, A.y, A.z);
+      for (int s0 = s_lo; s0 < s_hi && !stop; s0 += 4) {  // four samples' loads in flight
+        float4 Lw[4];
+        const long long i0 = V.path_off + (long long)s0 * V.npix + p - w0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (s0 + k < s_hi) Lw[k] = sld(ps.L + i0 + (long long)k * V.npix);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (s0 + k >= s_hi || stop) break;
+          float3 L = f3(Lw[k].x, Lw[k].y, Lw[k].z);
+          if (V.integrator == BC_INTEGRATOR_RECURSIVE) {  // the visible light samples, deepest vertex first
+            const long long i = i0 + (long long)k * V.npix;
+            for (int b = rr.nb[i] - 1; b >= 0; b--) {
+              const float4 A = rr.a[(size_t)b * rr.cap + i];
+              if (A.w == 1.0f) L = L + f3(A.x, A.y, A.z);
+            }
           }
-        const float3 c = clamp_sample(L, V.clamp);
-        acc = acc + c;
-        acc2 = fma3(c, c, acc2);
-        if (V.adaptive) stop = adaptive_step(V, c, &an, &sl, &ssl);
+          const float3 c = clamp_sample(L, V.clamp);
+          acc = acc + c;
+          acc2 = fma3(c, c, acc2);
+          if (V.adaptive) stop = adaptive_step(V, c, &an, &sl, &ssl);
+        }
       }
       if (V.adaptive) {
         ad.n[V.pix_off + p] = stop ? (an | kPixDone) : an;
@@ -1298,7 +1319,7 @@ __global__ void k_finish_views(const ViewGPU* __restrict__ views, int n_views, c
 // one-view-per-launch form the wave engine is measured against. Shadow rays are
 // traced in place; a lane idles once its path ends until the warp's longest
 // path of that sample is done.
-template <int STACK, bool SPH, bool ALT>
+template <int STACK, bool SPH, int MODE>
 __global__ void __launch_bounds__(128) k_render_plain(const ViewGPU* __restrict__ views, int v, int n_mats,
                                                       ShadeScene sc, const float4* __restrict__ seq,
                                                       float* __restrict__ sum, float* __restrict__ sumsq,
@@ -1337,7 +1358,7 @@ __global__ void __launch_bounds__(128) k_render_plain(const ViewGPU* __restrict_
         segs++;
         const GuideOut gd{guide_nd, guide_c, guide_jit, (b == 0 && guide) ? V.pix_off + p : -1};
         VertexOut out;
-        shade_vertex<ALT, false>(V, n_mats, sc, st, leaf.best_t, leaf.best_slot, b, gd, out, false);
+        shade_vertex<MODE>(V, n_mats, sc, st, leaf.best_t, leaf.best_slot, b, gd, out, false, nullptr);
         if (out.shadow) {
           shadows++;
           const Ray32 sr = make_ray(out.so.x, out.so.y, out.so.z, out.sd.x, out.sd.y, out.sd.z, 1e-4f);
@@ -1704,7 +1725,6 @@ struct WaveShape {
   bool lights;
   const GradArgs* grad;  // non-null: gradient render
   bool recursive;        // the batch has views of the recursive integrator
-  bool alt;              // the batch has views of the recursive or photon integrator
   bool photon;           // the batch has views of the photon integrator
   bool gather_sort;      // their gathers are sorted
   int gshift;            // list entry -> sort bin
@@ -1739,7 +1759,6 @@ static WaveShape wave_shape(int cap, int bounces, bool lights, const GradArgs* g
   w.lights = lights;
   w.grad = grad;
   w.recursive = false;
-  w.alt = false;
   w.photon = w.gather_sort = false;
   w.gshift = 0;
   return w;
@@ -1773,20 +1792,23 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
                                         c, cur, b, rb->guide_nd, rb->guide_c, rb->guide_jit, rec, rr, rb->ga,       \
                                         w.gshift, rb->sh_cap, ctx->d_status)
     if (w.shade_block == 128) {
-      if (w.alt) BC_SHADE_LAUNCH(k_shade_128<true>, 128);
-      else BC_SHADE_LAUNCH(k_shade_128<false>, 128);
+      if (w.recursive) BC_SHADE_LAUNCH(k_shade_128<kModeAll>, 128);
+      else if (w.photon) BC_SHADE_LAUNCH(k_shade_128<kModePhoton>, 128);
+      else BC_SHADE_LAUNCH(k_shade_128<kModePath>, 128);
     } else {
-      if (w.alt) BC_SHADE_LAUNCH(k_shade<true>, 256);
-      else BC_SHADE_LAUNCH(k_shade<false>, 256);
+      if (w.recursive) BC_SHADE_LAUNCH(k_shade<kModeAll>, 256);
+      else if (w.photon) BC_SHADE_LAUNCH(k_shade<kModePhoton>, 256);
+      else BC_SHADE_LAUNCH(k_shade<kModePath>, 256);
     }
 #undef BC_SHADE_LAUNCH
     if (w.photon) {
       if (w.gather_sort) {
         k_gather_count<<<w.acc_grid * 2, 256, 0, st>>>(rb->ga, c);
-        k_gather_scan<<<1, 1024, 0, st>>>(rb->ga);
+        k_gather_scan<<<kGatherBins / kGatherScan, kGatherScan / 4, 0, st>>>(rb->ga);
         k_gather_scatter<<<w.acc_grid * 2, 256, 0, st>>>(rb->ga, c);
       }
-      k_gather<<<w.acc_grid * 4, 128, 0, st>>>(rb->views, rb->ps, rb->ga, c, w.gather_sort ? 1 : 0);
+      k_gather<<<w.acc_grid * 4, 128, 0, st>>>(rb->views, rb->ps, rb->ga, c,
+                                                  w.gather_sort ? rb->ga.perm : rb->ga.list);
     }
     if (w.lights) rb->mark(st, kTimeConnect);
     if (w.lights)
@@ -1808,14 +1830,13 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
 // Runs `n_waves` waves, through one captured CUDA graph when the option allows.
 template <int STACK, bool SPH>
 static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const ShadeScene& sc, int64_t n_waves,
-                           int wave_paths, const GradArgs* grad, bool recursive, bool alt, int photon_entries) {
+                           int wave_paths, const GradArgs* grad, bool recursive, int photon_entries) {
   RenderBuffers* rb = ctx->rb;
   cudaStream_t st = ctx->stream;
   // generate's grid covers this render's wave, not the slots a larger earlier
   // render left allocated
   WaveShape w = wave_shape<STACK, SPH>(wave_paths, bounces, lights, grad, ctx->render_extend, ctx->render_shade_block);
   w.recursive = recursive;
-  w.alt = alt;
   w.photon = photon_entries > 0;
   w.gather_sort = w.photon && wave_paths >= kGatherSortPaths;
   while ((photon_entries >> w.gshift) >= kGatherBins) w.gshift++;
@@ -1846,7 +1867,6 @@ static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const Shad
     add_bytes(&rb->sh, sizeof(rb->sh));
     key.push_back((uintptr_t)rb->sh_cap);
     key.push_back((uintptr_t)recursive);
-    key.push_back((uintptr_t)alt);
     if (recursive) add_bytes(&rb->rr, sizeof(rb->rr));
     key.push_back((uintptr_t)(w.photon ? 1 + w.gather_sort : 0));
     key.push_back((uintptr_t)w.gshift);
@@ -1920,11 +1940,11 @@ static bc_status run_plain(bc_context* ctx, const ShadeScene& sc, const std::vec
     rb->mark(ctx->stream, kTimeOther);
     rb->launches++;
     if (alt)
-      k_render_plain<STACK, SPH, true><<<grid, 128, 0, ctx->stream>>>(
+      k_render_plain<STACK, SPH, kModePhoton><<<grid, 128, 0, ctx->stream>>>(
           rb->views, v, ctx->ds.n_mats, sc, rb->seq_xy, rb->sum, rb->want_sumsq ? rb->sumsq : nullptr, rb->guide_nd,
           rb->guide_c, rb->guide_jit, rb->cnt, ctx->d_status, rb->adapt);
     else
-      k_render_plain<STACK, SPH, false><<<grid, 128, 0, ctx->stream>>>(
+      k_render_plain<STACK, SPH, kModePath><<<grid, 128, 0, ctx->stream>>>(
           rb->views, v, ctx->ds.n_mats, sc, rb->seq_xy, rb->sum, rb->want_sumsq ? rb->sumsq : nullptr, rb->guide_nd,
           rb->guide_c, rb->guide_jit, rb->cnt, ctx->d_status, rb->adapt);
     cudaError_t e = cudaGetLastError();
@@ -2031,8 +2051,8 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     rb->rr_cap = cap;
   }
   if (photon_entries && rb->gather_cap < cap) {
-    cudaError_t e = rb->gather.ensure((size_t)cap * (3 * sizeof(float4) + 3 * sizeof(int32_t)) +
-                                      2 * kGatherBins * sizeof(int) + 8 * 256);
+    cudaError_t e = rb->gather.ensure((size_t)cap * (3 * sizeof(float4) + 4 * sizeof(int32_t)) +
+                                      (2 * kGatherBins + kGatherBins / kGatherScan) * sizeof(int) + 12 * 256);
     if (e) {
       rb->gather_cap = 0;
       return cuda_status(ctx, e, "photon gather queue");
@@ -2041,9 +2061,11 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     GatherSoA& g = rb->ga;
     g.bins = carve<int>(p, kGatherBins);
     g.base = carve<int>(p, kGatherBins);
+    g.totals = carve<int>(p, kGatherBins / kGatherScan);
     g.p = carve<float4>(p, cap);
     g.n = carve<float4>(p, cap);
     g.w = carve<float4>(p, cap);
+    g.list = carve<int32_t>(p, cap);
     g.key = carve<uint32_t>(p, cap);
     g.rank = carve<uint32_t>(p, cap);
     g.perm = carve<int32_t>(p, cap);
@@ -2135,20 +2157,14 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     else if (stack == 128) bst = sph ? run_plain<128, true>(ctx, sc, views, alt) : run_plain<128, false>(ctx, sc, views, alt);
     else bst = sph ? run_plain<256, true>(ctx, sc, views, alt) : run_plain<256, false>(ctx, sc, views, alt);
   } else if (stack == 64)
-    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries)
-              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries);
+    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
+              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
   else if (stack == 128)
-    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries)
-              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries);
+    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
+              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
   else
-    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries)
-              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, alt,
-                                photon_entries);
+    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
+              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
   if (bst) return bst;
   rb->mark(ctx->stream, kTimeOther);
   k_finish_views<<<sm_count() * 8, 256, 0, ctx->stream>>>(rb->views, n, rb->sum, rb->out, rb->adapt.n);
