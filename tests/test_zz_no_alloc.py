@@ -135,3 +135,56 @@ def test_noalloc_rejects_bad_arguments(native_lib):
     assert L.bc_post_process_noalloc(w, h, a.data_ptr(), g.data_ptr(), C.byref(sc), b.data_ptr(), rgba.data_ptr(),
                                      None) == 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 9), (33, 17), (65, 8), (7, 140)])
+@pytest.mark.parametrize("taa,bloom", [(0, 1), (1, 2), (2, 3), (3, 4), (3, 0)])
+def test_post_tile_edges_parity(post_ctx, orc, w, h, taa, bloom):
+    """Frames around the tiles of the denoise (32 x 8 rows a step apart, steps 1 to 16)
+    and bloom kernels (32 x 16; radii above 4 take the two-pass kernels), with sky, against
+    the 64-bit passes. Each pass rounds a weighted mean of positive values (9 taps, weights
+    within a few units each): 2e-5 over five passes leaves a factor of ten."""
+    import bcgx
+    img, g = _frame(w, h, 100 * w + h + taa)
+    g[h // 2:, : w // 3, 3] = -1.0
+    guides = np.zeros((h, w, 11))
+    guides[..., 3:6], guides[..., 9], guides[..., 10] = g[..., :3], g[..., 3], g[..., 3] >= 0
+    st = bcgx.ultra_realism_settings("CPU")
+    st.taa, st.txaa, st.bloom, st.exposure = taa, 0, bloom, 0.4
+    out, rgba = post_ctx.post_process(img, g, st)
+    ref = orc.atrous(img.astype(np.float64), guides, 2 + taa)
+    ref = orc.bloom(ref, bloom) if bloom else ref
+    assert (np.abs(out - ref) / np.maximum(np.abs(ref), 1e-3)).max() < 2e-5
+    tone = orc.to_rgba(out.astype(np.float64), st.exposure, st.gamma, st.hdr)
+    ch = [np.stack([(x >> s) & 255 for s in (0, 8, 16)], -1).astype(int) for x in (rgba, tone)]
+    assert np.abs(ch[0] - ch[1]).max() <= 1 and np.sum(ch[0] != ch[1]) <= 1 + 0.001 * ch[0].size
+
+
+def test_noalloc_post_under_capture(post_ctx):
+    """The chained launches record into a graph; its replays give the direct call's result."""
+    torch = pytest.importorskip("torch")
+    import bcgx
+    from bcgx._lib import lib
+
+    img, g = _frame(200, 120, 9)
+    sc = bcgx.ultra_realism_settings("CPU").c()
+    d_in, d_g = torch.from_numpy(img).cuda(), torch.from_numpy(g).cuda()
+    d_out, d_rgba = torch.zeros_like(d_in), torch.zeros((120, 200), dtype=torch.int32, device="cuda")
+
+    def call(stream):
+        assert lib().bc_post_process_noalloc(200, 120, d_in.data_ptr(), d_g.data_ptr(), C.byref(sc), d_out.data_ptr(),
+                                             d_rgba.data_ptr(), stream.cuda_stream) == 0
+
+    st = torch.cuda.Stream()
+    call(st)
+    st.synchronize()
+    want, want_rgba = d_out.clone(), d_rgba.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        call(st)
+    for _ in range(2):
+        d_out.zero_()
+        d_rgba.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(d_out, want) and torch.equal(d_rgba, want_rgba)
