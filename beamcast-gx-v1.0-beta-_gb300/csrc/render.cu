@@ -60,17 +60,8 @@ struct ShadowSoA {
   int32_t* path;
 };
 
-// Path replay records of a gradient render: for every path and bounce, the
-// material whose parameter the vertex depends on and the value the adjoint
-// needs (diffuse: radiance gathered before the albedo multiplied the
-// throughput; emitter: throughput times MIS weight). m < 0: no record.
+// Tag of an emitter's vertex record (GradRec, wave.h).
 constexpr int kEmitTag = 1 << 30;
-struct GradRec {
-  int32_t* m;   // [bounce * cap + path]
-  float4* v;    // [bounce * cap + path]
-  int32_t* nb;  // bounces shaded per path
-  int cap;
-};
 
 // Vertex records of the recursive integrator (traceRecursiveInner,
 // renderer.go:1569-1621). The reference samples directLight at a diffuse vertex
@@ -948,10 +939,11 @@ __device__ __forceinline__ void shade_body(const BatchState* __restrict__ bs,
       }
       s.flush_L();
       if (rec.m) {
-        const size_t r = (size_t)bounce * rec.cap + path;
+        const size_t slot = (rec.L ? (size_t)bs->w0 : 0) + path;
+        const size_t r = (size_t)bounce * rec.cap + slot;
         rec.m[r] = out.rec_m;
-        rec.v[r] = make_float4(out.rec_v.x, out.rec_v.y, out.rec_v.z, 0.0f);
-        rec.nb[path] = bounce + 1;
+        if (out.rec_m >= 0) rec.v[r] = make_float4(out.rec_v.x, out.rec_v.y, out.rec_v.z, 0.0f);
+        rec.nb[slot] = bounce + 1;
       }
     }
     const int qn = block_reserve<BLOCK>(&cnt->q[cur ^ 1], out.alive);
@@ -1220,60 +1212,104 @@ __global__ void k_accumulate(const BatchState* __restrict__ bs, const ViewGPU* _
   }
 }
 
-// ---- gradient (path replay) --------------------------------------------------------
-// After the last bounce of a wave every path knows its final radiance Lf. With
-// the adjoint d = dLoss/dImage(pixel) / spp of its pixel:
+// ---- gradient -----------------------------------------------------------------------
+// Every path knows its final radiance Lf and its vertex records. With the adjoint
+// d = dLoss/dImage(pixel) / spp of its pixel:
 //   diffuse vertex on material m : dL/d albedo_m = (Lf - L_before) / albedo_m
 //   emitter hit on material e    : dL/d emission_e = throughput * MIS weight
 // (everything a path gathers after the albedo of m multiplied its throughput is
 // linear in that albedo; Russian roulette probabilities are held fixed).
-// Per block sums in fp64 shared memory, one row of `partial` per block.
-__global__ void __launch_bounds__(256) k_gradient(const BatchState* __restrict__ bs, const ViewGPU* __restrict__ views,
-                                                  PathState ps, GradRec rec, GradArgs ga,
-                                                  const MatGPU* __restrict__ mats) {
-  extern __shared__ double sg[];
+// Per block sums in fp64 shared memory, one row of `partial` per block. Bound by the
+// latency of each path's chain of loads (records, material, parameter) and of its fp64
+// shared atomics: two blocks an SM (gradient_grid) of 256 threads took 3.0 ms for 16.8M
+// paths and 264 parameters, of 768 threads 1.55 ms (512: 1.66, 1024: 1.73).
+constexpr int kGradThreads = 768;
+__device__ __forceinline__ void gradient_of_path(double* sg, const GradRec& rec, size_t i, float3 dl, float3 Lf,
+                                                 const GradArgs& ga, const MatGPU* __restrict__ mats) {
+  const int nb = rec.nb[i];
+  for (int b = 0; b < nb; b++) {
+    const size_t r = (size_t)b * rec.cap + i;
+    const int m = rec.m[r];
+    if (m < 0) continue;
+    const int mm = m & ~kEmitTag;
+    const int k = ga.mat2param[mm];
+    if (k < 0) continue;
+    const float4 v = rec.v[r];
+    float gx, gy, gz;
+    if (m & kEmitTag) {
+      gx = dl.x * v.x;
+      gy = dl.y * v.y;
+      gz = dl.z * v.z;
+    } else {
+      const MatGPU M = mats[mm];
+      gx = M.cr > 0.0f ? dl.x * ((Lf.x - v.x) / M.cr) : 0.0f;
+      gy = M.cg > 0.0f ? dl.y * ((Lf.y - v.y) / M.cg) : 0.0f;
+      gz = M.cb > 0.0f ? dl.z * ((Lf.z - v.z) / M.cb) : 0.0f;
+    }
+    atomicAdd(&sg[3 * k], (double)gx);
+    atomicAdd(&sg[3 * k + 1], (double)gy);
+    atomicAdd(&sg[3 * k + 2], (double)gz);
+  }
+}
+
+__device__ __forceinline__ float3 path_adjoint(const GradArgs& ga, size_t pixel, int spp) {
+  const float* dp = ga.dimg + 3 * pixel;
+  const float inv = 1.0f / (float)spp;
+  return f3(dp[0] * inv, dp[1] * inv, dp[2] * inv);
+}
+
+__device__ __forceinline__ void gradient_row(const double* sg, const GradArgs& ga) {
+  __syncthreads();
   const int np3 = 3 * ga.n_params;
-  for (int k = threadIdx.x; k < np3; k += blockDim.x) sg[k] = 0.0;
+  double* row = ga.partial + (size_t)blockIdx.x * np3;
+  for (int k = threadIdx.x; k < np3; k += blockDim.x) row[k] += sg[k];
+}
+
+// of a replayed wave, after its last bounce
+__global__ void __launch_bounds__(kGradThreads) k_gradient(const BatchState* __restrict__ bs,
+                                                           const ViewGPU* __restrict__ views, PathState ps,
+                                                           GradRec rec, GradArgs ga,
+                                                           const MatGPU* __restrict__ mats) {
+  extern __shared__ double sg[];
+  for (int k = threadIdx.x; k < 3 * ga.n_params; k += blockDim.x) sg[k] = 0.0;
   __syncthreads();
   const long long w0 = bs->w0;
   const int n = (int)min((long long)bs->cap, bs->total - w0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const ViewGPU& V = views[__float_as_uint(ps.ray[2 * (size_t)i].w)];
-    const long long pix = (w0 + i - V.path_off) % V.npix;
-    const float* dp = ga.dimg + 3 * (size_t)(V.pix_off + pix);
-    const float inv = 1.0f / (float)V.spp;
-    const float3 dl = f3(dp[0] * inv, dp[1] * inv, dp[2] * inv);
+    const float3 dl = path_adjoint(ga, (size_t)(V.pix_off + (w0 + i - V.path_off) % V.npix), V.spp);
     if (dl.x == 0.0f && dl.y == 0.0f && dl.z == 0.0f) continue;
     const float4 Lw = ps.L[i];
-    const float3 Lf = f3(Lw.x, Lw.y, Lw.z);
-    const int nb = rec.nb[i];
-    for (int b = 0; b < nb; b++) {
-      const size_t r = (size_t)b * rec.cap + i;
-      const int m = rec.m[r];
-      if (m < 0) continue;
-      const int mm = m & ~kEmitTag;
-      const int k = ga.mat2param[mm];
-      if (k < 0) continue;
-      const float4 v = rec.v[r];
-      float gx, gy, gz;
-      if (m & kEmitTag) {
-        gx = dl.x * v.x;
-        gy = dl.y * v.y;
-        gz = dl.z * v.z;
-      } else {
-        const MatGPU M = mats[mm];
-        gx = M.cr > 0.0f ? dl.x * ((Lf.x - v.x) / M.cr) : 0.0f;
-        gy = M.cg > 0.0f ? dl.y * ((Lf.y - v.y) / M.cg) : 0.0f;
-        gz = M.cb > 0.0f ? dl.z * ((Lf.z - v.z) / M.cb) : 0.0f;
-      }
-      atomicAdd(&sg[3 * k], (double)gx);
-      atomicAdd(&sg[3 * k + 1], (double)gy);
-      atomicAdd(&sg[3 * k + 2], (double)gz);
-    }
+    gradient_of_path(sg, rec, i, dl, f3(Lw.x, Lw.y, Lw.z), ga, mats);
   }
+  gradient_row(sg, ga);
+}
+
+// of a whole render whose records were kept
+__global__ void __launch_bounds__(kGradThreads) k_gradient_kept(GradRec rec, long long n, int npix, int spp,
+                                                                GradArgs ga, const MatGPU* __restrict__ mats) {
+  extern __shared__ double sg[];
+  for (int k = threadIdx.x; k < 3 * ga.n_params; k += blockDim.x) sg[k] = 0.0;
   __syncthreads();
-  double* row = ga.partial + (size_t)blockIdx.x * np3;
-  for (int k = threadIdx.x; k < np3; k += blockDim.x) row[k] += sg[k];
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const float3 dl = path_adjoint(ga, (size_t)(i % npix), spp);
+    if (dl.x == 0.0f && dl.y == 0.0f && dl.z == 0.0f) continue;
+    const float4 Lw = rec.L[i];
+    gradient_of_path(sg, rec, (size_t)i, dl, f3(Lw.x, Lw.y, Lw.z), ga, mats);
+  }
+  gradient_row(sg, ga);
+}
+
+// The wave's final radiances into a whole render's records.
+__global__ void k_keep_radiance(const BatchState* __restrict__ bs, PathState ps, float4* __restrict__ L) {
+  const long long w0 = bs->w0;
+  const int n = (int)min((long long)bs->cap, bs->total - w0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) L[w0 + i] = ps.L[i];
+}
+
+size_t grad_rec_bytes(size_t paths, int bounces, bool whole) {
+  return paths * ((size_t)bounces * (sizeof(float4) + sizeof(int32_t)) + sizeof(int32_t) +
+                  (whole ? sizeof(float4) : 0)) + 5 * 256;
 }
 
 __global__ void k_advance(BatchState* bs, WaveCounters* cnt) {
@@ -1724,6 +1760,7 @@ struct WaveShape {
   int bounces;
   bool lights;
   const GradArgs* grad;  // non-null: gradient render
+  const GradRec* keep;   // non-null: leaves every path's vertex records there
   bool recursive;        // the batch has views of the recursive integrator
   bool photon;           // the batch has views of the photon integrator
   bool gather_sort;      // their gathers are sorted
@@ -1758,6 +1795,7 @@ static WaveShape wave_shape(int cap, int bounces, bool lights, const GradArgs* g
   w.bounces = bounces;
   w.lights = lights;
   w.grad = grad;
+  w.keep = nullptr;
   w.recursive = false;
   w.photon = w.gather_sort = false;
   w.gshift = 0;
@@ -1785,7 +1823,7 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
       k_extend_12<STACK, SPH><<<w.ext_grid, 128, 0, st>>>(sc.sv, rb->views, rb->ps, rb->q[cur], c, cur, ctx->d_status);
     else
       k_extend_10<STACK, SPH><<<w.ext_grid, 128, 0, st>>>(sc.sv, rb->views, rb->ps, rb->q[cur], c, cur, ctx->d_status);
-    const GradRec rec = w.grad ? rb->grec : GradRec{nullptr, nullptr, nullptr, 0};
+    const GradRec rec = w.grad ? rb->grec : w.keep ? *w.keep : GradRec{};
     rb->mark(st, kTimeShade);
 #define BC_SHADE_LAUNCH(KERNEL, BLOCK)                                                                         \
   KERNEL<<<w.shade_grid, BLOCK, 0, st>>>(rb->bs, rb->views, ctx->ds.n_mats, sc, rb->ps, rb->q[cur], rb->q[cur ^ 1], rb->sh, \
@@ -1817,9 +1855,10 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
   }
   if (w.grad) rb->mark(st, kTimeOther);
   if (w.grad)
-    k_gradient<<<gradient_grid(), 256, 3 * w.grad->n_params * sizeof(double), st>>>(rb->bs, rb->views, rb->ps,
+    k_gradient<<<gradient_grid(), kGradThreads, 3 * w.grad->n_params * sizeof(double), st>>>(rb->bs, rb->views, rb->ps,
                                                                                   rb->grec, *w.grad, sc.mats);
   rb->mark(st, kTimeAccumulate);
+  if (w.keep) k_keep_radiance<<<w.acc_grid, 256, 0, st>>>(rb->bs, rb->ps, w.keep->L);
   k_accumulate<<<w.acc_grid, 256, 0, st>>>(rb->bs, rb->views, rb->ps, rb->sum, rb->want_sumsq ? rb->sumsq : nullptr,
                                            rb->adapt, rr);
   rb->mark(st, kTimeOther);
@@ -1830,12 +1869,14 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
 // Runs `n_waves` waves, through one captured CUDA graph when the option allows.
 template <int STACK, bool SPH>
 static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const ShadeScene& sc, int64_t n_waves,
-                           int wave_paths, const GradArgs* grad, bool recursive, int photon_entries) {
+                           int wave_paths, const GradArgs* grad, const GradRec* keep, bool recursive,
+                           int photon_entries) {
   RenderBuffers* rb = ctx->rb;
   cudaStream_t st = ctx->stream;
   // generate's grid covers this render's wave, not the slots a larger earlier
   // render left allocated
   WaveShape w = wave_shape<STACK, SPH>(wave_paths, bounces, lights, grad, ctx->render_extend, ctx->render_shade_block);
+  w.keep = keep;
   w.recursive = recursive;
   w.photon = photon_entries > 0;
   w.gather_sort = w.photon && wave_paths >= kGatherSortPaths;
@@ -1845,7 +1886,7 @@ static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const Shad
   // settings): such a render is captured the second time its key is seen.
   bool use_graph = ctx->render_graph != 0 && !rb->ktiming;  // per-launch events need direct launches
   rb->launches += n_waves * (3 + (int64_t)bounces * (2 + (lights ? 1 : 0) + (w.photon ? (w.gather_sort ? 4 : 1) : 0)) +
-                             (grad ? 1 : 0));
+                             (grad || keep ? 1 : 0));
   rb->extend_launches += n_waves * (int64_t)bounces;
   if (use_graph) {
     // every value the captured launches were given
@@ -1872,7 +1913,8 @@ static bc_status run_waves(bc_context* ctx, int bounces, bool lights, const Shad
     key.push_back((uintptr_t)w.gshift);
     if (w.photon) add_bytes(&rb->ga, sizeof(rb->ga));
     add_bytes(&sc, sizeof(sc));
-    key.push_back((uintptr_t)(grad != nullptr));
+    if (keep) add_bytes(keep, sizeof(*keep));
+    key.push_back((uintptr_t)(grad != nullptr) + 2 * (uintptr_t)(keep != nullptr));
     if (grad) {
       add_bytes(grad, sizeof(*grad));
       add_bytes(&rb->grec, sizeof(rb->grec));
@@ -1954,7 +1996,7 @@ static bc_status run_plain(bc_context* ctx, const ShadeScene& sc, const std::vec
 }
 
 bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
-                       const GradArgs* grad) {
+                       const GradArgs* grad, const GradRec* keep) {
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (req.empty()) return set_error(ctx, BC_ERR_INVALID_ARG, "no views");
   bc_status bst;
@@ -2075,17 +2117,12 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     if (max_bounces > kMaxGradBounces) return set_error(ctx, BC_ERR_INVALID_ARG, "gradient renders allow 64 bounces");
     // stride: this render's wave size (path slots >= cap are never used by it)
     if (rb->rec_bounces < max_bounces || rb->rec_cap < cap) {
-      const size_t per = sizeof(int32_t) + sizeof(float4);
-      cudaError_t e = rb->rec.ensure((size_t)max_bounces * cap * per + (size_t)cap * sizeof(int32_t) + 4 * 256);
+      cudaError_t e = rb->rec.ensure(grad_rec_bytes(cap, max_bounces, false));
       if (e) {
         rb->rec_bounces = rb->rec_cap = 0;
         return cuda_status(ctx, e, "path replay records");
       }
-      char* p = (char*)rb->rec.p;
-      rb->grec.v = carve<float4>(p, (size_t)max_bounces * cap);
-      rb->grec.m = carve<int32_t>(p, (size_t)max_bounces * cap);
-      rb->grec.nb = carve<int32_t>(p, cap);
-      rb->grec.cap = cap;
+      rb->grec = grad_rec_carve(rb->rec.p, cap, max_bounces, false);
       rb->rec_bounces = max_bounces;
       rb->rec_cap = cap;
     }
@@ -2157,14 +2194,20 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
     else if (stack == 128) bst = sph ? run_plain<128, true>(ctx, sc, views, alt) : run_plain<128, false>(ctx, sc, views, alt);
     else bst = sph ? run_plain<256, true>(ctx, sc, views, alt) : run_plain<256, false>(ctx, sc, views, alt);
   } else if (stack == 64)
-    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
-              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
+    bst = sph ? run_waves<64, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries)
+              : run_waves<64, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries);
   else if (stack == 128)
-    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
-              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
+    bst = sph ? run_waves<128, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries)
+              : run_waves<128, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries);
   else
-    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries)
-              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, rec_bounces > 0, photon_entries);
+    bst = sph ? run_waves<256, true>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries)
+              : run_waves<256, false>(ctx, max_bounces, lights, sc, n_waves, bsh.cap, grad, keep, rec_bounces > 0,
+                                            photon_entries);
   if (bst) return bst;
   rb->mark(ctx->stream, kTimeOther);
   k_finish_views<<<sm_count() * 8, 256, 0, ctx->stream>>>(rb->views, n, rb->sum, rb->out, rb->adapt.n);
@@ -2199,6 +2242,24 @@ static bc_status render_rows_device(bc_context* ctx, const bc_camera& cam, const
   if (s.width < 1 || s.height < 1 || (int64_t)s.width * s.height > (1 << 26))
     return set_error(ctx, BC_ERR_INVALID_ARG, "invalid render size, rows, spp or bounces");
   return render_views(ctx, std::vector<ViewRequest>{r}, (size_t)s.width * s.height, rays, nullptr);
+}
+
+GradRec grad_rec_carve(void* base, size_t paths, int bounces, bool whole) {
+  char* p = (char*)base;
+  GradRec r;
+  r.v = carve<float4>(p, paths * bounces);
+  r.L = whole ? carve<float4>(p, paths) : nullptr;
+  r.m = carve<int32_t>(p, paths * bounces);
+  r.nb = carve<int32_t>(p, paths);
+  r.cap = (int)paths;
+  return r;
+}
+
+cudaError_t gradient_from_records(bc_context* ctx, const GradRec& rec, long long n, int npix, int spp,
+                                  const GradArgs& ga) {
+  k_gradient_kept<<<gradient_grid(), kGradThreads, 3 * ga.n_params * sizeof(double), ctx->stream>>>(
+      rec, n, npix, spp, ga, ctx->ds.mats);
+  return cudaGetLastError();
 }
 
 float* render_mean(bc_context* ctx) { return ctx->rb ? ctx->rb->out : nullptr; }

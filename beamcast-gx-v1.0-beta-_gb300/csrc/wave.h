@@ -19,6 +19,20 @@ struct ViewRequest {
   bool want_guides;
 };
 
+// Vertex records of a render's paths: for every path and bounce, the material whose
+// parameter the vertex depends on and the value the adjoint needs (diffuse: radiance
+// gathered before the albedo multiplied the throughput; emitter: throughput times MIS
+// weight). m < 0: no record.
+struct GradRec {
+  int32_t* m;   // [bounce * cap + path]
+  float4* v;    // [bounce * cap + path]
+  int32_t* nb;  // bounces shaded per path
+  int cap;      // paths: those of a wave, or of the whole render when L is given
+  float4* L;    // final radiance per path of the whole render (null: records of one wave)
+};
+size_t grad_rec_bytes(size_t paths, int bounces, bool whole);
+GradRec grad_rec_carve(void* p, size_t paths, int bounces, bool whole);
+
 // Gradient render (path replay): adjoint image and parameter map.
 struct GradArgs {
   const float* dimg;         // 3 per frame pixel: dLoss / dImage
@@ -28,9 +42,14 @@ struct GradArgs {
 };
 
 // Renders the views; each view's mean radiance ends in render_mean(ctx) at its
-// pix_off. With `grad`, also accumulates the path replay gradient into grad->partial.
+// pix_off. With `grad`, also accumulates the path replay gradient into grad->partial;
+// with `keep`, leaves the vertex records and radiances of every path there (path
+// integrator, fixed samples, the wave engine).
 bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
-                       const GradArgs* grad);
+                       const GradArgs* grad, const GradRec* keep = nullptr);
+// The gradient of one view's `n` paths (sample-major over npix pixels) from kept records.
+cudaError_t gradient_from_records(bc_context* ctx, const GradRec& rec, long long n, int npix, int spp,
+                                  const GradArgs& ga);
 float* render_mean(bc_context* ctx);
 
 // Photon maps (photon.cu). photon_map_for returns the map of resident scene

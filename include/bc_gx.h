@@ -337,13 +337,17 @@ bc_status bc_diff_set_target(bc_context* ctx, const float* target);
  * Writes `params` (3 * (n_albedo + n_emission) floats) into the resident
  * materials and renders the configured view with path seed `seed`.
  * image_out (may be NULL): width*height RGB mean radiance. loss_out (may be
- * NULL; needs a target): the L2 loss.
+ * NULL; needs a target): the L2 loss. The context keeps the paths' vertex
+ * records on the device for bc_backward: 20 bytes per path and bounce and 20
+ * per path, up to 8 GB and a quarter of the free memory; freed with the context.
  */
 bc_status bc_forward(bc_context* ctx, const float* params, uint64_t seed, float* image_out, double* loss_out);
 /*
  * Gradient of the loss at the last bc_forward. dloss_dimage: width*height RGB
  * floats, or NULL for the L2 loss against the target. grad_albedo:
  * 3 * n_albedo floats, grad_emission: 3 * n_emission floats (either may be NULL).
+ * Where the forward's records were not kept, or the scene was uploaded since,
+ * the paths are traced again (path replay), against the resident scene.
  */
 bc_status bc_backward(bc_context* ctx, const float* dloss_dimage, float* grad_albedo, float* grad_emission);
 

@@ -193,3 +193,55 @@ def test_diff_argument_errors(gpu_ctx, problem):
     gpu_ctx.forward(problem.init_params, SEED, want_image=False)
     with pytest.raises(bcgx.BCError, match="INVALID_ARG"):  # no target, no adjoint image
         gpu_ctx.backward()
+
+
+@pytest.mark.parametrize("wave_cap,rr_depth", [(1 << 26, 6), (4096, 6), (5000, 2)])
+def test_kept_records_match_replay(ctx, problem, wave_cap, rr_depth):
+    """The gradient from the records that a forward render kept (one wave, many waves, a
+    ragged last one) is that of a replay of its paths, which a forward through the
+    one-kernel form leaves to the backward render. Both sum the same fp32 terms in fp64."""
+    st = problem.settings.copy()
+    st.rr_depth = rr_depth
+    ctx.diff_configure(problem.cam, st, problem.albedo_materials, problem.emission_materials)
+    w = np.random.default_rng(3).uniform(-1, 1, (st.height, st.width, 3)).astype(np.float32)
+    old_cap = ctx.get_option("render_wave_cap")
+    grads = []
+    try:
+        ctx.set_option("render_wave_cap", wave_cap)
+        for engine in (0, 1, 0):
+            ctx.set_option("render_engine", engine)
+            ctx.forward(problem.init_params, SEED, want_image=False)
+            ctx.set_option("render_engine", 0)
+            grads.append(np.concatenate(ctx.backward(w)))
+            grads.append(np.concatenate(ctx.backward(2 * w)) / 2)  # another adjoint of the same forward
+    finally:
+        ctx.set_option("render_engine", 0)
+        ctx.set_option("render_wave_cap", old_cap)
+    scale = np.abs(grads[0]).max()
+    assert scale > 0
+    for g in grads[1:]:
+        assert np.abs(g - grads[0]).max() <= 1e-6 * scale
+
+
+def test_backward_after_another_upload_replays(ctx, problem):
+    """A scene uploaded after the forward makes its records stale: the backward render
+    sees the scene that is resident now."""
+    w = np.ones((problem.settings.height, problem.settings.width, 3), np.float32)
+    ctx.forward(0.5 * problem.init_params, SEED, want_image=False)
+    kept = np.concatenate(ctx.backward(w))
+    # the same geometry and material list, with the spec's own colours (init_params)
+    ctx.upload(scenes.to_scene(problem.spec))
+    now = np.concatenate(ctx.backward(w))
+    assert np.isfinite(now).all() and np.abs(now - kept).max() > 1e-3 * np.abs(kept).max()
+    ctx.cancel()
+    try:
+        with pytest.raises(bcgx.BCError):
+            ctx.backward(w)
+        ctx.reset_cancel()
+        ctx.diff_configure(problem.cam, problem.settings, problem.albedo_materials, problem.emission_materials)
+        ctx.forward(problem.init_params, SEED, want_image=False)
+        ctx.cancel()
+        with pytest.raises(bcgx.BCError):
+            ctx.backward(w)
+    finally:
+        ctx.reset_cancel()
