@@ -9,6 +9,9 @@ CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import math
+import threading
+import weakref
 
 import numpy as np
 
@@ -25,8 +28,53 @@ def gpu_available() -> tuple[bool, str]:
     return bool(ok), buf.value.decode(errors="replace")
 
 
+class _Outputs:
+    """Memory for a context's returned images. An image's memory comes back once the
+    caller has dropped every reference to it, and the next image of that size takes it:
+    fresh memory of a frame's size is mapped page by page while the device copies into
+    it, which takes far longer than the copy (a frame with guides, 960 x 540: 2.00 ->
+    1.12 ms; 1280 x 720: 6.04 -> 4.99 ms). Holds at most LIMIT bytes, given back with the context."""
+    LIMIT = 256 << 20
+    MIN = 256 << 10  # smaller arrays come from the allocator's heap, which stays mapped
+
+    def __init__(self):
+        self._free, self._bytes, self._open = [], 0, True
+        self._lock = threading.RLock()  # re-entrant: a collection may run a finalizer inside
+
+    def empty(self, shape, dtype) -> np.ndarray:
+        n = math.prod(shape) * np.dtype(dtype).itemsize
+        if n < self.MIN:
+            return np.empty(shape, dtype)
+        mem = None
+        with self._lock:
+            for i in range(len(self._free) - 1, -1, -1):
+                if self._free[i].nbytes == n:
+                    mem = self._free.pop(i)
+                    self._bytes -= n
+                    break
+        if mem is None:
+            mem = np.empty(n, np.uint8)
+        owner = (C.c_char * n).from_buffer(mem)  # every view of the image keeps it alive
+        weakref.finalize(owner, self._put, mem).atexit = False
+        return np.frombuffer(owner, dtype=dtype).reshape(shape)
+
+    def _put(self, mem):
+        with self._lock:
+            if not self._open or mem.nbytes > self.LIMIT:
+                return
+            self._free.append(mem)
+            self._bytes += mem.nbytes
+            while self._bytes > self.LIMIT:  # the longest unused first
+                self._bytes -= self._free.pop(0).nbytes
+
+    def close(self):
+        with self._lock:
+            self._free, self._bytes, self._open = [], 0, False
+
+
 class Context:
     def __init__(self, device: int = 0):
+        self._outputs = _Outputs()
         h = C.c_void_p()
         check(lib().bc_create(int(device), C.byref(h)))
         self._h = h
@@ -36,6 +84,7 @@ class Context:
         if getattr(self, "_h", None):
             lib().bc_destroy(self._h)
             self._h = None
+            self._outputs.close()
 
     def __del__(self):
         self.close()
@@ -134,8 +183,8 @@ class Context:
     # -- rendering --
     def render_rows(self, cam: Camera, settings: RenderSettings, y0: int, rows: int, guides: bool = False):
         W = settings.width
-        lin = np.empty((rows, W, 3), dtype=np.float32)
-        g = np.empty((rows, W, 3), dtype=np.uint32) if guides else None
+        lin = self._outputs.empty((rows, W, 3), np.float32)
+        g = self._outputs.empty((rows, W, 3), np.uint32) if guides else None
         rays = C.c_int64(0)
         cc, sc = cam.c(), settings.c()
         check(lib().bc_render_rows(self._h, C.byref(cc), C.byref(sc), int(y0), int(rows), ptr(lin, C.c_float),
@@ -144,9 +193,9 @@ class Context:
 
     def render_frame(self, cam: Camera, settings: RenderSettings, want_guides: bool = True, want_rgba: bool = True):
         W, H = settings.width, settings.height
-        lin = np.empty((H, W, 3), dtype=np.float32)
-        g = np.empty((H, W, 3), dtype=np.uint32) if want_guides else None
-        rgba = np.empty((H, W), dtype=np.uint32) if want_rgba else None
+        lin = self._outputs.empty((H, W, 3), np.float32)
+        g = self._outputs.empty((H, W, 3), np.uint32) if want_guides else None
+        rgba = self._outputs.empty((H, W), np.uint32) if want_rgba else None
         rays = C.c_int64(0)
         cc, sc = cam.c(), settings.c()
         check(lib().bc_render_frame(self._h, C.byref(cc), C.byref(sc), ptr(lin, C.c_float), ptr(g, C.c_uint32),
@@ -156,8 +205,8 @@ class Context:
     def render_moments(self, cam: Camera, settings: RenderSettings):
         """Per-pixel mean and mean of squares of the sample radiance (no post)."""
         W, H = settings.width, settings.height
-        mean = np.empty((H, W, 3), dtype=np.float32)
-        msq = np.empty((H, W, 3), dtype=np.float32)
+        mean = self._outputs.empty((H, W, 3), np.float32)
+        msq = self._outputs.empty((H, W, 3), np.float32)
         rays = C.c_int64(0)
         cc, sc = cam.c(), settings.c()
         check(lib().bc_render_moments(self._h, C.byref(cc), C.byref(sc), ptr(mean, C.c_float), ptr(msq, C.c_float),
@@ -176,7 +225,7 @@ class Context:
             vc[i].reserved = 0
             vc[i].camera = cam.c()
             vc[i].settings = st.c()
-            o = np.empty((st.height, st.width, 3), dtype=np.float32) if readback else None
+            o = self._outputs.empty((st.height, st.width, 3), np.float32) if readback else None
             outs.append(o)
             ptrs[i] = ptr(o, C.c_float)
         rays = C.c_int64(0)
@@ -247,7 +296,7 @@ class Context:
             want_loss = self._diff_has_target
         p = np.ascontiguousarray(params, dtype=np.float32).reshape(-1)
         assert p.size == 3 * (na + ne)
-        img = np.empty((H, W, 3), np.float32) if want_image else None
+        img = self._outputs.empty((H, W, 3), np.float32) if want_image else None
         loss = C.c_double(0)
         check(lib().bc_forward(self._h, ptr(p, C.c_float), int(seed), ptr(img, C.c_float),
                                C.byref(loss) if want_loss else None), self._h)
@@ -280,8 +329,8 @@ class Context:
         d.exposure = float(levels.get("exposure", 0.0))
         d.gamma = float(levels.get("gamma", 2.2))
         d.camera = cam.c()
-        out = np.empty((height, width, 3), np.float32)
-        rgba = np.empty((height, width), np.uint32) if want_rgba else None
+        out = self._outputs.empty((height, width, 3), np.float32)
+        rgba = self._outputs.empty((height, width), np.uint32) if want_rgba else None
         check(lib().bc_post_stack(self._h, C.byref(d), ptr(lin, C.c_float), ptr(g, C.c_float), ptr(out, C.c_float),
                                   ptr(rgba, C.c_uint32)), self._h)
         return out, rgba
@@ -295,8 +344,8 @@ class Context:
         H, W = linear.shape[:2]
         lin = np.ascontiguousarray(linear, dtype=np.float32)
         g = None if guide_nd is None else np.ascontiguousarray(guide_nd, dtype=np.float32)
-        out = np.empty((H, W, 3), dtype=np.float32)
-        rgba = np.empty((H, W), dtype=np.uint32) if want_rgba else None
+        out = self._outputs.empty((H, W, 3), np.float32)
+        rgba = self._outputs.empty((H, W), np.uint32) if want_rgba else None
         sc = settings.c()
         check(lib().bc_post_process(self._h, W, H, ptr(lin, C.c_float), ptr(g, C.c_float), C.byref(sc),
                                     ptr(out, C.c_float), ptr(rgba, C.c_uint32)), self._h)

@@ -1458,6 +1458,8 @@ struct RenderBuffers {
   size_t frame_px = 0;  // pixels of the frame buffers
   bcgx::DevBuf paths, shadow, queues, counters, seq, frame, table;
   bcgx::HostBuf staging;
+  bcgx::HostBuf readback;  // [kernel status | extension rays | rays of the photon maps built]
+  int n_readback = 0;
   bcgx::PathState ps{};
   bcgx::ShadowSoA sh{};
   int* q[2] = {nullptr, nullptr};
@@ -1534,6 +1536,7 @@ void destroy_render_buffers(bc_context* ctx) {
   rb->frame.release();
   rb->table.release();
   rb->staging.release();
+  rb->readback.release();
   rb->rec.release();
   rb->rrec.release();
   rb->gather.release();
@@ -1995,8 +1998,10 @@ static bc_status run_plain(bc_context* ctx, const ShadeScene& sc, const std::vec
   return BC_OK;
 }
 
-bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
-                       const GradArgs* grad, const GradRec* keep) {
+// Queues everything of render_views: the caller may queue more work on the frame behind
+// it and ends with wait_views.
+static bc_status enqueue_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px,
+                               const GradArgs* grad, const GradRec* keep) {
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (req.empty()) return set_error(ctx, BC_ERR_INVALID_ARG, "no views");
   bc_status bst;
@@ -2216,21 +2221,41 @@ bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, siz
   rb->launches += rb->want_sumsq ? 2 : 1;
   timing_end(ctx);
   e = cudaGetLastError();
-  unsigned long long r = 0;
-  std::vector<unsigned long long> pr(photon_rays.size(), 0);
-  if (!e) e = cudaMemcpyAsync(&r, &rb->cnt->rays, sizeof(r), cudaMemcpyDeviceToHost, ctx->stream);
-  for (size_t k = 0; k < photon_rays.size() && !e; k++)
-    e = cudaMemcpyAsync(&pr[k], photon_rays[k], sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
+  const int nr = 2 + (int)photon_rays.size();
+  if (!e) e = rb->readback.ensure(nr * sizeof(unsigned long long));
   if (e) return cuda_status(ctx, e, "render");
-  for (unsigned long long v : pr) r += v;  // Start counts the photon map's rays (renderer.go:2809)
-  if (rays) *rays = (int64_t)r;
-  timing_collect(ctx);
-  return check_kernel_status(ctx);
+  unsigned long long* h = static_cast<unsigned long long*>(rb->readback.p);
+  h[0] = 0;
+  e = cudaMemcpyAsync(h, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream);
+  if (!e) e = cudaMemcpyAsync(h + 1, &rb->cnt->rays, sizeof(*h), cudaMemcpyDeviceToHost, ctx->stream);
+  for (int k = 2; k < nr && !e; k++)
+    e = cudaMemcpyAsync(h + k, photon_rays[k - 2], sizeof(*h), cudaMemcpyDeviceToHost, ctx->stream);
+  rb->n_readback = nr;
+  return cuda_status(ctx, e, "render");
 }
 
-static bc_status render_rows_device(bc_context* ctx, const bc_camera& cam, const bc_settings& s, int y0, int rows,
-                                    bool want_guides, int64_t* rays) {
+// Waits for the stream; the counters, timing and kernel status of the render that
+// enqueue_views queued.
+static bc_status wait_views(bc_context* ctx, int64_t* rays, const char* what) {
+  RenderBuffers* rb = ctx->rb;
+  cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (e) return cuda_status(ctx, e, what);
+  const unsigned long long* h = static_cast<const unsigned long long*>(rb->readback.p);
+  unsigned long long r = 0;
+  for (int k = 1; k < rb->n_readback; k++) r += h[k];  // Start counts the photon map's rays (renderer.go:2809)
+  if (rays) *rays = (int64_t)r;
+  timing_collect(ctx);
+  return h[0] ? check_kernel_status(ctx) : BC_OK;
+}
+
+bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
+                       const GradArgs* grad, const GradRec* keep) {
+  const bc_status st = enqueue_views(ctx, req, frame_px, grad, keep);
+  return st ? st : wait_views(ctx, rays, "render");
+}
+
+static bc_status enqueue_rows(bc_context* ctx, const bc_camera& cam, const bc_settings& s, int y0, int rows,
+                              bool want_guides) {
   ViewRequest r;
   r.scene = 0;
   r.cam = cam;
@@ -2241,7 +2266,7 @@ static bc_status render_rows_device(bc_context* ctx, const bc_camera& cam, const
   r.want_guides = want_guides;
   if (s.width < 1 || s.height < 1 || (int64_t)s.width * s.height > (1 << 26))
     return set_error(ctx, BC_ERR_INVALID_ARG, "invalid render size, rows, spp or bounces");
-  return render_views(ctx, std::vector<ViewRequest>{r}, (size_t)s.width * s.height, rays, nullptr);
+  return enqueue_views(ctx, std::vector<ViewRequest>{r}, (size_t)s.width * s.height, nullptr, nullptr);
 }
 
 GradRec grad_rec_carve(void* base, size_t paths, int bounces, bool whole) {
@@ -2320,8 +2345,7 @@ bc_status bc_render_rows(bc_context* ctx, const bc_camera* cam, const bc_setting
                          int32_t rows, float* linear_out, uint32_t* guide_out, int64_t* rays_out) {
   if (!ctx || !cam || !settings || !linear_out) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
   cudaSetDevice(ctx->device);
-  int64_t rays = 0;
-  bc_status st = render_rows_device(ctx, *cam, *settings, y0, rows, guide_out != nullptr, &rays);
+  bc_status st = enqueue_rows(ctx, *cam, *settings, y0, rows, guide_out != nullptr);
   if (st) return st;
   RenderBuffers* rb = ctx->rb;
   const int W = settings->width, npix = W * rows;
@@ -2330,10 +2354,8 @@ bc_status bc_render_rows(bc_context* ctx, const bc_camera* cam, const bc_setting
   if (!e && guide_out)
     e = cudaMemcpyAsync(guide_out, rb->guide_c + 3 * (size_t)y0 * W, 3 * sizeof(uint32_t) * (size_t)npix,
                         cudaMemcpyDeviceToHost, ctx->stream);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_status(ctx, e, "render readback");
-  if (rays_out) *rays_out = rays;
-  return BC_OK;
+  return wait_views(ctx, rays_out, "render readback");
 }
 
 bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, float* linear_out,
@@ -2341,8 +2363,7 @@ bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settin
   if (!ctx || !cam || !settings) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
   cudaSetDevice(ctx->device);
   const bool need_guides = settings->denoise || guide_out;
-  int64_t rays = 0;
-  bc_status st = render_rows_device(ctx, *cam, *settings, 0, settings->height, need_guides, &rays);
+  bc_status st = enqueue_rows(ctx, *cam, *settings, 0, settings->height, need_guides);
   if (st) return st;
   RenderBuffers* rb = ctx->rb;
   const int npix = settings->width * settings->height;
@@ -2350,7 +2371,7 @@ bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settin
   if ((st = run_post(ctx, *settings))) return st;
   // the frame's device time runs to the end of the post stack
   rb->launches += (settings->denoise ? std::max(0, 2 + std::min(3, std::max(settings->taa, settings->txaa))) : 0) +
-                  (settings->bloom > 0 ? 2 : 0) + 1;
+                  (settings->bloom > 3 ? 3 : 1);  // bloom of levels 1 to 3 tone maps too
   timing_end(ctx);
   cudaError_t e = cudaSuccess;
   if (linear_out)
@@ -2360,11 +2381,8 @@ bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settin
                         ctx->stream);
   if (!e && rgba_out)
     e = cudaMemcpyAsync(rgba_out, rb->rgba, sizeof(uint32_t) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_status(ctx, e, "frame readback");
-  timing_collect(ctx);
-  if (rays_out) *rays_out = rays;
-  return BC_OK;
+  return wait_views(ctx, rays_out, "frame readback");
 }
 
 bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, float* mean_out,
@@ -2374,8 +2392,7 @@ bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_sett
   cudaSetDevice(ctx->device);
   if (!ctx->rb) ctx->rb = new RenderBuffers();
   ctx->rb->want_sumsq = true;
-  int64_t rays = 0;
-  bc_status st = render_rows_device(ctx, *cam, *settings, 0, settings->height, false, &rays);
+  bc_status st = enqueue_rows(ctx, *cam, *settings, 0, settings->height, false);
   ctx->rb->want_sumsq = false;
   if (st) return st;
   RenderBuffers* rb = ctx->rb;
@@ -2384,10 +2401,8 @@ bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_sett
       cudaMemcpyAsync(mean_out, rb->out, 3 * sizeof(float) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
   if (!e)
     e = cudaMemcpyAsync(meansq_out, rb->post_tmp, 3 * sizeof(float) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_status(ctx, e, "moments readback");
-  if (rays_out) *rays_out = rays;
-  return BC_OK;
+  return wait_views(ctx, rays_out, "moments readback");
 }
 
 bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views, float* const* linear_out,
@@ -2398,8 +2413,7 @@ bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views
   long long px = 0;
   bc_status bst = batch_requests(ctx, views, n_views, &req, &px);
   if (bst) return bst;
-  int64_t rays = 0;
-  bc_status st = render_views(ctx, req, (size_t)px, &rays, nullptr);
+  bc_status st = enqueue_views(ctx, req, (size_t)px, nullptr, nullptr);
   if (st) return st;
   RenderBuffers* rb = ctx->rb;
   cudaError_t e = cudaSuccess;
@@ -2408,10 +2422,8 @@ bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views
       e = cudaMemcpyAsync(linear_out[v], rb->out + 3 * (size_t)req[v].pix_off,
                           3 * sizeof(float) * (size_t)req[v].s.width * req[v].s.height, cudaMemcpyDeviceToHost,
                           ctx->stream);
-  if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_status(ctx, e, "batch readback");
-  if (rays_out) *rays_out = rays;
-  return BC_OK;
+  return wait_views(ctx, rays_out, "batch readback");
 }
 
 }  // extern "C"
