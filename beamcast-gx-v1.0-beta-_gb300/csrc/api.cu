@@ -223,6 +223,7 @@ static bc_status install_scene(bc_context* ctx, const PackedScene& ps, const std
   ds.n_prims = ps.n_prims;
   ds.stack_need = ps.stack_need;
   ds.has_spheres = ps.has_spheres;
+  ds.flat = ps.flat;
   for (int k = 0; k < 3; k++) {
     ds.lo[k] = ps.scene_lo[k];
     ds.hi[k] = ps.scene_hi[k];
@@ -271,6 +272,10 @@ static bc_status keep_geometry_map(bc_context* ctx, const bc_scene_desc& d, cons
   g.n_node8 = (int32_t)ps.nodes.size();
   g.has_tris = false;
   for (int32_t i = 0; i < d.n_prims && !g.has_tris; i++) g.has_tris = d.prim_kind[i] == BC_PRIM_TRIANGLE;
+  g.flat_topology.clear();
+  if (ps.flat)  // a geometry update asks flat_scene again, of this topology
+    for (const int32_t* a : {d.prim_kind, d.order, d.node_left, d.node_right, d.node_start, d.node_count})
+      g.flat_topology.emplace_back(a, a + (a == d.prim_kind || a == d.order ? d.n_prims : d.n_nodes));
   g.valid = true;
   return BC_OK;
 }

@@ -59,6 +59,7 @@ struct GeomInfo {
   bool valid = false;  // the resident scene came from bc_scene_upload and kept its BVH8 child map
   int32_t n_binary = 0, n_lights = 0, n_materials = 0, n_node8 = 0;
   bool has_tris = false;
+  std::vector<std::vector<int32_t>> flat_topology;  // of a flat scene: kinds, order, left, right, start, count
 };
 
 }  // namespace bcgx

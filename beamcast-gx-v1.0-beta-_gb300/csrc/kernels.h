@@ -21,6 +21,7 @@ struct DeviceScene {
   int32_t n_mats = 0, n_lights = 0, n_prims = 0;
   int32_t stack_need = 0;
   bool has_spheres = false;
+  bool flat = false;  // at most kFlatPrims primitives: the renderer tests them all
   float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // scene bounds (ray order grid)
 };
 

@@ -24,6 +24,9 @@ constexpr uint32_t kLeafBit = 0x80000000u;
 constexpr uint32_t kSlotMask = 0x07ffffffu;
 constexpr int32_t kMaxIndex = 1 << 27;
 
+// Scenes of at most kFlatPrims primitives can be traced without their tree.
+constexpr int kFlatPrims = 24;
+
 // Status bits written by kernels (never a trap): the host turns them into errors.
 constexpr unsigned kStatusStackOverflow = 1u;
 constexpr unsigned kStatusTimeout = 2u;

@@ -422,6 +422,52 @@ void pack_binary(const bc_scene_desc& d, std::vector<BinNode>* out) {
   }
 }
 
+bool flat_scene(const bc_scene_desc& d) {
+  if (d.n_prims < 1 || d.n_prims > kFlatPrims || d.n_nodes < 1) return false;
+  const auto inside = [](const double* lo, const double* hi, const double* box) {
+    for (int k = 0; k < 3; k++) {
+      const double slack = 1e-9 * (1.0 + std::fabs(lo[k]) + std::fabs(hi[k]));  // A + E1 rounds where B did not
+      if (!(lo[k] >= box[k] - slack && hi[k] <= box[k + 3] + slack)) return false;
+    }
+    return true;
+  };
+  std::vector<uint8_t> seen(d.n_prims, 0);
+  std::vector<int32_t> todo{0};
+  for (size_t visited = 0; !todo.empty(); visited++) {
+    if (visited >= (size_t)d.n_nodes) return false;
+    const int32_t i = todo.back();
+    todo.pop_back();
+    const double* box = d.node_box + 6 * (size_t)i;
+    if (d.node_count[i] == 0) {
+      for (const int32_t c : {d.node_left[i], d.node_right[i]}) {
+        if (!inside(d.node_box + 6 * (size_t)c, d.node_box + 6 * (size_t)c + 3, box)) return false;
+        todo.push_back(c);
+      }
+      continue;
+    }
+    for (int32_t s = d.node_start[i]; s < d.node_start[i] + d.node_count[i]; s++) {
+      if (seen[s]) return false;
+      seen[s] = 1;
+      const int32_t p = d.order[s];
+      double lo[3], hi[3];
+      for (int k = 0; k < 3; k++) {
+        if (d.prim_kind[p] == BC_PRIM_TRIANGLE) {
+          const double a = d.prim_a[3 * p + k], b = a + d.prim_e1[3 * p + k], c = a + d.prim_e2[3 * p + k];
+          lo[k] = std::min(a, std::min(b, c));
+          hi[k] = std::max(a, std::max(b, c));
+        } else {
+          lo[k] = d.prim_center[3 * p + k] - d.prim_radius[p];
+          hi[k] = d.prim_center[3 * p + k] + d.prim_radius[p];
+        }
+      }
+      if (!inside(lo, hi, box)) return false;
+    }
+  }
+  for (const uint8_t s : seen)
+    if (!s) return false;
+  return true;
+}
+
 bc_status pack_scene(const bc_scene_desc& d, PackedScene* out, std::string* err, const CollapseParams& cp) {
   bc_status st = validate(d, err);
   if (st != BC_OK) return st;
@@ -433,6 +479,7 @@ bc_status pack_scene(const bc_scene_desc& d, PackedScene* out, std::string* err,
     pack_binary(d, &out->bin);
     pack_materials(d, out);
     pack_lights(d, out);
+    out->flat = flat_scene(d);
     for (int k = 0; k < 3; k++) {
       out->scene_lo[k] = round_down_f32(d.node_box[k]);
       out->scene_hi[k] = round_up_f32(d.node_box[3 + k]);
@@ -504,6 +551,7 @@ bc_status pack_scene_set(const bc_scene_desc* d, int n, PackedScene* out, std::v
     out->depth = std::max(out->depth, ps.depth);
     out->stack_need = std::max(out->stack_need, ps.stack_need);
     out->has_spheres = out->has_spheres || ps.has_spheres;
+    out->flat = n == 1 && ps.flat;
     for (int a = 0; a < 3; a++) {  // bounds of the whole set
       out->scene_lo[a] = k == 0 ? ps.scene_lo[a] : std::min(out->scene_lo[a], ps.scene_lo[a]);
       out->scene_hi[a] = k == 0 ? ps.scene_hi[a] : std::max(out->scene_hi[a], ps.scene_hi[a]);

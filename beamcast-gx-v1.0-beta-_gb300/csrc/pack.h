@@ -24,6 +24,7 @@ struct PackedScene {
   int32_t n_prims = 0, n_binary = 0;
   int32_t depth = 0, stack_need = 0;
   bool has_spheres = false;
+  bool flat = false;  // flat_scene
   float scene_lo[3] = {0, 0, 0}, scene_hi[3] = {0, 0, 0};
 };
 
@@ -64,6 +65,10 @@ bc_status pack_scene(const bc_scene_desc& d, PackedScene* out, std::string* err,
 // `ranges[k]` tells where each scene starts. stack_need is the maximum.
 bc_status pack_scene_set(const bc_scene_desc* d, int n, PackedScene* out, std::vector<SceneRange>* ranges,
                          std::string* err, const CollapseParams& cp = CollapseParams());
+// Whether testing every primitive finds what a walk of the tree finds: at most
+// kFlatPrims primitives, each in exactly one leaf, inside all the boxes above it (a
+// caller's tree is otherwise only checked for bounds).
+bool flat_scene(const bc_scene_desc& d);
 // The caller's binary BVH as BinNode records (validated descriptor).
 void pack_binary(const bc_scene_desc& d, std::vector<BinNode>* out);
 // Sphere-light records and per-primitive light selection pdfs of a scene.

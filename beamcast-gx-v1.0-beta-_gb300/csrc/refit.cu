@@ -123,6 +123,16 @@ bc_status update_geometry(bc_context* ctx, const bc_scene_desc& d) {
   }
   if (!e) e = cudaStreamSynchronize(ctx->stream);  // the host arrays of lp die here
   if (e) return cuda_status(ctx, e, "geometry update");
+  if (!gi.flat_topology.empty()) {  // the boxes moved: do they still hold what lies below them?
+    bc_scene_desc t = d;
+    t.prim_kind = gi.flat_topology[0].data();
+    t.order = gi.flat_topology[1].data();
+    t.node_left = gi.flat_topology[2].data();
+    t.node_right = gi.flat_topology[3].data();
+    t.node_start = gi.flat_topology[4].data();
+    t.node_count = gi.flat_topology[5].data();
+    ctx->ds.flat = flat_scene(t);
+  }
   return BC_OK;
 }
 

@@ -406,6 +406,7 @@ __global__ void k_generate(const BatchState* __restrict__ bs, const ViewGPU* __r
 // All three compute the same hits.
 constexpr int kExtendVariants = 3;
 
+
 template <int STACK, bool SPH, int VAR>
 __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restrict__ views, PathState ps,
                                             const int* __restrict__ queue, WaveCounters* cnt, int cur,
@@ -455,6 +456,138 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
       __stcs(ps.hit + at, make_float2(leaf.best_t, __int_as_float(leaf.best_slot)));
       at = -1;
     }
+  }
+}
+
+// ---- scenes without a walk ---------------------------------------------------------
+// A scene of at most kFlatPrims primitives is not walked: every ray tests every
+// primitive from shared memory, in lockstep with its warp. A walk of such a tree spends
+// its time on control flow with half of the lanes idle. The hits are the walk's: the
+// tests are, and where its answer could hang on its order or on the rounding of a box
+// face (the two nearest hits within kFlatTie; a hit, or the ray's origin, as near to a
+// face as the slab test may place it wrongly; a ray of extreme size), the walk is asked,
+// by about one ray in a thousand. Bound by the issue of the tests. Per frame, walk against
+// flat: 9 primitives, 960 x 540: extend 350 -> 234 us, connect 137 -> 105 us; 1280 x 720:
+// 1,042 -> 659 and 292 -> 239 us; random triangles, 640 x 360, 16 samples: 4 of them 189
+// -> 111 us, 16: 212 -> 179, 24: 248 -> 229, 32: 271 -> 294; spheres 16: 221 -> 169, 32:
+// 253 -> 250: hence the line at 24. (Pairs of triangles through the two-wide fp32
+// instructions, or tests without branches and with one division at the end, were slower:
+// 1.0 to 1.3 times this.)
+constexpr float kFlatTie = 1e-5f;  // relative
+// How far the walk's slab test may place two faces of a box from one another wrongly:
+// each by 2^15 grid steps times 2^-24, a step being at most 2/255 of the node's extent
+// (3.1e-5 of it for the two), and by the roundings of p / d - o / d, a few 2^-24 of the
+// coordinates. Of the scene's extent and of the coordinates' size:
+constexpr float kFlatFace = 4e-5f, kFlatRound = 1e-6f;
+constexpr float kFlatLargest = 1e6f;  // coordinates beyond are the walk's
+
+struct FlatScene {
+  float4 tri[3 * kFlatPrims];
+  float2 shape[kFlatPrims];  // of a triangle: its least altitude over |E1 x E2|, and 1 / |E1 x E2|
+};
+
+__device__ __forceinline__ void load_flat(FlatScene& f, const float4* __restrict__ tri, int n_slots) {
+  for (int k = threadIdx.x; k < 3 * n_slots; k += blockDim.x) f.tri[k] = tri[k];
+  for (int k = threadIdx.x; k < n_slots; k += blockDim.x) {
+    const float4 E1 = tri[3 * k + 1], E2 = tri[3 * k + 2];
+    const float3 e1 = f3(E1.x, E1.y, E1.z), e2 = f3(E2.x, E2.y, E2.z), e3 = e2 - e1;
+    const float3 n = f3(fdiff(e1.y, e2.z, e1.z, e2.y), fdiff(e1.z, e2.x, e1.x, e2.z), fdiff(e1.x, e2.y, e1.y, e2.x));
+    const float longest = sqrtf(fmaxf(dot3(e1, e1), fmaxf(dot3(e2, e2), dot3(e3, e3))));
+    f.shape[k] = make_float2(1.0f / longest, 1.0f / sqrtf(dot3(n, n)));  // altitude = |E1 x E2| / longest
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ float largest_of(float x, float y, float z) {
+  return fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
+}
+// Whether the ray is one for the flat tests; adds its share to `face`, the distance that
+// a hit has to keep from box faces.
+__device__ __forceinline__ bool flat_ray(const Ray32& r, float* face) {
+  const float o = largest_of(r.ox, r.oy, r.oz), d = largest_of(r.dx, r.dy, r.dz);
+  *face += kFlatRound * o;
+  return o < kFlatLargest && d < kFlatLargest && d > 1.0f / kFlatLargest;  // false for a NaN
+}
+
+// tri_hit32 or sphere_hit32 of slot s, and by how much the hit is clear of box faces and
+// the ray's origin of the face that the hit lies on: distances, less where the ray meets
+// the surface at a low angle and moves far along it while a face moves little. The faces
+// of a triangle's box meet its edges or contain it, those of a sphere's box touch it.
+template <bool SPH>
+__device__ __forceinline__ bool flat_hit(const FlatScene& f, int s, const Ray32& r, float tmax, float* t,
+                                         float* clear) {
+  const float4 A = f.tri[3 * s], E1 = f.tri[3 * s + 1], E2 = f.tri[3 * s + 2];
+  if (SPH && E2.w < 0.0f) {
+    if (!sphere_hit32(A, E1, r, tmax, t)) return false;
+    const float x = fmaf(*t, r.dx, r.ox) - A.x, y = fmaf(*t, r.dy, r.oy) - A.y, z = fmaf(*t, r.dz, r.oz) - A.z;
+    const float cosine = fabsf(x * r.dx + y * r.dy + z * r.dz) * E1.y;  // E1.y = 1 / radius
+    *clear = cosine * fminf(*t, A.w - largest_of(x, y, z));
+    return true;
+  }
+  float u, v, adet;
+  if (!tri_hit32(A, E1, E2, r, tmax, t, &u, &v, &adet)) return false;
+  const float2 shape = f.shape[s];
+  *clear = fminf(fminf(fminf(u, v), adet - u - v) * shape.x, *t * adet * shape.y);
+  return true;
+}
+
+template <int STACK, class Leaf>
+__device__ __forceinline__ void walk_fast(const SceneView& sv, const Ray32& r, Leaf& leaf, unsigned* status) {
+  FastWalker<STACK, kLeafVote> w;
+  w.reset(r);
+  while (!w.step(sv, r, leaf, status)) {
+  }
+}
+template <int STACK, bool SPH>
+__device__ __noinline__ float2 walk_closest(const SceneView* sv, const Ray32* r, unsigned* status) {
+  FastClosestLeaf<SPH> leaf(*sv, *r, 1e30f);
+  walk_fast<STACK>(*sv, *r, leaf, status);
+  return make_float2(leaf.best_t, __int_as_float(leaf.best_slot));
+}
+template <int STACK, bool SPH>
+__device__ __noinline__ bool walk_any(const SceneView* sv, const Ray32* r, float tmax, unsigned* status) {
+  FastAnyLeaf<SPH> leaf(*sv, *r, tmax);
+  walk_fast<STACK>(*sv, *r, leaf, status);
+  return leaf.done;
+}
+
+template <int STACK, bool SPH>
+__global__ void __launch_bounds__(128, 10)
+    k_extend_flat(SceneView sv, int n_slots, float scene_face, PathState ps, const int* __restrict__ queue,
+                  WaveCounters* cnt, int cur, unsigned* status) {
+  __shared__ FlatScene f;
+  const int n = *((volatile int*)&cnt->q[cur]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    atomicAdd(&cnt->rays, (unsigned long long)n);
+    cnt->q[cur ^ 1] = 0;  // the queue and shadow list this bounce's shade fills
+    cnt->shadow = 0;
+    cnt->gather = 0;
+  }
+  if (blockIdx.x * blockDim.x >= n) return;
+  load_flat(f, sv.tri, n_slots);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const size_t path = (size_t)queue[i];
+    const float4 o = sld(ps.ray + 2 * path), d = sld(ps.ray + 2 * path + 1);
+    const Ray32 r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, 1e-4f);
+    float face = scene_face, best = 1e30f, limit = 1e30f;
+    const bool usual = flat_ray(r, &face);
+    int slot = -1;
+    float clear = 1e30f;  // of the nearest hit
+    for (int s = 0; s < n_slots; s++) {
+      float t, c;
+      if (flat_hit<SPH>(f, s, r, limit, &t, &c)) {  // nearer than best, or hardly farther
+        clear = t < best * (1.0f - kFlatTie) ? c : 0.0f;
+        if (t < best) {
+          best = t;
+          limit = t * (1.0f + kFlatTie);
+          slot = s;
+        }
+      }
+    }
+    float2 hit = make_float2(best, __int_as_float(slot));
+    const bool sure = usual && clear > face && best > 2.0f * r.tmin;
+    if (!sure) hit = walk_closest<STACK, SPH>(&sv, &r, status);
+    __stcs(ps.hit + i, hit);
   }
 }
 
@@ -1116,6 +1249,19 @@ __global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ view
 }
 
 // ---- connect -----------------------------------------------------------------
+// Shadow ray i met no occluder: its light sample counts.
+__device__ __forceinline__ void add_unoccluded(const PathState& ps, const ShadowSoA& sh, const RecurRec& rr, int i) {
+  const int path = sh.path[i];
+  const float4 c = sh.c[i];
+  const int tag = __float_as_int(c.w);  // 0, or the recursive record's bounce + 1
+  if (tag == 0) {
+    const float4 L = ps.L[path];
+    ps.L[path] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0.0f);
+  } else {
+    rr.a[(size_t)(tag - 1) * rr.cap + path].w = 1.0f;
+  }
+}
+
 template <int STACK, bool SPH>
 __global__ void __launch_bounds__(128) k_connect(SceneView sv, PathState ps, ShadowSoA sh, WaveCounters* cnt,
                                                  RecurRec rr, long long sh_cap, unsigned* status) {
@@ -1153,19 +1299,33 @@ __global__ void __launch_bounds__(128) k_connect(SceneView sv, PathState ps, Sha
     }
     if (!__any_sync(0xffffffffu, i >= 0)) break;
     if (i >= 0 && w.step(sv, r, leaf, status)) {
-      if (!leaf.done) {  // no occluder: the light sample counts
-        const int path = sh.path[i];
-        const float4 c = sh.c[i];
-        const int tag = __float_as_int(c.w);  // 0, or the recursive record's bounce + 1
-        if (tag == 0) {
-          const float4 L = ps.L[path];
-          ps.L[path] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0.0f);
-        } else {
-          rr.a[(size_t)(tag - 1) * rr.cap + path].w = 1.0f;
-        }
-      }
+      if (!leaf.done) add_unoccluded(ps, sh, rr, i);
       i = -1;
     }
+  }
+}
+
+template <int STACK, bool SPH>
+__global__ void __launch_bounds__(128, 10)
+    k_connect_flat(SceneView sv, int n_slots, float scene_face, PathState ps, ShadowSoA sh, WaveCounters* cnt,
+                   RecurRec rr, long long sh_cap, unsigned* status) {
+  __shared__ FlatScene f;
+  const int n = (int)min((long long)*((volatile int*)&cnt->shadow), sh_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&cnt->shadow_rays, (unsigned long long)n);
+  if (blockIdx.x * blockDim.x >= n) return;
+  load_flat(f, sv.tri, n_slots);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 o = sh.o[i], d = sh.d[i];
+    const Ray32 r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, 1e-4f);
+    float face = scene_face;
+    const bool usual = flat_ray(r, &face);
+    bool occluded = false;
+    float t = 0.0f, clear = 1e30f;
+    for (int s = 0; s < n_slots && !occluded; s++) occluded = flat_hit<SPH>(f, s, r, o.w, &t, &clear);
+    const bool sure =
+        usual && (!occluded || (clear > face && t > 2.0f * r.tmin && t < o.w * (1.0f - kFlatTie)));
+    if (!sure) occluded = walk_any<STACK, SPH>(&sv, &r, o.w, status);
+    if (!occluded) add_unoccluded(ps, sh, rr, i);
   }
 }
 
@@ -1814,6 +1974,8 @@ struct WaveShape {
   bool lights;
   const GradArgs* grad;  // non-null: gradient render
   const GradRec* keep;   // non-null: leaves every path's vertex records there
+  bool flat;             // the scene is not walked (k_extend_flat, k_connect_flat)
+  float flat_face;       // what a hit there keeps clear of a box face
   bool adaptive;         // the batch has views that sample adaptively
   bool recursive;        // the batch has views of the recursive integrator
   bool photon;           // the batch has views of the photon integrator
@@ -1871,7 +2033,10 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
   // zeroes the work counters of the next extend and of its connect.
   for (int b = 0; b < w.bounces; b++) {
     rb->mark(st, kTimeExtend);
-    if (w.ext == 0)
+    if (w.flat)
+      k_extend_flat<STACK, SPH><<<sm_count() * 40, 128, 0, st>>>(sc.sv, ctx->ds.n_prims, w.flat_face, rb->ps,
+                                                                 rb->q[cur], c, cur, ctx->d_status);
+    else if (w.ext == 0)
       k_extend<STACK, SPH><<<w.ext_grid, 128, 0, st>>>(sc.sv, rb->views, rb->ps, rb->q[cur], c, cur, ctx->d_status);
     else if (w.ext == 2)
       k_extend_12<STACK, SPH><<<w.ext_grid, 128, 0, st>>>(sc.sv, rb->views, rb->ps, rb->q[cur], c, cur, ctx->d_status);
@@ -1908,7 +2073,10 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
                                                   w.gather_sort ? rb->ga.perm : rb->ga.list);
     }
     if (w.lights) rb->mark(st, kTimeConnect);
-    if (w.lights)
+    if (w.lights && w.flat)
+      k_connect_flat<STACK, SPH><<<sm_count() * 20, 128, 0, st>>>(sc.sv, ctx->ds.n_prims, w.flat_face, rb->ps, rb->sh,
+                                                                  c, rr, rb->sh_cap, ctx->d_status);
+    else if (w.lights)
       k_connect<STACK, SPH><<<w.con_grid, 128, 0, st>>>(sc.sv, rb->ps, rb->sh, c, rr, rb->sh_cap, ctx->d_status);
     cur ^= 1;
   }
@@ -1919,8 +2087,8 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
   rb->mark(st, kTimeAccumulate);
   if (w.keep) k_keep_radiance<<<w.acc_grid, 256, 0, st>>>(rb->bs, rb->ps, w.keep->L);
   const auto accumulate = w.recursive ? k_accumulate<true> : k_accumulate<false>;
-  accumulate<<<w.acc_grid * (w.recursive ? 1 : 2), 256, 0, st>>>(rb->bs, rb->views, rb->ps, rb->sum, rb->want_sumsq ? rb->sumsq : nullptr,
-                                         rb->adapt, rr);
+  accumulate<<<w.acc_grid * (w.recursive ? 1 : 2), 256, 0, st>>>(
+      rb->bs, rb->views, rb->ps, rb->sum, rb->want_sumsq ? rb->sumsq : nullptr, rb->adapt, rr);
   rb->mark(st, kTimeOther);
   k_advance<<<1, 32, 0, st>>>(rb->bs, c);
   return cudaGetLastError();
@@ -1939,6 +2107,14 @@ static bc_status run_waves(bc_context* ctx, int bounces, const BatchKinds& kinds
   WaveShape w = wave_shape<STACK, SPH>(wave_paths, bounces, lights, grad, ctx->render_extend, ctx->render_shade_block);
   w.keep = keep;
   w.adaptive = kinds.adaptive;
+  float size = 0.0f, extent = 0.0f;
+  for (int k = 0; k < 3; k++) {
+    const float lo = (float)ctx->ranges[0].lo[k], hi = (float)ctx->ranges[0].hi[k];
+    size = std::max(size, std::max(std::fabs(lo), std::fabs(hi)));
+    extent = std::max(extent, hi - lo);
+  }
+  w.flat = ctx->ds.flat && size < kFlatLargest;
+  w.flat_face = kFlatFace * extent + kFlatRound * size;
   w.recursive = recursive;
   w.photon = photon_entries > 0;
   w.gather_sort = w.photon && wave_paths >= kGatherSortPaths;
@@ -1969,6 +2145,8 @@ static bc_status run_waves(bc_context* ctx, int bounces, const BatchKinds& kinds
     add_bytes(&rb->ps, sizeof(rb->ps));
     add_bytes(&rb->sh, sizeof(rb->sh));
     key.push_back((uintptr_t)rb->sh_cap);
+    key.push_back(w.flat ? (uintptr_t)ctx->ds.n_prims : 0);
+    add_bytes(&w.flat_face, sizeof(w.flat_face));
     key.push_back((uintptr_t)recursive + 2 * (uintptr_t)w.adaptive);
     if (recursive) add_bytes(&rb->rr, sizeof(rb->rr));
     key.push_back((uintptr_t)(w.photon ? 1 + w.gather_sort : 0));

@@ -312,7 +312,9 @@ __device__ __forceinline__ float fdot(float ax, float ay, float az, float bx, fl
 // Plain fp32 triangle test for rendering (reference thresholds), with the
 // barycentric and distance tests on the numerators (u det, v det, t det
 // against det), so a missed triangle costs no division.
-__device__ __forceinline__ bool tri_hit32(float4 A, float4 E1, float4 E2, const Ray32& r, float tmax, float* t_out) {
+// u_out, v_out, det_out: the barycentric numerators and |det| of a hit.
+__device__ __forceinline__ bool tri_hit32(float4 A, float4 E1, float4 E2, const Ray32& r, float tmax, float* t_out,
+                                          float* u_out = nullptr, float* v_out = nullptr, float* det_out = nullptr) {
   const float hx = fdiff(r.dy, E2.z, r.dz, E2.y);
   const float hy = fdiff(r.dz, E2.x, r.dx, E2.z);
   const float hz = fdiff(r.dx, E2.y, r.dy, E2.x);
@@ -333,6 +335,11 @@ __device__ __forceinline__ bool tri_hit32(float4 A, float4 E1, float4 E2, const 
   const float t = __fdiv_rn(eq, det);
   if (t < r.tmin || t > tmax) return false;
   *t_out = t;
+  if (u_out) {
+    *u_out = un;
+    *v_out = vn;
+    *det_out = adet;
+  }
   return true;
 }
 

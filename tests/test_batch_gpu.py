@@ -162,3 +162,65 @@ def test_batch_argument_errors(gpu_ctx):
     a = gpu_ctx.render_frame(cams[0], st, want_guides=False, want_rgba=False)["linear"]
     b, _ = gpu_ctx.render_batch([(0, cams[0], st)])
     assert np.array_equal(a, b[0])
+
+
+def _soup(n_tris, n_spheres, seed):
+    r = np.random.default_rng(seed)
+    sp = scenes.SceneSpec(name="soup")
+    mats = [sp.material(bcgx.Material(kind=k, color=(0.8, 0.7, 0.6), roughness=0.1, ior=1.5)) for k in (0, 1, 2)]
+    light = sp.material(bcgx.Material(kind=3, emission=(6.0, 5.0, 4.0)))
+    if n_tris:
+        c = r.random((n_tris, 1, 3))
+        v = c + (r.random((n_tris, 3, 3)) - 0.5) * 1.5
+        v[::3, :, 1] = np.round(v[::3, :, 1])  # axis-aligned ones: boxes without thickness
+        sp.triangles(v.reshape(n_tris, 9), r.integers(0, 3, n_tris))
+    for i in range(n_spheres):
+        sp.sphere(r.random(3), 0.25, light if i == 0 else mats[i % 3])
+    return sp
+
+
+@pytest.mark.parametrize("n_tris,n_spheres", [(1, 0), (2, 1), (0, 24), (23, 1), (24, 0), (25, 0), (12, 13)])
+def test_unwalked_scenes_match_the_walk(gpu_ctx, n_tris, n_spheres):
+    """A scene of at most 24 primitives resident alone is rendered without its tree; in a
+    set of two it is walked. Same images, bit for bit."""
+    sc = scenes.to_scene(_soup(n_tris, n_spheres, 7 * n_tris + n_spheres))
+    cams = [bcgx.Camera((0.5, 0.5, 2.8), (0.5, 0.5, 0.5), (0, 1, 0), 50.0),
+            bcgx.Camera((0.4, 0.6, 0.5), (0.9, 0.1, 0.2), (0, 1, 0), 90.0)]
+    views = [(0, cams[k], _settings(160, 120, 16, 8, 50 + k)) for k in range(2)]
+    gpu_ctx.upload_set([sc, sc], set_id=900 + n_tris, revision=1)
+    walked, rays_walked = gpu_ctx.render_batch(views)
+    gpu_ctx.upload(sc)
+    flat, rays_flat = gpu_ctx.render_batch(views)
+    assert rays_flat == rays_walked
+    for a, b in zip(flat, walked):
+        assert np.array_equal(a, b)
+
+
+def test_unwalked_scene_needs_a_sound_tree(gpu_ctx):
+    """A tree that leaves a primitive outside its boxes is walked, as the caller built it,
+    also when a geometry update brings such boxes, and no longer when one mends them."""
+    sc = scenes.to_scene(_soup(9, 0, 3))
+    views = [(0, bcgx.Camera((0.5, 0.5, 2.8), (0.5, 0.5, 0.5), (0, 1, 0), 50.0), _settings(96, 64, 4, 4, 5))]
+    good = sc.arrays()
+    boxes = good.node_box.copy()
+    leaf = int(np.flatnonzero(good.node_count)[0])
+
+    def shrink(a, on):
+        a.node_box[:] = boxes
+        if on:
+            a.node_box.reshape(-1, 6)[leaf, 3:] = a.node_box.reshape(-1, 6)[leaf, :3] + 1e-3
+
+    gpu_ctx.upload(good, scene_id=77, topology_rev=1, geometry_rev=1)
+    want, _ = gpu_ctx.render_batch(views)
+    shrink(good, True)
+    gpu_ctx.upload_set([good, good], set_id=78, revision=1)
+    cut, _ = gpu_ctx.render_batch(views)
+    assert not np.array_equal(cut[0], want[0])
+    gpu_ctx.upload(good, scene_id=79, topology_rev=1, geometry_rev=1)
+    assert np.array_equal(gpu_ctx.render_batch(views)[0][0], cut[0])
+    shrink(good, False)
+    gpu_ctx.upload(good, scene_id=80, topology_rev=1, geometry_rev=1)
+    for rev, on in ((2, True), (3, False)):  # updates of the resident scene's geometry
+        shrink(good, on)
+        gpu_ctx.upload(good, scene_id=80, topology_rev=1, geometry_rev=rev)
+        assert np.array_equal(gpu_ctx.render_batch(views)[0][0], cut[0] if on else want[0])
