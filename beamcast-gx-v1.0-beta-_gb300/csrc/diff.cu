@@ -300,7 +300,8 @@ bc_status bc_backward(bc_context* ctx, const float* dloss_dimage, float* grad_al
   ga.mat2param = d.d_mat2param.as<int32_t>();
   ga.n_params = np;
   ga.partial = d.d_partial.as<double>();
-  if (d.kept && ctx->has_scene && d.kept_gen == ctx->scene_gen) {
+  const bool from_records = d.kept && ctx->has_scene && d.kept_gen == ctx->scene_gen;
+  if (from_records) {
     if (*(volatile int*)ctx->h_cancel || ctx->cancel.load()) return set_error(ctx, BC_ERR_CANCELLED, "render cancelled");
     const int spp = effective_spp(d.st);
     e = gradient_from_records(ctx, d.rec, (long long)px * spp, (int)px, spp, ga);
@@ -316,6 +317,7 @@ bc_status bc_backward(bc_context* ctx, const float* dloss_dimage, float* grad_al
   if (!e) e = cudaMemcpyAsync(h, d.d_grad.p, np3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
   if (!e) e = cudaStreamSynchronize(ctx->stream);
   if (e) return cuda_status(ctx, e, "gradient readback");
+  if (from_records) collect_timing(ctx);
   for (int k = 0; k < np3; k++) {
     if (k < 3 * d.n_alb) {
       if (grad_albedo) grad_albedo[k] = (float)h[k];

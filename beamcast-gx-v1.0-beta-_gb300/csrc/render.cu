@@ -2501,7 +2501,7 @@ static bc_status enqueue_rows(bc_context* ctx, const bc_camera& cam, const bc_se
 
 GradRec grad_rec_carve(void* base, size_t paths, int bounces, bool whole) {
   char* p = (char*)base;
-  GradRec r;
+  GradRec r{};  // its bytes, padding too, are part of a captured wave's key
   r.v = carve<float4>(p, paths * bounces);
   r.L = whole ? carve<float4>(p, paths) : nullptr;
   r.m = carve<int32_t>(p, paths * bounces);
@@ -2512,10 +2512,14 @@ GradRec grad_rec_carve(void* base, size_t paths, int bounces, bool whole) {
 
 cudaError_t gradient_from_records(bc_context* ctx, const GradRec& rec, long long n, int npix, int spp,
                                   const GradArgs& ga) {
+  timing_begin(ctx);
   k_gradient_kept<<<gradient_grid(), kGradThreads, 3 * ga.n_params * sizeof(double), ctx->stream>>>(
       rec, n, npix, spp, ga, ctx->ds.mats);
+  ctx->rb->launches++;
+  timing_end(ctx);
   return cudaGetLastError();
 }
+void collect_timing(bc_context* ctx) { timing_collect(ctx); }
 
 float* render_mean(bc_context* ctx) { return ctx->rb ? ctx->rb->out : nullptr; }
 

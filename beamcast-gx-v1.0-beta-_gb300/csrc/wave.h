@@ -47,9 +47,11 @@ struct GradArgs {
 // integrator, fixed samples, the wave engine).
 bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
                        const GradArgs* grad, const GradRec* keep = nullptr);
-// The gradient of one view's `n` paths (sample-major over npix pixels) from kept records.
+// The gradient of one view's `n` paths (sample-major over npix pixels) from kept records;
+// collect_timing once the stream has drained (bc_last_timing).
 cudaError_t gradient_from_records(bc_context* ctx, const GradRec& rec, long long n, int npix, int spp,
                                   const GradArgs& ga);
+void collect_timing(bc_context* ctx);
 float* render_mean(bc_context* ctx);
 
 // Photon maps (photon.cu). photon_map_for returns the map of resident scene
