@@ -250,8 +250,12 @@ __device__ __forceinline__ TriClass tri_classify(float4 A, float4 E1, float4 E2,
 // error 8u of tc times |d|, two of the fused sum), so E = 64u (max|C| + max|oc|)
 // bounds |perp|'s error with a factor two to spare, and E / |d| (and 16u |tc|)
 // that of tc. The margins exceed the rounding of the fp64 test's discriminant by
-// far (relative to |oc|^2: 1e-11 against 1e-15). Comparisons with a NaN are false:
-// such a sphere is undecided.
+// far (relative to |oc|^2: 1e-11 against 1e-15).
+// The bounds hold while no square or product overflows, so a ray or sphere of
+// extreme size is undecided: |d|^2 beyond 1e30 (and within 2 of the fp64 test's
+// limit 1e-18, where rounding could take the other side), coordinates, distances or
+// radii beyond 1e15, and NaNs, which fail these comparisons or, in the origin, the
+// later ones. E's constant covers squares that underflow (lengths below 1e-21).
 // The fp64 test costs a warp some 60 operations of a pipe with 1/64 of the fp32
 // rate: with it at every sphere of every visited leaf, 200,003 camera rays over
 // 822 spheres took 102 us; with this test and one settlement per ray, 34 us.
@@ -261,16 +265,17 @@ __device__ __forceinline__ TriClass sphere_classify(float4 C, const Ray32& r, fl
   c.t = 0.0f;
   c.et = __int_as_float(0x7f800000);
   const float dl2 = r.dx * r.dx + r.dy * r.dy + r.dz * r.dz;
-  if (!(dl2 > 1e-18f)) return c;
+  if (!(dl2 > 2e-18f && dl2 < 1e30f)) return c;
   const float ocx = r.ox - C.x, ocy = r.oy - C.y, ocz = r.oz - C.z;
   const float inv = 1.0f / dl2, il = sqrtf(inv);
   const float tc = -(ocx * r.dx + ocy * r.dy + ocz * r.dz) * inv;
   const float px = fmaf(tc, r.dx, ocx), py = fmaf(tc, r.dy, ocy), pz = fmaf(tc, r.dz, ocz);
   const float p2 = px * px + py * py + pz * pz;
   const float M = fmaxf(fabsf(C.x), fmaxf(fabsf(C.y), fabsf(C.z))) + fmaxf(fabsf(ocx), fmaxf(fabsf(ocy), fabsf(ocz)));
-  const float E = fmaf(64.0f * kU, M, 1e-30f);
+  const float E = fmaf(64.0f * kU, M, 1e-21f);
   const float rad = fabsf(C.w), rhi = rad * (1.0f + 8.0f * kU), rlo = rad * (1.0f - 8.0f * kU);
   const float lim = rhi + E;
+  if (!(fmaxf(M, rad) < 1e15f)) return c;
   if (p2 > lim * lim * (1.0f + 16.0f * kU)) {
     c.state = kMiss;
     return c;

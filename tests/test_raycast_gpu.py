@@ -405,3 +405,27 @@ def test_sphere_edges_parity(gpu_ctx, orc, offset):
     _check(gpu_ctx, ref, rays)
     occ_ref, _ = ref.occluded_f32(rays)
     assert np.array_equal(gpu_ctx.occluded(rays), occ_ref)
+
+
+# |d|^2 or o.d beyond the range of fp32 for the last three, and around the fp64 test's
+# limit |d|^2 = 1e-18 for the first.
+@pytest.mark.parametrize("length", [1e-9, 1e-4, 1e10, 1e18, 2e19, 1e25, 1e30])
+def test_sphere_direction_lengths_parity(gpu_ctx, orc, length):
+    """No limit is stated on the length of a direction: hits lie at distances in units of it."""
+    rng = np.random.default_rng(23)
+    spec = scenes.SceneSpec(name="spheres", bvh_mode="SAH", bvh_bins=16, bvh_leaf=4)
+    m = spec.material(scenes.Material(scenes.MAT_DIFFUSE, (0.5, 0.5, 0.5)))
+    for c, r in zip(rng.uniform(-4, 4, (60, 3)), rng.uniform(0.2, 0.9, 60)):
+        spec.sphere(c, r, m)
+    k = 8192
+    rays = np.zeros((k, 8), np.float32)
+    rays[:, 0:3] = rng.uniform(-5, 5, (k, 3))
+    d = rng.normal(size=(k, 3))
+    d *= length * (1.0 + 1e-7 * rng.normal(size=(k, 1))) / np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 4:7], rays[:, 7] = d, 1e30
+    rays[::3, 7] = rng.uniform(0.0, 6.0, len(rays[::3])) / length
+    gpu_ctx.upload(scenes.to_scene(spec))
+    ref = orc.OracleScene.from_spec(spec)
+    _check(gpu_ctx, ref, rays)
+    occ_ref, _ = ref.occluded_f32(rays)
+    assert occ_ref.any() and np.array_equal(gpu_ctx.occluded(rays), occ_ref)
