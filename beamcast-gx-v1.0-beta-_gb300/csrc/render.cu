@@ -502,10 +502,12 @@ __device__ __forceinline__ float largest_of(float x, float y, float z) {
   return fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
 }
 // Whether the ray is one for the flat tests; adds its share to `face`, the distance that
-// a hit has to keep from box faces.
-__device__ __forceinline__ bool flat_ray(const Ray32& r, float* face) {
+// a hit has to keep from box faces; *inv_len is 1 / |d| (a camera's rays are not of unit
+// length).
+__device__ __forceinline__ bool flat_ray(const Ray32& r, float* face, float* inv_len) {
   const float o = largest_of(r.ox, r.oy, r.oz), d = largest_of(r.dx, r.dy, r.dz);
   *face += kFlatRound * o;
+  *inv_len = 1.0f / sqrtf(dot3(f3(r.dx, r.dy, r.dz), f3(r.dx, r.dy, r.dz)));
   return o < kFlatLargest && d < kFlatLargest && d > 1.0f / kFlatLargest;  // false for a NaN
 }
 
@@ -513,21 +515,23 @@ __device__ __forceinline__ bool flat_ray(const Ray32& r, float* face) {
 // the ray's origin of the face that the hit lies on: distances, less where the ray meets
 // the surface at a low angle and moves far along it while a face moves little. The faces
 // of a triangle's box meet its edges or contain it, those of a sphere's box touch it.
+// adet and the sphere's x . d carry |d|: inv_len takes it out of the cosine beside a
+// distance along the surface, and t brings it to the distance to the origin.
 template <bool SPH>
-__device__ __forceinline__ bool flat_hit(const FlatScene& f, int s, const Ray32& r, float tmax, float* t,
-                                         float* clear) {
+__device__ __forceinline__ bool flat_hit(const FlatScene& f, int s, const Ray32& r, float inv_len, float tmax,
+                                         float* t, float* clear) {
   const float4 A = f.tri[3 * s], E1 = f.tri[3 * s + 1], E2 = f.tri[3 * s + 2];
   if (SPH && E2.w < 0.0f) {
     if (!sphere_hit32(A, E1, r, tmax, t)) return false;
     const float x = fmaf(*t, r.dx, r.ox) - A.x, y = fmaf(*t, r.dy, r.oy) - A.y, z = fmaf(*t, r.dz, r.oz) - A.z;
     const float cosine = fabsf(x * r.dx + y * r.dy + z * r.dz) * E1.y;  // E1.y = 1 / radius
-    *clear = cosine * fminf(*t, A.w - largest_of(x, y, z));
+    *clear = cosine * fminf(*t, (A.w - largest_of(x, y, z)) * inv_len);
     return true;
   }
   float u, v, adet;
   if (!tri_hit32(A, E1, E2, r, tmax, t, &u, &v, &adet)) return false;
   const float2 shape = f.shape[s];
-  *clear = fminf(fminf(fminf(u, v), adet - u - v) * shape.x, *t * adet * shape.y);
+  *clear = fminf(fminf(fminf(u, v), adet - u - v) * shape.x * inv_len, *t * adet * shape.y);
   return true;
 }
 
@@ -569,13 +573,13 @@ __global__ void __launch_bounds__(128, 10)
     const size_t path = (size_t)queue[i];
     const float4 o = sld(ps.ray + 2 * path), d = sld(ps.ray + 2 * path + 1);
     const Ray32 r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, 1e-4f);
-    float face = scene_face, best = 1e30f, limit = 1e30f;
-    const bool usual = flat_ray(r, &face);
+    float face = scene_face, inv_len, best = 1e30f, limit = 1e30f;
+    const bool usual = flat_ray(r, &face, &inv_len);
     int slot = -1;
     float clear = 1e30f;  // of the nearest hit
     for (int s = 0; s < n_slots; s++) {
       float t, c;
-      if (flat_hit<SPH>(f, s, r, limit, &t, &c)) {  // nearer than best, or hardly farther
+      if (flat_hit<SPH>(f, s, r, inv_len, limit, &t, &c)) {  // nearer than best, or hardly farther
         clear = t < best * (1.0f - kFlatTie) ? c : 0.0f;
         if (t < best) {
           best = t;
@@ -1317,11 +1321,11 @@ __global__ void __launch_bounds__(128, 10)
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 o = sh.o[i], d = sh.d[i];
     const Ray32 r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z, 1e-4f);
-    float face = scene_face;
-    const bool usual = flat_ray(r, &face);
+    float face = scene_face, inv_len;
+    const bool usual = flat_ray(r, &face, &inv_len);
     bool occluded = false;
     float t = 0.0f, clear = 1e30f;
-    for (int s = 0; s < n_slots && !occluded; s++) occluded = flat_hit<SPH>(f, s, r, o.w, &t, &clear);
+    for (int s = 0; s < n_slots && !occluded; s++) occluded = flat_hit<SPH>(f, s, r, inv_len, o.w, &t, &clear);
     const bool sure =
         usual && (!occluded || (clear > face && t > 2.0f * r.tmin && t < o.w * (1.0f - kFlatTie)));
     if (!sure) occluded = walk_any<STACK, SPH>(&sv, &r, o.w, status);

@@ -224,3 +224,32 @@ def test_unwalked_scene_needs_a_sound_tree(gpu_ctx):
         shrink(good, on)
         gpu_ctx.upload(good, scene_id=80, topology_rev=1, geometry_rev=rev)
         assert np.array_equal(gpu_ctx.render_batch(views)[0][0], cut[0] if on else want[0])
+
+
+@pytest.mark.parametrize("spheres", [False, True])
+@pytest.mark.parametrize("up_along_edge", [False, True])
+def test_unwalked_scene_matches_the_walk_at_the_rim_of_a_wide_view(gpu_ctx, spheres, up_along_edge):
+    """The edge where two least faces of the scene's boxes meet, seen from outside, forty
+    tangent units off the view axis: a camera's rays there are forty units long. The walk
+    loses some of the hits within 1e-5 of such an edge, whatever the rays' length."""
+    sp = scenes.SceneSpec(name="edge")
+    m = sp.material(bcgx.Material(kind=0, color=(0.8, 0.7, 0.6)))
+    light = sp.material(bcgx.Material(kind=3, emission=(5.0, 4.0, 3.0)))
+    sp.triangles(scenes.quad((0, 0, 0), (0, 1, 0), (0, 1, 1), (0, 0, 1)), m if spheres else light)
+    sp.triangles(scenes.quad((1, 0, 0), (1, 1, 0), (1, 1, 1), (1, 0, 1)), m)
+    for k in range(4 if spheres else 0):
+        sp.sphere((0.1, 0.1, 0.1 + 0.25 * k), 0.1, light)
+    sc = scenes.to_scene(sp)
+    eye, side, off = np.array([-0.5, 0.2, 0.5]), np.array([0.0, 0.0, 1.0]), 40.0
+    d = np.array([0.0, 0.0, 0.5]) - eye
+    d /= np.linalg.norm(d)
+    n = np.cross(d, side)
+    axis = (d + off * n) / np.hypot(1.0, off)
+    cam = bcgx.Camera(tuple(eye), tuple(eye + axis), tuple(side if up_along_edge else n),
+                      float(2 * np.degrees(np.arctan(1.02 * off + 0.1))))
+    views = [(0, cam, _settings(1280, 720, 128, 2, 7))]
+    gpu_ctx.upload_set([sc, sc], set_id=950 + 2 * spheres + up_along_edge, revision=1)
+    walked, rays_walked = gpu_ctx.render_batch(views)
+    gpu_ctx.upload(sc)
+    flat, rays_flat = gpu_ctx.render_batch(views)
+    assert rays_flat == rays_walked and np.array_equal(flat[0], walked[0])
