@@ -8,6 +8,7 @@ CPU fallback.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import math
 import threading
@@ -33,25 +34,33 @@ class _Outputs:
     caller has dropped every reference to it, and the next image of that size takes it:
     fresh memory of a frame's size is mapped page by page while the device copies into
     it, which takes far longer than the copy (a frame with guides, 960 x 540: 2.00 ->
-    1.12 ms; 1280 x 720: 6.04 -> 4.99 ms). Holds at most LIMIT bytes, given back with the context."""
+    1.12 ms; 1280 x 720: 6.04 -> 4.99 ms). A caller that keeps every image gets fresh memory each
+    time. Holds at most LIMIT bytes, given back with the context."""
     LIMIT = 256 << 20
     MIN = 256 << 10  # smaller arrays come from the allocator's heap, which stays mapped
 
     def __init__(self):
         self._free, self._bytes, self._open = [], 0, True
-        self._lock = threading.RLock()  # re-entrant: a collection may run a finalizer inside
+        # Finalizers run wherever a collection does, inside the locked parts below too, so
+        # they only append here; whoever holds the lock, or gets it, sorts the memory in.
+        self._returned = collections.deque()
+        self._lock = threading.Lock()
 
     def empty(self, shape, dtype) -> np.ndarray:
         n = math.prod(shape) * np.dtype(dtype).itemsize
         if n < self.MIN:
             return np.empty(shape, dtype)
         mem = None
-        with self._lock:
-            for i in range(len(self._free) - 1, -1, -1):
-                if self._free[i].nbytes == n:
-                    mem = self._free.pop(i)
-                    self._bytes -= n
-                    break
+        if self._lock.acquire(blocking=False):  # else another call has it: fresh memory
+            try:
+                for i in range(len(self._free) - 1, -1, -1):
+                    if self._free[i].nbytes == n:
+                        mem = self._free.pop(i)
+                        self._bytes -= n
+                        break
+            finally:
+                self._lock.release()
+            self._sort_in()
         if mem is None:
             mem = np.empty(n, np.uint8)
         owner = (C.c_char * n).from_buffer(mem)  # every view of the image keeps it alive
@@ -59,17 +68,27 @@ class _Outputs:
         return np.frombuffer(owner, dtype=dtype).reshape(shape)
 
     def _put(self, mem):
-        with self._lock:
-            if not self._open or mem.nbytes > self.LIMIT:
-                return
-            self._free.append(mem)
-            self._bytes += mem.nbytes
-            while self._bytes > self.LIMIT:  # the longest unused first
-                self._bytes -= self._free.pop(0).nbytes
+        self._returned.append(mem)
+        self._sort_in()
+
+    def _sort_in(self):
+        while self._returned and self._lock.acquire(blocking=False):
+            try:
+                while self._returned:
+                    mem = self._returned.popleft()
+                    if not self._open or mem.nbytes > self.LIMIT:
+                        continue
+                    self._free.append(mem)
+                    self._bytes += mem.nbytes
+                    while self._bytes > self.LIMIT:  # the longest unused first
+                        self._bytes -= self._free.pop(0).nbytes
+            finally:
+                self._lock.release()
 
     def close(self):
         with self._lock:
             self._free, self._bytes, self._open = [], 0, False
+        self._sort_in()
 
 
 class Context:

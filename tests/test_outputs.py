@@ -48,3 +48,48 @@ def test_memory_is_bounded_and_given_back(monkeypatch):
     assert pool._bytes == 0 and not pool._free
     small = pool.empty((4, 4), np.float32)
     assert small.flags.owndata
+
+
+class _Collects(np.ndarray):
+    """Memory in the pool whose look at the size runs a collection."""
+    run = None
+
+    @property
+    def nbytes(self):
+        if _Collects.run:
+            run, _Collects.run = _Collects.run, None
+            run()
+        return self.size
+
+
+@pytest.mark.parametrize("mb", [2, 3, 6])
+def test_memory_that_returns_inside_a_scan_shifts_nothing(monkeypatch, mb):
+    """A collection inside empty() may return other images, and their return may evict
+    what the scan has passed."""
+    monkeypatch.setattr(_Outputs, "LIMIT", 7 << 20)
+    pool = _Outputs()
+    pool._put(np.empty(3 << 20, np.uint8))
+    pool._put(np.empty(3 << 20, np.uint8).view(_Collects))
+    _Collects.run = lambda: pool._put(np.empty(mb << 20, np.uint8))
+    a = pool.empty((512, 512, 3), np.float32)
+    assert _Collects.run is None
+    a[:] = 1.0
+    assert a.sum() == a.size
+    assert pool._bytes == sum(m.size for m in pool._free) <= pool.LIMIT
+
+
+def test_pool_serves_several_threads():
+    import threading
+    pool, bad = _Outputs(), []
+
+    def work(k):
+        for i in range(300):
+            a = pool.empty((256, 256 + 64 * (i % 3)), np.float32)
+            a[:] = k
+            if not (a == k).all():
+                bad.append((k, i))
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad and pool._bytes == sum(m.nbytes for m in pool._free)
