@@ -529,6 +529,11 @@ bc_status bc_set_option(bc_context* ctx, const char* name, int64_t value) {
     ctx->test_status_bits = (unsigned)value;
     return BC_OK;
   }
+  if (n == "test_fail_readback") {  // test hook: the next render call takes its read-back to have failed
+    if (value != 0 && value != 1) return set_error(ctx, BC_ERR_INVALID_ARG, "test_fail_readback must be 0 or 1");
+    ctx->test_fail_readback = (int)value;
+    return BC_OK;
+  }
   if (n == "raycast_chunk") {
     if (value < 65536 || value > (1LL << 28))
       return set_error(ctx, BC_ERR_INVALID_ARG, "raycast_chunk must be in [65536, 2^28]");

@@ -101,6 +101,7 @@ struct bc_context {
   // read and cleared only by bc_sync, so their kernel status reaches their caller
   unsigned* d_status_async = nullptr;
   unsigned test_status_bits = 0;  // bc_set_option "test_status_bits": raised by the next device-pointer call
+  int test_fail_readback = 0;  // bc_set_option "test_fail_readback": the next render call's read-back fails
   // work counters of the persistent ray-cast kernels: [0], [1] the two streams of
   // bc_raycast, [2] bc_raycast_device
   unsigned long long* d_work = nullptr;

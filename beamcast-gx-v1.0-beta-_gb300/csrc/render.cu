@@ -2239,10 +2239,8 @@ static bc_status run_plain(bc_context* ctx, const ShadeScene& sc, const std::vec
   return BC_OK;
 }
 
-// Queues everything of render_views: the caller may queue more work on the frame behind
-// it and ends with wait_views.
-static bc_status enqueue_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px,
-                               const GradArgs* grad, const GradRec* keep) {
+static bc_status queue_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px,
+                             const GradArgs* grad, const GradRec* keep) {
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (req.empty()) return set_error(ctx, BC_ERR_INVALID_ARG, "no views");
   bc_status bst;
@@ -2468,6 +2466,25 @@ static bc_status enqueue_views(bc_context* ctx, const std::vector<ViewRequest>& 
   return cuda_status(ctx, e, "render");
 }
 
+// A call that fails with work queued: waits for it, so that nothing is written behind the
+// failed return (a copy into the caller's pinned memory, the read-back words), and drops
+// the kernel status of the render that is given up.
+static bc_status abandon_views(bc_context* ctx, bc_status st) {
+  const std::string why = ctx->err;
+  cudaStreamSynchronize(ctx->stream);
+  check_kernel_status(ctx);
+  cudaGetLastError();
+  return set_error(ctx, st, why);
+}
+
+// Queues everything of render_views: the caller may queue more work on the frame behind
+// it and ends with finish_views, or with abandon_views on an error.
+static bc_status enqueue_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px,
+                               const GradArgs* grad, const GradRec* keep) {
+  const bc_status st = queue_views(ctx, req, frame_px, grad, keep);
+  return st ? abandon_views(ctx, st) : BC_OK;
+}
+
 // Waits for the stream; the counters, timing and kernel status of the render that
 // enqueue_views queued.
 static bc_status wait_views(bc_context* ctx, int64_t* rays, const char* what) {
@@ -2480,6 +2497,13 @@ static bc_status wait_views(bc_context* ctx, int64_t* rays, const char* what) {
   if (rays) *rays = (int64_t)r;
   timing_collect(ctx);
   return h[0] ? check_kernel_status(ctx) : BC_OK;
+}
+
+// The end of a call whose read-back was queued with result `e`.
+static bc_status finish_views(bc_context* ctx, cudaError_t e, int64_t* rays, const char* what) {
+  if (!e && ctx->test_fail_readback) e = cudaErrorUnknown;
+  ctx->test_fail_readback = 0;
+  return e ? abandon_views(ctx, cuda_status(ctx, e, what)) : wait_views(ctx, rays, what);
 }
 
 bc_status render_views(bc_context* ctx, const std::vector<ViewRequest>& req, size_t frame_px, int64_t* rays,
@@ -2592,8 +2616,7 @@ bc_status bc_render_rows(bc_context* ctx, const bc_camera* cam, const bc_setting
   if (!e && guide_out)
     e = cudaMemcpyAsync(guide_out, rb->guide_c + 3 * (size_t)y0 * W, 3 * sizeof(uint32_t) * (size_t)npix,
                         cudaMemcpyDeviceToHost, ctx->stream);
-  if (e) return cuda_status(ctx, e, "render readback");
-  return wait_views(ctx, rays_out, "render readback");
+  return finish_views(ctx, e, rays_out, "render readback");
 }
 
 bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, float* linear_out,
@@ -2606,7 +2629,7 @@ bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settin
   RenderBuffers* rb = ctx->rb;
   const int npix = settings->width * settings->height;
   rb->mark(ctx->stream, kTimePost);
-  if ((st = run_post(ctx, *settings))) return st;
+  if ((st = run_post(ctx, *settings))) return abandon_views(ctx, st);
   // the frame's device time runs to the end of the post stack
   rb->launches += (settings->denoise ? std::max(0, 2 + std::min(3, std::max(settings->taa, settings->txaa))) : 0) +
                   (settings->bloom > 3 ? 3 : 1);  // bloom of levels 1 to 3 tone maps too
@@ -2619,8 +2642,7 @@ bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settin
                         ctx->stream);
   if (!e && rgba_out)
     e = cudaMemcpyAsync(rgba_out, rb->rgba, sizeof(uint32_t) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e) return cuda_status(ctx, e, "frame readback");
-  return wait_views(ctx, rays_out, "frame readback");
+  return finish_views(ctx, e, rays_out, "frame readback");
 }
 
 bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, float* mean_out,
@@ -2639,8 +2661,7 @@ bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_sett
       cudaMemcpyAsync(mean_out, rb->out, 3 * sizeof(float) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
   if (!e)
     e = cudaMemcpyAsync(meansq_out, rb->post_tmp, 3 * sizeof(float) * (size_t)npix, cudaMemcpyDeviceToHost, ctx->stream);
-  if (e) return cuda_status(ctx, e, "moments readback");
-  return wait_views(ctx, rays_out, "moments readback");
+  return finish_views(ctx, e, rays_out, "moments readback");
 }
 
 bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views, float* const* linear_out,
@@ -2660,8 +2681,7 @@ bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views
       e = cudaMemcpyAsync(linear_out[v], rb->out + 3 * (size_t)req[v].pix_off,
                           3 * sizeof(float) * (size_t)req[v].s.width * req[v].s.height, cudaMemcpyDeviceToHost,
                           ctx->stream);
-  if (e) return cuda_status(ctx, e, "batch readback");
-  return wait_views(ctx, rays_out, "batch readback");
+  return finish_views(ctx, e, rays_out, "batch readback");
 }
 
 }  // extern "C"

@@ -198,3 +198,41 @@ def test_render_argument_errors(gpu_ctx):
     assert e.value.status == 7
     with pytest.raises(bcgx.BCError):
         gpu_ctx.render_rows(cam, st, st.height - 1, 4)
+
+
+@pytest.mark.parametrize("call", ["rows", "frame", "moments", "batch"])
+def test_failed_readback_leaves_nothing_queued(gpu_ctx, call):
+    """A render call whose read-back fails returns with its work done: pinned memory it was
+    given is not written behind the return (the hook fails the call once the copies are
+    queued), and the next call is not affected."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    from bcgx._lib import lib
+    spec, cam, st = scenes.cornell_box()
+    st.width, st.height, st.spp, st.denoise, st.bloom = 1280, 720, 64, False, 0
+    gpu_ctx.upload(scenes.to_scene(spec))
+    h, cc, sc, n = gpu_ctx.handle, cam.c(), st.c(), st.width * st.height
+
+    def render(a, b):
+        pa, pb = (C.cast(x.data_ptr(), C.POINTER(C.c_float)) for x in (a, b))
+        if call == "rows":
+            return lib().bc_render_rows(h, C.byref(cc), C.byref(sc), 0, st.height, pa, None, None)
+        if call == "frame":
+            return lib().bc_render_frame(h, C.byref(cc), C.byref(sc), pa, None, None, None)
+        if call == "moments":
+            return lib().bc_render_moments(h, C.byref(cc), C.byref(sc), pa, pb, None)
+        v = (bcgx._lib.ViewC * 1)()
+        v[0].scene, v[0].reserved, v[0].camera, v[0].settings = 0, 0, cc, sc
+        return lib().bc_render_batch(h, v, 1, (C.POINTER(C.c_float) * 1)(pa), None)
+
+    def images():
+        return [torch.zeros(3 * n, dtype=torch.float32).pin_memory() for _ in range(2)]
+
+    want, got = images(), images()
+    assert render(*want) == 0 and float(want[0].sum()) > 0
+    gpu_ctx.set_option("test_fail_readback", 1)
+    assert render(*got) != 0
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])  # at once: nothing is pending
+    again = images()
+    assert render(*again) == 0 and torch.equal(again[0], want[0]) and torch.equal(again[1], want[1])
