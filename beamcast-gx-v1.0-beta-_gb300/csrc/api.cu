@@ -25,6 +25,30 @@ bc_status cuda_status(bc_context* ctx, cudaError_t e, const char* what) {
   return set_error(ctx, e == cudaErrorMemoryAllocation ? BC_ERR_OOM : BC_ERR_DEVICE, m);
 }
 
+static thread_local bc_context* t_context = nullptr;
+
+void use_context(bc_context* ctx) {
+  cudaSetDevice(ctx->device);
+  t_context = ctx;
+}
+
+static cudaError_t try_alloc(void** p, size_t bytes) {
+  if (t_context && t_context->test_fail_allocs > 0) {
+    t_context->test_fail_allocs--;
+    return cudaErrorMemoryAllocation;
+  }
+  return cudaMalloc(p, bytes);
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  cudaError_t e = try_alloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && t_context && release_kept_records(t_context)) {
+    cudaGetLastError();
+    e = try_alloc(p, bytes);
+  }
+  return e;
+}
+
 // Reads and clears a kernel status word once `stream` has drained.
 bc_status check_status_word(bc_context* ctx, unsigned* d_word, cudaStream_t stream) {
   unsigned h = 0;
@@ -142,8 +166,9 @@ bc_status bc_create(int device_ordinal, bc_context** out) {
 
 void bc_destroy(bc_context* ctx) {
   if (!ctx) return;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  t_context = nullptr;
   destroy_render_buffers(ctx);
   destroy_diff_state(ctx);
   destroy_post_state(ctx);
@@ -291,7 +316,7 @@ bc_status bc_scene_upload(bc_context* ctx, const bc_scene_desc* scene, uint64_t 
   if (ctx->has_scene && !ctx->is_set && ctx->scene_id == scene_id && ctx->topo_rev == topology_rev &&
       ctx->geom_rev == geometry_rev && same_pack)
     return BC_OK;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   bc_status st;
   if (ctx->has_scene && !ctx->is_set && ctx->scene_id == scene_id && ctx->topo_rev == topology_rev && same_pack) {
     // only the geometry moved: rewrite primitives and node boxes on the device
@@ -331,7 +356,7 @@ bc_status bc_scene_set_upload(bc_context* ctx, const bc_scene_desc* scenes, int3
   if (ctx->has_scene && ctx->is_set && ctx->scene_id == set_id && ctx->geom_rev == revision &&
       (int32_t)ctx->ranges.size() == n_scenes && ctx->packed_merge == ctx->scene_leaf_merge)
     return BC_OK;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   PackedScene ps;
   std::vector<SceneRange> ranges;
   std::string err;
@@ -362,7 +387,7 @@ bc_status bc_raycast_device(bc_context* ctx, const float* d_rays, int64_t n, flo
     return set_error(ctx, BC_ERR_INVALID_ARG, "bad ray-cast arguments");
   if (((uintptr_t)d_rays & 15u) != 0) return set_error(ctx, BC_ERR_INVALID_ARG, "rays must be 16-byte aligned");
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   void* order = nullptr;
   if (ctx->raycast_sort && n >= kMinOrderedRays && n < (int64_t(1) << 31)) {
@@ -390,7 +415,7 @@ bc_status bc_raycast(bc_context* ctx, const float* rays, int64_t n, float* t_out
   if (n < 0 || (n > 0 && (!rays || !t_out || !prim_out))) return set_error(ctx, BC_ERR_INVALID_ARG, "bad ray-cast arguments");
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (n == 0) return BC_OK;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaError_t e;
   if ((e = ctx->d_rays.ensure((size_t)n * 32)) || (e = ctx->d_t.ensure((size_t)n * 4)) ||
       (e = ctx->d_prim.ensure((size_t)n * 4)))
@@ -439,7 +464,7 @@ bc_status bc_occluded_device(bc_context* ctx, const float* d_rays, int64_t n, ui
   if (n < 0 || (n > 0 && (!d_rays || !d_out))) return set_error(ctx, BC_ERR_INVALID_ARG, "bad any-hit arguments");
   if (((uintptr_t)d_rays & 15u) != 0) return set_error(ctx, BC_ERR_INVALID_ARG, "rays must be 16-byte aligned");
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   void* rec = nullptr;
   void* order = nullptr;
@@ -460,7 +485,7 @@ bc_status bc_occluded_device(bc_context* ctx, const float* d_rays, int64_t n, ui
 
 bc_status bc_sync(bc_context* ctx, void* stream) {
   if (!ctx) return set_error(nullptr, BC_ERR_INVALID_ARG, "NULL context");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   return check_status_word(ctx, ctx->d_status_async, stream ? (cudaStream_t)stream : ctx->stream);
 }
 
@@ -469,7 +494,7 @@ bc_status bc_occluded(bc_context* ctx, const float* rays, int64_t n, uint8_t* ou
   if (n < 0 || (n > 0 && (!rays || !out))) return set_error(ctx, BC_ERR_INVALID_ARG, "bad any-hit arguments");
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (n == 0) return BC_OK;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaError_t e;
   if ((e = ctx->d_rays.ensure((size_t)n * 32)) || (e = ctx->d_occ.ensure((size_t)n)))
     return cuda_status(ctx, e, "any-hit buffers");
@@ -527,6 +552,20 @@ bc_status bc_set_option(bc_context* ctx, const char* name, int64_t value) {
   if (n == "test_status_bits") {  // test hook: the next device-pointer call raises these status bits
     if (value < 0 || value > 0xffffffffLL) return set_error(ctx, BC_ERR_INVALID_ARG, "test_status_bits is 32 bits");
     ctx->test_status_bits = (unsigned)value;
+    return BC_OK;
+  }
+  if (n == "diff_keep_records") {
+    if (value != 0 && value != 1) return set_error(ctx, BC_ERR_INVALID_ARG, "diff_keep_records must be 0 or 1");
+    ctx->diff_keep_records = (int)value;
+    if (!value) {
+      use_context(ctx);
+      release_kept_records(ctx);
+    }
+    return BC_OK;
+  }
+  if (n == "test_fail_allocs") {  // test hook: the context's next device allocations fail
+    if (value < 0 || value > 1000) return set_error(ctx, BC_ERR_INVALID_ARG, "test_fail_allocs must be in [0, 1000]");
+    ctx->test_fail_allocs = (int)value;
     return BC_OK;
   }
   if (n == "test_fail_readback") {  // test hook: the next render call takes its read-back to have failed
@@ -594,6 +633,7 @@ bc_status bc_get_option(const bc_context* ctx, const char* name, int64_t* value)
   if (n == "render_extend") { *value = ctx->render_extend; return BC_OK; }
   if (n == "render_shade_block") { *value = ctx->render_shade_block; return BC_OK; }
   if (n == "render_timing") { *value = ctx->render_timing; return BC_OK; }
+  if (n == "diff_keep_records") { *value = ctx->diff_keep_records; return BC_OK; }
   if (n == "scene_leaf_merge") { *value = ctx->scene_leaf_merge; return BC_OK; }
   return BC_ERR_INVALID_ARG;
 }

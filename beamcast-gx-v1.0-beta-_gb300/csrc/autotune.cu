@@ -65,7 +65,7 @@ extern "C" {
 bc_status bc_autotune_raycast(bc_context* ctx, const float* d_rays, int64_t n, bc_tune_report* out) {
   if (!ctx || !d_rays || n < 1) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument or no rays");
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaError_t e = ctx->d_t.ensure((size_t)n * 4);
   if (!e) e = ctx->d_prim.ensure((size_t)n * 4);
   if (e) return cuda_status(ctx, e, "autotune buffers");
@@ -121,7 +121,7 @@ bc_status bc_autotune_raycast(bc_context* ctx, const float* d_rays, int64_t n, b
 
 bc_status bc_autotune_render(bc_context* ctx, const bc_view* views, int32_t n_views, bc_tune_report* out) {
   if (!ctx || !views || n_views < 1) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument or no views");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   std::vector<ViewRequest> req;
   long long px = 0;
   bc_status st = batch_requests(ctx, views, n_views, &req, &px);

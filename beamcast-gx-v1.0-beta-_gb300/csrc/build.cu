@@ -986,7 +986,7 @@ extern "C" bc_status bc_build_sah(bc_context* ctx, int32_t n_prims, const double
   if (bins > 32) bins = 32;
   if (leaf_size < 1) leaf_size = 4;
   if (leaf_size > 16) leaf_size = 16;
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   return build_sah_device(ctx, n_prims, prim_box, centroid, bins, leaf_size, n_nodes_out, node_box, node_left,
                           node_right, node_start, node_count, order_out);
 }

@@ -12,6 +12,11 @@
 
 namespace bcgx {
 
+// Device memory for the context that this thread last entered (use_context). Where there
+// is none left, memory that the context can do without is given back first (the vertex
+// records kept by bc_forward).
+cudaError_t device_alloc(void** p, size_t bytes);  // api.cu
+
 // Growable device buffer owned by a context.
 struct DevBuf {
   void* p = nullptr;
@@ -21,7 +26,7 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = device_alloc(&p, bytes);
     if (e == cudaSuccess) cap = bytes;
     return e;
   }
@@ -101,6 +106,8 @@ struct bc_context {
   // read and cleared only by bc_sync, so their kernel status reaches their caller
   unsigned* d_status_async = nullptr;
   unsigned test_status_bits = 0;  // bc_set_option "test_status_bits": raised by the next device-pointer call
+  int diff_keep_records = 1;   // bc_forward keeps vertex records (bc_set_option "diff_keep_records")
+  int test_fail_allocs = 0;    // bc_set_option "test_fail_allocs": that many device allocations fail
   int test_fail_readback = 0;  // bc_set_option "test_fail_readback": the next render call's read-back fails
   // work counters of the persistent ray-cast kernels: [0], [1] the two streams of
   // bc_raycast, [2] bc_raycast_device
@@ -130,6 +137,9 @@ bc_status set_error(bc_context* ctx, bc_status st, const std::string& msg);
 bc_status cuda_status(bc_context* ctx, cudaError_t e, const char* what);
 bc_status check_kernel_status(bc_context* ctx);
 bc_status check_status_word(bc_context* ctx, unsigned* d_word, cudaStream_t stream);
+// Entry of a call: the context's device, and the context that device_alloc serves.
+void use_context(bc_context* ctx);
+bool release_kept_records(bc_context* ctx);  // diff.cu: false where there are none to give back
 void destroy_render_buffers(bc_context* ctx);
 void destroy_diff_state(bc_context* ctx);
 void destroy_post_state(bc_context* ctx);

@@ -21,6 +21,7 @@ struct DiffState {
   bcgx::DevBuf d_param_mat, d_mat2param, d_params, d_target, d_dimg, d_partial, d_grad, d_loss;
   bcgx::DevBuf d_kept;
   bcgx::HostBuf h_stage;
+  bool keeping = false;     // a forward render is writing them
   bool kept = false;        // d_kept holds the vertex records of the last forward,
   uint64_t kept_gen = 0;    // rendered from this upload of the scene
   bcgx::GradRec rec{};
@@ -107,13 +108,34 @@ __global__ void k_sum_rows(const double* __restrict__ partial, int rows, int col
 // (the path integrator with every sample taken, through the wave engine). Keeping them
 // costs a forward render about 2% (512 x 512, 64 samples, 200K triangles: 34.3 -> 35.1
 // ms) and saves the backward one a whole render (36.4 -> 1.55 ms).
+// They are the first memory to go: when another allocation of the context fails, when the
+// option is turned off, and when a new problem or a forward that cannot use them leaves
+// most of them idle.
 constexpr size_t kKeptBytes = 8ull << 30;
-static bool keep_records(bc_context* ctx, DiffState& d) {
-  const bc_settings& s = d.st;
-  if (s.integrator != BC_INTEGRATOR_PATH || s.adaptive_sampling || ctx->render_engine == 1) return false;
+
+// Bytes of the records of a forward render, 0: none are kept.
+static size_t kept_bytes(const bc_context* ctx, const bc_settings& s) {
+  if (!ctx->diff_keep_records || s.integrator != BC_INTEGRATOR_PATH || s.adaptive_sampling || ctx->render_engine == 1)
+    return 0;
   const size_t paths = (size_t)s.width * s.height * (size_t)effective_spp(s);
   const size_t bytes = grad_rec_bytes(paths, s.bounces, true);
-  if (paths > (size_t)INT32_MAX || bytes > kKeptBytes) return false;
+  return paths > (size_t)INT32_MAX || bytes > kKeptBytes ? 0 : bytes;
+}
+
+bool release_kept_records(bc_context* ctx) {
+  DiffState* d = ctx->diff;
+  if (!d || d->keeping || !d->d_kept.p) return false;
+  d->kept = false;
+  d->d_kept.release();
+  return true;
+}
+
+static bool keep_records(bc_context* ctx, DiffState& d) {
+  const bc_settings& s = d.st;
+  const size_t paths = (size_t)s.width * s.height * (size_t)effective_spp(s);
+  const size_t bytes = kept_bytes(ctx, s);
+  if (d.d_kept.cap / 2 > bytes) release_kept_records(ctx);
+  if (!bytes) return false;
   if (d.d_kept.cap < bytes) {
     size_t free_bytes = 0, total_bytes = 0;
     if (cudaMemGetInfo(&free_bytes, &total_bytes) || bytes > free_bytes / 4 || d.d_kept.ensure(bytes)) {
@@ -177,7 +199,7 @@ bc_status bc_diff_configure(bc_context* ctx, const bc_diff_desc* desc) {
     pm[k] = m;
     m2p[m] = k;
   }
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   if (!ctx->diff) ctx->diff = new DiffState();
   DiffState& d = *ctx->diff;
   d.configured = false;
@@ -186,6 +208,7 @@ bc_status bc_diff_configure(bc_context* ctx, const bc_diff_desc* desc) {
   const size_t np3 = 3 * (size_t)(na + ne);
   const size_t px3 = 3 * (size_t)s.width * s.height;
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (d.d_kept.cap / 2 > kept_bytes(ctx, s)) release_kept_records(ctx);
   if (!e) e = d.d_param_mat.ensure(pm.size() * sizeof(int32_t));
   if (!e) e = d.d_mat2param.ensure(std::max<size_t>(1, m2p.size()) * sizeof(int32_t));
   if (!e) e = d.d_params.ensure(np3 * sizeof(float));
@@ -211,7 +234,7 @@ bc_status bc_diff_configure(bc_context* ctx, const bc_diff_desc* desc) {
 bc_status bc_diff_set_target(bc_context* ctx, const float* target) {
   if (!ctx || !target) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
   if (!ctx->diff || !ctx->diff->configured) return set_error(ctx, BC_ERR_INVALID_ARG, "bc_diff_configure first");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   DiffState& d = *ctx->diff;
   const size_t bytes = 3 * (size_t)d.st.width * d.st.height * sizeof(float);
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
@@ -227,7 +250,7 @@ bc_status bc_forward(bc_context* ctx, const float* params, uint64_t seed, float*
   if (!ctx->diff || !ctx->diff->configured) return set_error(ctx, BC_ERR_INVALID_ARG, "bc_diff_configure first");
   DiffState& d = *ctx->diff;
   if (loss_out && !d.has_target) return set_error(ctx, BC_ERR_INVALID_ARG, "loss needs a target (bc_diff_set_target)");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   const int np = d.n_alb + d.n_em;
   d.forward_done = false;
   d.kept = false;
@@ -243,9 +266,16 @@ bc_status bc_forward(bc_context* ctx, const float* params, uint64_t seed, float*
   if ((e = cudaGetLastError())) return cuda_status(ctx, e, "parameter update");
   const size_t px = (size_t)d.st.width * d.st.height;
   int64_t rays = 0;
-  const bool keep = keep_records(ctx, d);
+  bool keep = keep_records(ctx, d);
+  d.keeping = keep;
   bc_status st = render_views(ctx, std::vector<ViewRequest>{diff_view(d, seed)}, px, &rays, nullptr,
                               keep ? &d.rec : nullptr);
+  d.keeping = false;
+  if (st == BC_ERR_OOM && keep) {  // the render's own buffers come first
+    keep = false;
+    release_kept_records(ctx);
+    st = render_views(ctx, std::vector<ViewRequest>{diff_view(d, seed)}, px, &rays, nullptr);
+  }
   if (st) return st;
   d.kept = keep;
   d.kept_gen = ctx->scene_gen;
@@ -281,7 +311,7 @@ bc_status bc_backward(bc_context* ctx, const float* dloss_dimage, float* grad_al
   DiffState& d = *ctx->diff;
   if (!dloss_dimage && !d.dimg_from_loss)
     return set_error(ctx, BC_ERR_INVALID_ARG, "no adjoint image: pass dloss_dimage or set a target before bc_forward");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   const size_t px = (size_t)d.st.width * d.st.height;
   const int np = d.n_alb + d.n_em;
   const int np3 = 3 * np;

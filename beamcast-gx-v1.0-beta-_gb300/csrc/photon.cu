@@ -477,7 +477,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
                        ((p2 * 4 + 255) / 256) * 256 + ((np * 8 + 255) / 256) * 256 + ((tsize * 4 + 255) / 256) * 256 +
                        256 + (((size_t)max_cells * 4 + 255) / 256) * 256 + (((size_t)max_cells * 8 + 255) / 256) * 256 +
                        (max_cells ? ((size_t)list_cap * 48 + 255) / 256 * 256 : 0);
-  cudaError_t e = cudaMalloc(&p.mem, bytes);
+  cudaError_t e = device_alloc(&p.mem, bytes);
   if (e) {
     p.mem = nullptr;
     return cuda_status(ctx, e, "photon map");
@@ -650,7 +650,7 @@ extern "C" bc_status bc_photon_map(bc_context* ctx, int32_t scene, const bc_sett
   if (!ctx->has_scene) return set_error(ctx, BC_ERR_NO_SCENE, "no scene uploaded");
   if (scene < 0 || scene >= (int32_t)ctx->ranges.size())
     return set_error(ctx, BC_ERR_INVALID_ARG, "scene outside the resident set");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   PhotonEntry* p = nullptr;
   const unsigned long long* built = nullptr;
   bc_status st = photon_entry(ctx, scene, *settings, photon_clock(ctx), &p, &built);

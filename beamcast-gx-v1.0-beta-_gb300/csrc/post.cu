@@ -496,7 +496,7 @@ extern "C" bc_status bc_post_process(bc_context* ctx, int32_t width, int32_t hei
     return set_error(ctx, BC_ERR_INVALID_ARG, "bad post-process arguments");
   if (settings->denoise && !guide_nd) return set_error(ctx, BC_ERR_INVALID_ARG, "denoise needs guides");
   if ((int64_t)width * height > (1 << 26)) return set_error(ctx, BC_ERR_INVALID_ARG, "frame too large");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   PostTargets t;
   bc_status st = ensure_post_scratch(ctx, width * height, &t);
   if (st) return st;
@@ -952,7 +952,7 @@ extern "C" bc_status bc_post_stack(bc_context* ctx, const bc_post_desc* d, const
   const bool need_guides = d->hbao > 0 || d->hbao_plus > 0 || d->denoise || tw > 0 ||
                            (d->debug_view >= 1 && d->debug_view <= 4);
   if (need_guides && !guides_in) return set_error(ctx, BC_ERR_INVALID_ARG, "these passes need guides");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   cudaStream_t st = ctx->stream;
   const size_t n = (size_t)rw * rh, no = (size_t)W * H;
   const size_t bytes = n * (3 * 12 + 4 * 16 + 48) + no * (2 * 12 + 4) + 64 + 16 * 256;

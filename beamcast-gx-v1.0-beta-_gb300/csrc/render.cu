@@ -2606,7 +2606,7 @@ extern "C" {
 bc_status bc_render_rows(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, int32_t y0,
                          int32_t rows, float* linear_out, uint32_t* guide_out, int64_t* rays_out) {
   if (!ctx || !cam || !settings || !linear_out) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   bc_status st = enqueue_rows(ctx, *cam, *settings, y0, rows, guide_out != nullptr);
   if (st) return st;
   RenderBuffers* rb = ctx->rb;
@@ -2622,7 +2622,7 @@ bc_status bc_render_rows(bc_context* ctx, const bc_camera* cam, const bc_setting
 bc_status bc_render_frame(bc_context* ctx, const bc_camera* cam, const bc_settings* settings, float* linear_out,
                           uint32_t* guide_out, uint32_t* rgba_out, int64_t* rays_out) {
   if (!ctx || !cam || !settings) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   const bool need_guides = settings->denoise || guide_out;
   bc_status st = enqueue_rows(ctx, *cam, *settings, 0, settings->height, need_guides);
   if (st) return st;
@@ -2649,7 +2649,7 @@ bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_sett
                             float* meansq_out, int64_t* rays_out) {
   if (!ctx || !cam || !settings || !mean_out || !meansq_out)
     return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   if (!ctx->rb) ctx->rb = new RenderBuffers();
   ctx->rb->want_sumsq = true;
   bc_status st = enqueue_rows(ctx, *cam, *settings, 0, settings->height, false);
@@ -2667,7 +2667,7 @@ bc_status bc_render_moments(bc_context* ctx, const bc_camera* cam, const bc_sett
 bc_status bc_render_batch(bc_context* ctx, const bc_view* views, int32_t n_views, float* const* linear_out,
                           int64_t* rays_out) {
   if (!ctx || !views || n_views < 1) return set_error(ctx, BC_ERR_INVALID_ARG, "NULL argument or no views");
-  cudaSetDevice(ctx->device);
+  use_context(ctx);
   std::vector<ViewRequest> req;
   long long px = 0;
   bc_status bst = batch_requests(ctx, views, n_views, &req, &px);

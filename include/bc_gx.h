@@ -339,7 +339,9 @@ bc_status bc_diff_set_target(bc_context* ctx, const float* target);
  * image_out (may be NULL): width*height RGB mean radiance. loss_out (may be
  * NULL; needs a target): the L2 loss. The context keeps the paths' vertex
  * records on the device for bc_backward: 20 bytes per path and bounce and 20
- * per path, up to 8 GB and a quarter of the free memory; freed with the context.
+ * per path, up to 8 GB and a quarter of the free memory. They are given back when
+ * another allocation of the context would fail, when a smaller problem is
+ * configured, with the option "diff_keep_records" 0, and with the context.
  */
 bc_status bc_forward(bc_context* ctx, const float* params, uint64_t seed, float* image_out, double* loss_out);
 /*
@@ -447,6 +449,9 @@ bc_status bc_post_process_noalloc(int32_t width, int32_t height, const float* d_
  *                        Morton code on a 64^3 grid over the scene bounds, then
  *                        direction octant); results are returned in the caller's
  *                        order either way.
+ *   "diff_keep_records"  1 (default): bc_forward keeps vertex records for bc_backward;
+ *                        0: it keeps none (2% faster, for forward-only loops), and
+ *                        bc_backward traces the paths again.
  *   "photon_grid"        1 (default): a photon gather reads its cell's neighbour
  *                        list, built with the map; 0: 27 hash lookups.
  *                        Both give the same photons in the same order.

@@ -245,3 +245,63 @@ def test_backward_after_another_upload_replays(ctx, problem):
             ctx.backward(w)
     finally:
         ctx.reset_cancel()
+
+
+@pytest.fixture()
+def fresh(native_lib, problem):
+    """A context of its own: every buffer of a call's first use is a new allocation."""
+    c = bcgx.Context(0)
+    c.upload(scenes.to_scene(problem.spec))
+    c.diff_configure(problem.cam, problem.settings, problem.albedo_materials, problem.emission_materials)
+    yield c
+    c.close()
+
+
+def test_kept_records_give_way_to_other_allocations(fresh, problem):
+    """The hook fails the context's next device allocations. Kept records are given back
+    and the allocation tried again; the gradient then comes from a replay."""
+    w = np.random.default_rng(5).uniform(-1, 1, (problem.settings.height, problem.settings.width, 3)).astype(np.float32)
+    fresh.forward(problem.init_params, SEED, want_image=False)
+    kept = np.concatenate(fresh.backward(w))
+    rays = scenes.random_rays(1000, seed=3)
+    fresh.set_option("test_fail_allocs", 1)
+    fresh.raycast(rays)
+    replayed = np.concatenate(fresh.backward(w))
+    assert np.abs(replayed - kept).max() <= 1e-6 * np.abs(kept).max()
+    fresh.set_option("test_fail_allocs", 1)  # nothing is left to give back
+    with pytest.raises(bcgx.BCError, match="OOM"):
+        fresh.raycast(np.concatenate([rays] * 80))
+    fresh.raycast(rays)
+
+
+def test_forward_renders_without_records_where_both_do_not_fit(fresh, problem):
+    fresh.set_option("render_wave_cap", 4096)
+    want, _ = fresh.forward(problem.init_params, SEED)
+    fresh.set_option("render_wave_cap", 1 << 26)
+    fresh.set_option("test_fail_allocs", 1)  # the larger wave's path buffers
+    got, _ = fresh.forward(problem.init_params, SEED)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("by", ["option", "configure"])
+def test_records_can_be_declined_and_are_given_back(fresh, problem, by):
+    torch = pytest.importorskip("torch")
+    st = problem.settings.copy()
+    st.width, st.height = 8 * st.width, 4 * st.height
+    fresh.diff_configure(problem.cam, st, problem.albedo_materials, problem.emission_materials)
+    held = st.width * st.height * st.spp * 20 * (st.bounces + 1)  # 220 MB
+    fresh.forward(problem.init_params, SEED, want_image=False)
+    w = np.ones((st.height, st.width, 3), np.float32)
+    kept = np.concatenate(fresh.backward(w))
+    before = torch.cuda.mem_get_info()[0]
+    if by == "option":
+        fresh.set_option("diff_keep_records", 0)
+        assert torch.cuda.mem_get_info()[0] >= before + 0.9 * held
+        fresh.forward(problem.init_params, SEED, want_image=False)
+        assert fresh.get_option("diff_keep_records") == 0
+        assert torch.cuda.mem_get_info()[0] >= before + 0.9 * held
+        replayed = np.concatenate(fresh.backward(w))
+        assert np.abs(replayed - kept).max() <= 1e-6 * np.abs(kept).max()
+    else:
+        fresh.diff_configure(problem.cam, problem.settings, problem.albedo_materials, problem.emission_materials)
+        assert torch.cuda.mem_get_info()[0] >= before + 0.9 * held
