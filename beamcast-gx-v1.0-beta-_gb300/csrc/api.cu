@@ -390,7 +390,7 @@ bc_status bc_raycast_device(bc_context* ctx, const float* d_rays, int64_t n, flo
   use_context(ctx);
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   void* order = nullptr;
-  if (ctx->raycast_sort && n >= kMinOrderedRays && n < (int64_t(1) << 31)) {
+  if (ctx->raycast_sort && n >= min_ordered_rays(ctx->ds) && n < (int64_t(1) << 31)) {
     cudaError_t e = ctx->d_order[2].ensure(ray_order_bytes(n));
     if (e) return cuda_status(ctx, e, "ray order buffers");
     order = ctx->d_order[2].p;
@@ -427,7 +427,7 @@ bc_status bc_raycast(bc_context* ctx, const float* rays, int64_t n, float* t_out
   const int64_t chunk = ctx->raycast_chunk;
   cudaStream_t streams[2] = {ctx->stream, ctx->aux_stream};
   void* order[2] = {nullptr, nullptr};
-  if (ctx->raycast_sort && n >= kMinOrderedRays)
+  if (ctx->raycast_sort && n >= min_ordered_rays(ctx->ds))
     for (int k = 0; k < 2; k++) {
       if ((e = ctx->d_order[k].ensure(ray_order_bytes(std::min(chunk, n))))) return cuda_status(ctx, e, "ray order buffers");
       order[k] = ctx->d_order[k].p;
@@ -472,7 +472,7 @@ bc_status bc_occluded_device(bc_context* ctx, const float* d_rays, int64_t n, ui
     cudaError_t e = ctx->d_rec_any.ensure(any_record_bytes(n));
     if (e) return cuda_status(ctx, e, "any-hit record buffers");
     rec = ctx->d_rec_any.p;
-    if (ctx->raycast_sort && n >= kMinOrderedRays && n < (int64_t(1) << 31)) {
+    if (ctx->raycast_sort && n >= min_ordered_rays(ctx->ds) && n < (int64_t(1) << 31)) {
       if ((e = ctx->d_order[2].ensure(ray_order_bytes(n)))) return cuda_status(ctx, e, "ray order buffers");
       order = ctx->d_order[2].p;
     }
@@ -503,7 +503,7 @@ bc_status bc_occluded(bc_context* ctx, const float* rays, int64_t n, uint8_t* ou
   if (ctx->raycast_split && !cast_in_groups(ctx->ds, n, true)) {
     if ((e = ctx->d_rec_any.ensure(any_record_bytes(n)))) return cuda_status(ctx, e, "any-hit record buffers");
     rec = ctx->d_rec_any.p;
-    if (ctx->raycast_sort && n >= kMinOrderedRays && n < (int64_t(1) << 31)) {
+    if (ctx->raycast_sort && n >= min_ordered_rays(ctx->ds) && n < (int64_t(1) << 31)) {
       if ((e = ctx->d_order[2].ensure(ray_order_bytes(n)))) return cuda_status(ctx, e, "ray order buffers");
       order = ctx->d_order[2].p;
     }

@@ -31,10 +31,10 @@ int stack_variant(int need);
 // Exact closest hit over n rays (8 floats each); see bc_raycast in bc_gx.h.
 // `work` is an 8-byte device counter private to this launch's stream (persistent kernels).
 // order_scratch (ray_order_bytes(n) bytes, or NULL): rays are traced in a
-// spatially coherent order (batches of at least kMinOrderedRays rays).
+// spatially coherent order (batches of at least min_ordered_rays(s) rays).
 // rec_scratch (exact_record_bytes(n) bytes, or NULL): the exact closest hit of
 // a triangle-only scene runs as separate walk and fp64 settlement passes.
-constexpr int64_t kMinOrderedRays = 1 << 20;
+int64_t min_ordered_rays(const DeviceScene& s);
 // Small batches of a triangle-only scene are cast by groups of eight lanes in
 // one launch without scratch, where `split` (bc_set_option "raycast_split") allows.
 constexpr int64_t kGroupRaysClosest = 32768, kGroupRaysAny = 65536;

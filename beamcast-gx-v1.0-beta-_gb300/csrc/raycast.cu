@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(128) k_closest_fast_persistent(SceneView sv, c
 }
 
 // ---- ray order -------------------------------------------------------------------
-// Batches of at least kMinOrderedRays rays that come in no order of their own
+// Batches of at least min_ordered_rays rays that come in no order of their own
 // (k_ray_probe) are traced in the order of a 21-bit key: the Morton code of the origin
 // on a 64^3 grid over the scene bounds, then the direction octant, so a warp's
 // rays start near each other and head the same way (fewer divergent node
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(kScanBlock) k_ray_probe(const float4* __restri
                                                           int32_t* __restrict__ flag) {
   reinterpret_cast<int4*>(bins)[blockIdx.x * kScanBlock + threadIdx.x] = make_int4(0, 0, 0, 0);
   if (blockIdx.x != 0) return;
-  const int64_t i = (n - 1) / kScanBlock * threadIdx.x;  // n >= kMinOrderedRays: i + 1 < n
+  const int64_t i = (n - 1) / kScanBlock * threadIdx.x;  // n >= 2 kScanBlock: i + 1 < n
   const uint3 p = ray_cell(__ldg(rays + 2 * i), lo, scale), q = ray_cell(__ldg(rays + 2 * i + 2), lo, scale);
   const bool apart = abs((int)p.x - (int)q.x) > 1 || abs((int)p.y - (int)q.y) > 1 || abs((int)p.z - (int)q.z) > 1;
   const int count = __syncthreads_count(apart);
@@ -1353,14 +1353,24 @@ size_t ray_order_bytes(int64_t n) {
   return (size_t)kKeyBins * 4 + (size_t)(kKeyBins / kScanBlock) * 4 + (size_t)n * 8 + 5 * 256;
 }
 
+// The least batch that is ordered. Ordering is worth more in a scene that caches hold
+// less of: rays with random origins, us per closest-hit call as they come / ordered, at
+// 262,144 / 524,288 / 786,432 / 1,048,575 rays: 200,000 triangles 702 / 724, 1041 / 1071,
+// 1367 / 1398, 1712 / 1743; 500,000: 787 / 824, 1180 / 1190, 1549 / 1556, 1926 / 1913;
+// 1,000,000: 814 / 826, 1220 / 1232, 1663 / 1606, 2016 / 1970; 2,000,000: 866 / 966,
+// 1287 / 1279, 1768 / 1691, 2171 / 2074. A batch that the probe finds in an order of its own
+// pays 30 us for the five launches (786,432 camera rays, 1,000,000 triangles: 740 -> 770;
+// ordered they would take 1,860).
+int64_t min_ordered_rays(const DeviceScene& s) { return s.n_prims >= 3 << 18 ? 5 << 17 : 1 << 20; }
+
 // Spatially coherent ray order (see k_ray_keys) into order_scratch; *perm is
 // left NULL when the batch is not ordered (no scratch, fewer than
-// kMinOrderedRays rays, 2^31 rays or more: the order holds 32-bit indices, or a
+// min_ordered_rays rays, 2^31 rays or more: the order holds 32-bit indices, or a
 // scene with spheres, whose kernels read rays in order).
 static cudaError_t order_rays(const DeviceScene& s, const float4* rays, int64_t n, void* order_scratch,
                               const int32_t** perm, cudaStream_t st) {
   *perm = nullptr;
-  if (!order_scratch || n < kMinOrderedRays || n >= (int64_t(1) << 31) || s.has_spheres) return cudaSuccess;
+  if (!order_scratch || n < min_ordered_rays(s) || n >= (int64_t(1) << 31) || s.has_spheres) return cudaSuccess;
   char* q = (char*)order_scratch;
   int32_t* bins = (int32_t*)q;
   int32_t* totals = (int32_t*)(q + (size_t)kKeyBins * 4);

@@ -444,8 +444,9 @@ bc_status bc_post_process_noalloc(int32_t width, int32_t height, const float* d_
  *   "raycast_exact"      1 (default): bc_raycast is exact as documented there;
  *                        0: plain fp32 closest hit, t = the fp32 distance, with no
  *                        exactness contract near edges and ties.
- *   "raycast_sort"       1 (default): batches of at least 1,048,576 rays that come
- *                        in no spatial order of their own are traced in one (origin
+ *   "raycast_sort"       1 (default): batches of at least 1,048,576 rays (655,360 in
+ *                        a scene of 786,432 primitives or more) that come in no
+ *                        spatial order of their own are traced in one (origin
  *                        Morton code on a 64^3 grid over the scene bounds, then
  *                        direction octant); results are returned in the caller's
  *                        order either way.

@@ -429,3 +429,19 @@ def test_sphere_direction_lengths_parity(gpu_ctx, orc, length):
     _check(gpu_ctx, ref, rays)
     occ_ref, _ = ref.occluded_f32(rays)
     assert occ_ref.any() and np.array_equal(gpu_ctx.occluded(rays), occ_ref)
+
+
+@pytest.mark.parametrize("n", [655_359, 655_360, 655_437])
+def test_ray_order_of_large_scenes_changes_no_result(gpu_ctx, n):
+    """Scenes of 786,432 primitives and more order their rays from 655,360 on."""
+    gpu_ctx.upload(scenes.to_scene(scenes.random_triangles(786_432, seed=scenes.SEED_TRIS + 11)))
+    rays = scenes.random_rays(n, seed=24)
+    t1, p1 = gpu_ctx.raycast(rays)
+    o1 = gpu_ctx.occluded(rays)
+    try:
+        gpu_ctx.set_option("raycast_sort", 0)
+        t0, p0 = gpu_ctx.raycast(rays)
+        o0 = gpu_ctx.occluded(rays)
+    finally:
+        gpu_ctx.set_option("raycast_sort", 1)
+    assert np.array_equal(p0, p1) and np.array_equal(t0, t1) and np.array_equal(o0, o1)
