@@ -123,7 +123,7 @@ struct bc_context {
   bc_timing last_timing{};              // bc_last_timing
   struct DiffState* diff = nullptr;  // differentiable rendering (diff.cu)
   struct PhotonCache* photons = nullptr;  // photon maps of the photon-mapping integrator (photon.cu)
-  int photon_grid = 1;                    // gathers read the neighbour lists (bc_set_option "photon_grid")
+  int photon_grid = 1;                    // gathers read cell runs and neighbour lists (bc_set_option "photon_grid")
   uint64_t scene_gen = 0;                 // bumped by every scene or geometry upload
   // rendering state (render.cu)
   struct RenderBuffers* rb = nullptr;

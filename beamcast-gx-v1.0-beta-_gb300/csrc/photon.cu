@@ -349,8 +349,8 @@ __global__ void k_photon_runs(PhotonView pm, const PhotonGrid* __restrict__ grid
   }
 }
 
-__global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, const int* __restrict__ runs,
-                               int2* __restrict__ list, float4* __restrict__ lent, int cap) {
+__global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, int2* __restrict__ list,
+                               float4* __restrict__ lent, int cap) {
   const int gx = grid->dim[0];
   if (gx == 0) return;
   const int gy = grid->dim[1], gz = grid->dim[2];
@@ -363,7 +363,7 @@ __global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, con
     }
     int n = 0;
     for (int c = 0; c < 27; c++) {
-      const int u = runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
+      const int u = pm.runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
       if (u >= 0) n += pm.span[u].y;
     }
     int at = 0;
@@ -374,7 +374,7 @@ __global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, con
     list[i] = make_int2(at, n);
     if (at < 0) continue;
     for (int c = 0; c < 27 && n > 0; c++) {
-      const int u = runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
+      const int u = pm.runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
       if (u < 0) continue;
       const int2 sp = pm.span[u];
       for (int k = sp.x; k < sp.x + sp.y; k++) {
@@ -399,6 +399,12 @@ struct PhotonEntry {
   int* header = nullptr;
   unsigned long long* rays = nullptr;
   const float4 *pos_u = nullptr, *nrm_u = nullptr, *flux_u = nullptr;
+  bcgx::PhotonGrid* grid = nullptr;  // with lists to build: their box,
+  long long cells = 0;               // its largest size in cells,
+  int list_cap = 0;                  // and their entries
+  void* lists = nullptr;             // memory of the lists: the end of `mem`, or
+  bool lists_apart = false;          // an allocation of their own
+  bool used = false;                 // by an earlier render call
   bcgx::PhotonView view{};
 };
 
@@ -413,7 +419,9 @@ constexpr size_t kPhotonCacheEntries = 16;
 
 static void free_entry(PhotonEntry& p) {
   if (p.mem) cudaFree(p.mem);
-  p.mem = nullptr;
+  if (p.lists_apart) cudaFree(p.lists);
+  p.mem = p.lists = nullptr;
+  p.lists_apart = false;
 }
 
 void destroy_photon_state(bc_context* ctx) {
@@ -446,8 +454,22 @@ static cudaError_t trace_pass(bc_context* ctx, const PhotonTraceArgs& a) {
   return sph ? launch_trace<256, true>(a, ctx->d_status, st) : launch_trace<256, false>(a, ctx->d_status, st);
 }
 
-// Builds the map of `scene` for (seed, level, max_bounces) into a new entry.
-static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, PhotonEntry* out) {
+// Neighbour lists cost a launch, 1.5 KB of memory a photon and 8 bytes a cell. A level-1
+// map (512 photons: 27 run lookups find little to read) gets them for a render of
+// kListPaths paths or more, or once the map is used again; others get them for their
+// first render. Level 1, a new map every frame, without / with lists: 96 x 54, 1 sample 414
+// / 421 us, 384 x 216, 2 samples 439 / 462, 640 x 360, 4 samples 558 / 598, 960 x 540, 8
+// samples 1,467 / 1,337; level 2: 555 / 445, 588 / 525, 702 / 675, 1,719 / 1,436.
+constexpr long long kListPaths = 1 << 20;
+static bool wants_lists(int level, long long paths) { return level > 1 || paths >= kListPaths; }
+static size_t list_index_bytes(long long cells) { return ((size_t)cells * sizeof(int2) + 255) / 256 * 256; }
+static size_t list_bytes(long long cells, int entries) {
+  return list_index_bytes(cells) + 3 * (size_t)entries * sizeof(float4);
+}
+
+// Builds the map of `scene` for (seed, level, max_bounces) into a new entry, with room
+// for its neighbour lists where `lists`.
+static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, bool lists, PhotonEntry* out) {
   const SceneRange& sr = ctx->ranges[scene];
   PhotonEntry& p = *out;
   p.gen = ctx->scene_gen;
@@ -470,14 +492,18 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   int p2max = 2;
   while (p2max < p.np) p2max <<= 1;
   const int tsize = 2 * p2max;
-  const int list_cap = photon_list_entries(s);
   const size_t a = (size_t)p.attempts, np = (size_t)p.np, p2 = (size_t)p2max;
-  const size_t bytes = 4 * 256 + ((a * 4 + 255) / 256) * 256 * 2 + ((np * 16 + 255) / 256) * 256 * 6 +
-                       ((np * 8 + 255) / 256) * 256 * 2 + ((p2 * 8 + 255) / 256) * 256 +
-                       ((p2 * 4 + 255) / 256) * 256 + ((np * 8 + 255) / 256) * 256 + ((tsize * 4 + 255) / 256) * 256 +
-                       256 + (((size_t)max_cells * 4 + 255) / 256) * 256 + (((size_t)max_cells * 8 + 255) / 256) * 256 +
-                       (max_cells ? ((size_t)list_cap * 48 + 255) / 256 * 256 : 0);
-  cudaError_t e = device_alloc(&p.mem, bytes);
+  const size_t map_bytes = 4 * 256 + ((a * 4 + 255) / 256) * 256 * 2 + ((np * 16 + 255) / 256) * 256 * 6 +
+                           ((np * 8 + 255) / 256) * 256 * 2 + ((p2 * 8 + 255) / 256) * 256 +
+                           ((p2 * 4 + 255) / 256) * 256 + ((np * 8 + 255) / 256) * 256 +
+                           ((tsize * 4 + 255) / 256) * 256 + 256 + (((size_t)max_cells * 4 + 255) / 256) * 256;
+  lists = lists && max_cells > 0;
+  cudaError_t e = device_alloc(&p.mem, map_bytes + (lists ? list_bytes(max_cells, photon_list_entries(s)) : 0));
+  if (e == cudaErrorMemoryAllocation && lists) {
+    cudaGetLastError();
+    lists = false;
+    e = device_alloc(&p.mem, map_bytes);
+  }
   if (e) {
     p.mem = nullptr;
     return cuda_status(ctx, e, "photon map");
@@ -501,8 +527,7 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   int* table = take<int>(c, tsize);
   PhotonGrid* grid = take<PhotonGrid>(c, 1);
   int* runs = max_cells ? take<int>(c, (size_t)max_cells) : nullptr;
-  int2* list = max_cells ? take<int2>(c, (size_t)max_cells) : nullptr;
-  float4* lent = max_cells ? take<float4>(c, 3 * (size_t)list_cap) : nullptr;
+  if (lists) p.lists = c;
   p.pos_u = pos_u;
   p.nrm_u = nrm_u;
   p.flux_u = flux_u;
@@ -543,25 +568,6 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
                                       flux, table, tsize, (float)radius, max_cells, grid, ctx->d_status);
     e = cudaGetLastError();
   }
-  PhotonView hv{};
-  hv.pos = pos;
-  hv.nrm = nrm;
-  hv.flux = flux;
-  hv.ukey = ukey;
-  hv.span = span;
-  hv.table = table;
-  hv.mask = tsize - 1;
-  if (!e && list) {
-    const int blocks = (int)std::min<long long>(1024, (max_cells + 255) / 256);
-    k_photon_runs<<<blocks, 256, 0, st>>>(hv, grid, runs);
-    k_photon_lists<<<(int)std::min<long long>(4096, (max_cells + 63) / 64), 64, 0, st>>>(hv, grid, runs, list, lent,
-                                                                                        list_cap);
-    e = cudaGetLastError();
-  }
-  if (e) {
-    free_entry(p);
-    return cuda_status(ctx, e, "photon map build");
-  }
   p.view.pos = pos;
   p.view.nrm = nrm;
   p.view.flux = flux;
@@ -572,19 +578,53 @@ static bc_status build_entry(bc_context* ctx, int scene, const bc_settings& s, P
   p.view.cell = (float)radius;
   p.view.r2 = (float)(radius * radius);
   p.view.pir2 = (float)(M_PI * radius * radius);
-  p.view.grid = list ? grid : nullptr;
+  if (!e && runs) {
+    p.grid = grid;
+    p.cells = max_cells;
+    p.list_cap = photon_list_entries(s);
+    p.view.grid = grid;
+    p.view.runs = runs;
+    k_photon_runs<<<(int)std::min<long long>(1024, (max_cells + 255) / 256), 256, 0, st>>>(p.view, grid, runs);
+    e = cudaGetLastError();
+  }
+  if (e) {
+    free_entry(p);
+    return cuda_status(ctx, e, "photon map build");
+  }
+  return BC_OK;
+}
+
+// The neighbour lists of a map that a render of `paths` paths is about to gather from,
+// where it wants them (wants_lists). Where there is no memory for them the render does
+// without.
+static cudaError_t build_lists(bc_context* ctx, PhotonEntry& p, long long paths) {
+  const bool wanted = p.used || wants_lists(p.level, paths);
+  p.used = true;
+  if (!wanted || !p.grid || p.view.list) return cudaSuccess;
+  if (!p.lists) {
+    if (device_alloc(&p.lists, list_bytes(p.cells, p.list_cap))) {
+      cudaGetLastError();
+      p.lists = nullptr;
+      return cudaSuccess;
+    }
+    p.lists_apart = true;
+  }
+  int2* list = static_cast<int2*>(p.lists);
+  float4* lent = reinterpret_cast<float4*>(static_cast<char*>(p.lists) + list_index_bytes(p.cells));
+  k_photon_lists<<<(int)std::min<long long>(4096, (p.cells + 63) / 64), 64, 0, ctx->stream>>>(p.view, p.grid, list,
+                                                                                             lent, p.list_cap);
   p.view.list = list;
   p.view.lent = lent;
-  return BC_OK;
+  return cudaGetLastError();
 }
 
 uint64_t photon_clock(bc_context* ctx) { return ctx->photons ? ctx->photons->clock : 0; }
 
 // The cached map for (scene, seed, PhotonMapping level, max(2, bounces)) or a
-// newly built one; *built_rays is the new map's device ray counter, or null.
+// newly built one (with room for lists where `lists`); *built_rays is the new map's device ray counter, or null.
 // Maps used after the clock read `pin` (by views of the same render) stay.
-static bc_status photon_entry(bc_context* ctx, int scene, const bc_settings& s, uint64_t pin, PhotonEntry** out,
-                              const unsigned long long** built_rays) {
+static bc_status photon_entry(bc_context* ctx, int scene, const bc_settings& s, uint64_t pin, bool lists,
+                              PhotonEntry** out, const unsigned long long** built_rays) {
   if (!ctx->photons) ctx->photons = new PhotonCache();
   PhotonCache& c = *ctx->photons;
   if (built_rays) *built_rays = nullptr;
@@ -617,7 +657,7 @@ static bc_status photon_entry(bc_context* ctx, int scene, const bc_settings& s, 
     }
   }
   PhotonEntry p;
-  bc_status st = build_entry(ctx, scene, s, &p);
+  bc_status st = build_entry(ctx, scene, s, lists, &p);
   if (st) return st;
   p.stamp = ++c.clock;
   c.e.push_back(p);
@@ -626,14 +666,20 @@ static bc_status photon_entry(bc_context* ctx, int scene, const bc_settings& s, 
   return BC_OK;
 }
 
-bc_status photon_map_for(bc_context* ctx, int scene, const bc_settings& s, uint64_t pin, PhotonView* view,
-                         const unsigned long long** built_rays) {
+bc_status photon_map_for(bc_context* ctx, int scene, const bc_settings& s, uint64_t pin, long long paths,
+                         PhotonView* view, const unsigned long long** built_rays) {
   PhotonEntry* p = nullptr;
-  bc_status st = photon_entry(ctx, scene, s, pin, &p, built_rays);
+  bc_status st = photon_entry(ctx, scene, s, pin, ctx->photon_grid && wants_lists(s.photon_mapping, paths), &p,
+                              built_rays);
   if (st) return st;
+  if (ctx->photon_grid) {
+    const cudaError_t e = build_lists(ctx, *p, paths);
+    if (e) return cuda_status(ctx, e, "photon neighbour lists");
+  }
   *view = p->view;  // an empty map has a null table
   if (!ctx->photon_grid) {
     view->grid = nullptr;
+    view->runs = nullptr;
     view->list = nullptr;
   }
   return BC_OK;
@@ -653,7 +699,7 @@ extern "C" bc_status bc_photon_map(bc_context* ctx, int32_t scene, const bc_sett
   use_context(ctx);
   PhotonEntry* p = nullptr;
   const unsigned long long* built = nullptr;
-  bc_status st = photon_entry(ctx, scene, *settings, photon_clock(ctx), &p, &built);
+  bc_status st = photon_entry(ctx, scene, *settings, photon_clock(ctx), false, &p, &built);
   if (st) return st;
   int header[2] = {0, 0};
   unsigned long long rays = 0;

@@ -17,10 +17,10 @@ namespace bcgx {
 constexpr uint64_t kPhotonStream = 0xFFFFFFFFull;  // sample index of the photon emission streams
 constexpr int kGatherMax = 64;                      // tracePhotonMapped gathers at most 64 photons
 
-// Box of a photon map's neighbour lists, written on the device with the map:
+// Box of a photon map's cell runs and neighbour lists, written on the device with the map:
 // the photons' cells and two more on each side, [g0, g0 + dim), so the 27
 // neighbours of every cell within one cell of a photon's are in it;
-// dim[0] == 0: no lists (the hash lookup serves).
+// dim[0] == 0: neither (the hash lookup serves).
 struct PhotonGrid {
   long long g0[3];
   int dim[3];
@@ -36,7 +36,8 @@ struct PhotonView {
   const int* table;                 // 0: empty slot, else distinct-key index + 1; null: empty map
   int mask;                         // table size - 1
   float cell, r2, pir2;             // cell size (= radius), radius^2, pi radius^2
-  const PhotonGrid* grid;           // null: no neighbour lists
+  const PhotonGrid* grid;           // null: no runs and no neighbour lists
+  const int* runs;                  // per cell of the box: the run its key's lookup gives, -1: none
   const int2* list;                 // per cell of the box: (first entry, entries); first < 0: none, use the hash
   const float4* lent;               // list entries, three float4 each: (position, normal x) (normal y z, flux x y) (flux z)
 };
@@ -80,15 +81,16 @@ __device__ __forceinline__ bool gather_photon(float r2, float3 P, float3 N, floa
 // of the cells is visited twice, as the reference's map lookups do.
 // A cell's neighbour list holds exactly those photons in exactly that order, so
 // a gather is one lookup (gather_run) and one contiguous run (gather_sum) whose
-// loads do not depend on what the candidates before them gave.
+// loads do not depend on what the candidates before them gave. Without lists the cells'
+// runs are read in their box (27 loads), and looked up in the hash outside of it.
 
 // The run of p's cell: (first entry, entries), entries 0 where the gather is
-// zero; first < 0: no list, the hash serves. A point more than one cell outside
+// zero; first < 0: no list, the cells' runs serve. A point more than one cell outside
 // the photons' cells has no photon within the radius (cells are one radius
 // wide), so its gather is zero, as the loop would find.
 __device__ __forceinline__ int2 gather_run(const PhotonView& pm, float3 p) {
   if (!pm.table) return make_int2(0, 0);
-  const PhotonGrid* G = pm.list ? pm.grid : nullptr;
+  const PhotonGrid* G = pm.grid;
   const int gx = G ? __ldg(&G->dim[0]) : 0;
   if (gx == 0) return make_int2(-1, 0);
   const int gy = __ldg(&G->dim[1]), gz = __ldg(&G->dim[2]);
@@ -96,7 +98,7 @@ __device__ __forceinline__ int2 gather_run(const PhotonView& pm, float3 p) {
   const long long ly = (long long)floorf(p.y / pm.cell) - __ldg(&G->g0[1]);
   const long long lz = (long long)floorf(p.z / pm.cell) - __ldg(&G->g0[2]);
   if (lx < 1 || ly < 1 || lz < 1 || lx > gx - 2 || ly > gy - 2 || lz > gz - 2) return make_int2(0, 0);
-  return __ldg(pm.list + (lz * gy + ly) * (long long)gx + lx);
+  return pm.list ? __ldg(pm.list + (lz * gy + ly) * (long long)gx + lx) : make_int2(-1, 0);
 }
 
 __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, float3 p, float3 n) {
@@ -117,11 +119,17 @@ __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, flo
     const long long cx = (long long)floorf(p.x / pm.cell);
     const long long cy = (long long)floorf(p.y / pm.cell);
     const long long cz = (long long)floorf(p.z / pm.cell);
+    // gather_run has found the cell at least one inside the box
+    const PhotonGrid* G = pm.grid;
+    const int gx = G ? __ldg(&G->dim[0]) : 0, gy = gx ? __ldg(&G->dim[1]) : 0;
+    const int* runs = nullptr;
+    if (gx) runs = pm.runs + ((cz - __ldg(&G->g0[2])) * gy + cy - __ldg(&G->g0[1])) * (long long)gx + cx - __ldg(&G->g0[0]);
     bool full = false;
     for (int dz = -1; dz <= 1 && !full; dz++)
       for (int dy = -1; dy <= 1 && !full; dy++)
         for (int dx = -1; dx <= 1 && !full; dx++) {
-          const int u = photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
+          const int u = runs ? __ldg(runs + (dz * gy + dy) * (long long)gx + dx)
+                             : photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
           if (u < 0) continue;
           const int2 sp = __ldg(pm.span + u);
           for (int i = sp.x; i < sp.x + sp.y && !full; i++) {

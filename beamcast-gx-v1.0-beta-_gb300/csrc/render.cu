@@ -2294,7 +2294,7 @@ static bc_status queue_views(bc_context* ctx, const std::vector<ViewRequest>& re
     if (V.integrator == BC_INTEGRATOR_RECURSIVE) rec_bounces = std::max(rec_bounces, V.bounces);
     if (V.integrator == BC_INTEGRATOR_PHOTON) {  // built once per frame (renderer.go:2728-2734), then cached
       const unsigned long long* built = nullptr;
-      if ((bst = photon_map_for(ctx, r.scene, r.s, photon_pin, &V.pm, &built))) return bst;
+      if ((bst = photon_map_for(ctx, r.scene, r.s, photon_pin, (long long)V.npix * V.spp, &V.pm, &built))) return bst;
       if (built) photon_rays.push_back(built);
       photon_entries = std::max(photon_entries, photon_list_entries(r.s));
     }

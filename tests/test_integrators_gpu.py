@@ -273,3 +273,42 @@ def test_dense_photon_table_equals_hash_lookups(gpu_ctx):
         finally:
             gpu_ctx.set_option("photon_grid", 1)
         assert np.array_equal(dense, hashed), level
+
+
+@pytest.mark.parametrize("level", [1, 3])
+def test_photon_gathers_agree_with_and_without_lists(native_lib, level):
+    """A map's first small render at level 1 reads the runs of 27 cells, later ones and large
+    ones the neighbour lists; a context whose lists find no memory stays with the runs."""
+    spec, cam = scenes.cornell_reference_scene()
+    st = bcgx.quality("Draft")
+    st.width, st.height, st.spp, st.bounces, st.seed = 160, 90, 2, 4, 31
+    st.integrator, st.photon_mapping = bcgx.INTEGRATOR_PHOTON, level
+    st.denoise, st.bloom, st.adaptive_sampling = False, 0, False
+    large = st.copy()
+    large.width, large.height, large.spp = 1280, 720, 2  # 1.8M paths
+
+    def images(fails):
+        ctx = bcgx.Context(0)
+        try:
+            ctx.upload(scenes.to_scene(spec))
+            ctx.photon_map(st)  # a map without room for lists
+            out = []
+            for s in (st, st, large):
+                ctx.render_frame(cam, st if s is st else large, want_guides=False)  # buffers of that size
+                ctx.upload(scenes.to_scene(spec))
+                ctx.photon_map(s)
+                ctx.set_option("test_fail_allocs", 1 if fails else 0)
+                out.append(ctx.render_frame(cam, s, want_guides=False)["linear"])
+                out.append(ctx.render_frame(cam, s, want_guides=False)["linear"])
+                ctx.set_option("test_fail_allocs", 0)
+                ctx.set_option("photon_grid", 0)
+                out.append(ctx.render_frame(cam, s, want_guides=False)["linear"])
+                ctx.set_option("photon_grid", 1)
+            return out
+        finally:
+            ctx.close()
+
+    with_lists, without = images(False), images(True)
+    for k in range(0, 9, 3):
+        for a in (*with_lists[k:k + 3], *without[k:k + 3]):
+            assert np.array_equal(a, with_lists[k])
