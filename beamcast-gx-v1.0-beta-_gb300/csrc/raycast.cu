@@ -75,8 +75,8 @@ __device__ __forceinline__ const int32_t* walk_order(const int32_t* perm);
 // warp's lanes are idle (one atomic per warp for all of them), so the warp does
 // not idle until its slowest ray ends. The exact kernel parks each finished ray's contenders in a
 // per-warp queue in shared memory; when 32 are parked, the warp settles them
-// in fp64 with every lane active. Triangle-only scenes (spheres settle at
-// once and use the kernels above).
+// in fp64 with every lane active. Triangle-only scenes: the settlement here runs the
+// triangles' test alone (spheres use the kernels above).
 constexpr int kParkTie = 0x100;  // npend flag: the walk already compared two equal fp64 distances
 
 struct ParkQueue {
@@ -992,7 +992,8 @@ __global__ void __launch_bounds__(128) k_tie_replay(SceneView sv, const BinNode*
 // the visited node and a lane per triangle of a leaf; the stack lies in shared
 // memory, contenders in the lanes' registers, and the same kernel settles them in
 // fp64 (and replays exact ties), so a call is one launch. 1,000 rays against
-// 20,000 triangles, among other calls: 118 -> 31 us.
+// 20,000 triangles, among other calls: 118 -> 31 us. Bound by latency: 18% of the issue
+// slots, 6% of the warps resident, three waiting cycles on a load per instruction.
 // A lane holds at most one contender: a primitive that may be the closest hit,
 // with the lower end of its distance interval. `hi` is the least upper end of
 // the certain ones; contenders beyond it are dropped. When more than eight
@@ -1404,7 +1405,13 @@ bool cast_in_groups(const DeviceScene& s, int64_t n, bool any) {
 
 // Groups per warp: one while the warps fit the chip a few times, then two, then
 // four; and past 8,192 rays 64 registers (spilling a little) for eight blocks per SM
-// instead of four without spills.
+// instead of four without spills. us per call, closest hit, 20,000 triangles, at 1,000 /
+// 4,000 / 6,000 / 8,000 / 16,000 / 32,000 rays: one group a warp at four blocks 33 / 48 /
+// 54 / 63 / 105 / 192, two 45 / 47 / 56 / 63 / 96 / 163, four 49 / 54 / 60 / 58 / 87 / 145;
+// at eight blocks one 43 / 49 / 55 / 63 / 95 / 163, two 62 / 64 / 61 / 63 / 92 / 144, four
+// 66 / 72 / 78 / 77 / 88 / 136. The lines lie by these; over 1,000,000 triangles one group
+// at four blocks leads longer: 96 / 104 / 123 / 147 / 233 / 403, four 118 / 141 / 123 / 166 /
+// 189 / 309, four at eight blocks 159 / 192 / 164 / 227 / 197 / 304.
 template <bool ANY>
 static cudaError_t cast_groups(const DeviceScene& s, const float4* rays, int64_t n, float* t, int32_t* p, uint8_t* occ,
                                unsigned* status, cudaStream_t st) {

@@ -84,7 +84,12 @@ struct RecurRec {
 // k_gather adds their photon radiance. Sorted by the photon run, the lanes of a
 // warp read the same candidates.
 constexpr int kGatherBins = 1 << 16, kGatherScan = 1024;  // bins, bins per scan block
-constexpr int kGatherSortPaths = 1 << 20;  // waves of at least this many paths sort their gathers
+// Waves of at least this many paths sort their gathers. Cornell-like room, 8 bounces, device
+// time sorted / unsorted: level 3 720 / 690 us at 0.92M paths, 768 / 729 at 1.04M, 1,029 / 1,054
+// at 2.1M, 1,580 / 1,765 at 4.1M, 4,310 / 5,240 at 14.7M; level 1 (few photons to share)
+// 650 / 599, 689 / 626, 908 / 853, 1,358 / 1,369, 3,870 / 3,980; level 4 980 / 909, 1,040 / 943,
+// 1,330 / 1,292, 1,858 / 2,050, 4,720 / 5,800.
+constexpr int kGatherSortPaths = 1 << 20;
 struct GatherSoA {
   float4* p;       // by queue position: point, first list entry
   float4* n;       // facing normal, list entries
@@ -466,7 +471,8 @@ __device__ __forceinline__ void extend_body(SceneView sv, const ViewGPU* __restr
 // tests are, and where its answer could hang on its order or on the rounding of a box
 // face (the two nearest hits within kFlatTie; a hit, or the ray's origin, as near to a
 // face as the slab test may place it wrongly; a ray of extreme size), the walk is asked,
-// by about one ray in a thousand. Bound by the issue of the tests. Per frame, walk against
+// by about one ray in a thousand. Bound by the issue of the tests (69% of the slots, 20 of
+// 32 lanes active; the short launches of late bounces by latency). Per frame, walk against
 // flat: 9 primitives, 960 x 540: extend 350 -> 234 us, connect 137 -> 105 us; 1280 x 720:
 // 1,042 -> 659 and 292 -> 239 us; random triangles, 640 x 360, 16 samples: 4 of them 189
 // -> 111 us, 16: 212 -> 179, 24: 248 -> 229, 32: 271 -> 294; spheres 16: 221 -> 169, 32:
@@ -1170,7 +1176,8 @@ __global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_bod
 // waits for the block's longest run on the first bounce, and later bounces run
 // 7 of 32 lanes, each on its own candidates. Here the vertices are listed,
 // counting-sorted by their run (k_gather_count, k_gather_scan, k_gather_scatter)
-// and gathered with the lanes of a warp on the same run.
+// and gathered with the lanes of a warp on the same run (26 of 32 lanes active; bound by
+// the latency of the candidates' loads, issue 36%, L1 50%).
 __global__ void __launch_bounds__(256) k_gather_count(GatherSoA ga, const WaveCounters* cnt) {
   const int n = cnt->gather;
   const int lane = threadIdx.x & 31;

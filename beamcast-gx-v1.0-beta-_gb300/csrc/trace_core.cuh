@@ -565,9 +565,9 @@ __device__ __forceinline__ void walk(const SceneView& sv, const Ray32& r, Leaf& 
 // hit more than one child, the sorting network and the pushes have nothing to
 // do: the single hit child (if any) is picked with selects; when none hit more
 // than four, they are ordered with five comparisons instead of the network.
-template <int STACK, class W>
-__device__ __forceinline__ uint32_t order_children(float nr[8], uint32_t ch[8], uint2* st, int& sp, float tlim,
-                                                   unsigned* status, W& walker) {
+template <class W>
+__device__ __forceinline__ uint32_t order_children(float nr[8], uint32_t ch[8], float tlim, unsigned* status,
+                                                   W& walker) {
   const float kInf = __int_as_float(0x7f800000);
   int hits = 0;
 #pragma unroll
@@ -682,7 +682,7 @@ struct Walker {
       float nr[8];
       uint32_t ch[8];
       node_children_fused<true>(sv.nodes + ref, rp, r.tmin, leaf.tlim, nr, ch);
-      ref = order_children<STACK>(nr, ch, st, sp, leaf.tlim, status, *this);
+      ref = order_children(nr, ch, leaf.tlim, status, *this);
       if (ref != kEnd && (ref & kLeafBit)) {
         if (pending != 0) break;
         pending = ref;
@@ -742,7 +742,7 @@ struct FastWalker {
       float nr[8];
       uint32_t ch[8];
       node_children_fused<false>(sv.nodes + ref, rp, r.tmin, leaf.tlim, nr, ch);
-      ref = order_children<STACK>(nr, ch, st, sp, leaf.tlim, status, *this);
+      ref = order_children(nr, ch, leaf.tlim, status, *this);
       if (ref != kEnd && (ref & kLeafBit)) {
         if (pending != 0) break;
         pending = ref;
