@@ -513,7 +513,7 @@ __device__ __forceinline__ float largest_of(float x, float y, float z) {
 __device__ __forceinline__ bool flat_ray(const Ray32& r, float* face, float* inv_len) {
   const float o = largest_of(r.ox, r.oy, r.oz), d = largest_of(r.dx, r.dy, r.dz);
   *face += kFlatRound * o;
-  *inv_len = 1.0f / sqrtf(dot3(f3(r.dx, r.dy, r.dz), f3(r.dx, r.dy, r.dz)));
+  *inv_len = rsqrtf(dot3(f3(r.dx, r.dy, r.dz), f3(r.dx, r.dy, r.dz)));
   return o < kFlatLargest && d < kFlatLargest && d > 1.0f / kFlatLargest;  // false for a NaN
 }
 
