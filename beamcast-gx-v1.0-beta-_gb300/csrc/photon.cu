@@ -332,12 +332,8 @@ __global__ void __launch_bounds__(1024) k_photon_grid(const int* __restrict__ he
 
 namespace bcgx {
 
-// The neighbour lists, a thread per cell of the box: the photons of the 27
-// cells around it, each cell's run looked up in the hash table exactly as a
-// gather would look it up, in the gather's order. `runs` holds the lookups (run
-// index or -1, written by k_photon_runs). A cell whose list would not fit in
-// the remaining entries gets none, and gathers there use the hash. Every photon
-// is in the lists of at most 27 cells (more only where cell keys collide).
+// The run of every cell of the box (run index or -1), looked up in the hash table exactly
+// as a gather would look it up.
 __global__ void k_photon_runs(PhotonView pm, const PhotonGrid* __restrict__ grid, int* __restrict__ runs) {
   const int gx = grid->dim[0];
   if (gx == 0) return;
@@ -349,41 +345,70 @@ __global__ void k_photon_runs(PhotonView pm, const PhotonGrid* __restrict__ grid
   }
 }
 
-__global__ void k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid, int2* __restrict__ list,
-                               float4* __restrict__ lent, int cap) {
+// The neighbour lists: the photons of the 27 cells around each cell, in the gather's order.
+// A cell with more than kLongRun photons around it, or whose list would not fit in the
+// remaining entries, gets none, and gathers there read the runs. Every photon is in the
+// lists of at most 27 cells, of more where cell keys collide (they do for cells mirrored
+// about the origin). A warp counts 32 cells, one a lane, and then copies them one after the
+// other with all its lanes.
+__global__ void __launch_bounds__(64) k_photon_lists(PhotonView pm, PhotonGrid* __restrict__ grid,
+                                                     int2* __restrict__ list, float4* __restrict__ lent, int cap) {
+  __shared__ int first[2][28], from[2][27];  // of the 27 runs: entries before each, first photon
   const int gx = grid->dim[0];
   if (gx == 0) return;
   const int gy = grid->dim[1], gz = grid->dim[2];
   const long long total = (long long)gx * gy * gz;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % gx), y = (int)((i / gx) % gy), z = (int)(i / ((long long)gx * gy));
-    if (x < 1 || y < 1 || z < 1 || x > gx - 2 || y > gy - 2 || z > gz - 2) {
-      list[i] = make_int2(-1, 0);  // a gather there is zero without a lookup
-      continue;
-    }
-    int n = 0;
-    for (int c = 0; c < 27; c++) {
-      const int u = pm.runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
-      if (u >= 0) n += pm.span[u].y;
-    }
-    int at = 0;
-    if (n > 0) {
-      at = atomicAdd(&grid->used, n);
-      if (at < 0 || at > cap - n) at = -1;
-    }
-    list[i] = make_int2(at, n);
-    if (at < 0) continue;
-    for (int c = 0; c < 27 && n > 0; c++) {
-      const int u = pm.runs[i + ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1];
-      if (u < 0) continue;
-      const int2 sp = pm.span[u];
-      for (int k = sp.x; k < sp.x + sp.y; k++) {
-        const float4 P = pm.pos[k], N = pm.nrm[k], F = pm.flux[k];
-        float4* e = lent + 3 * (size_t)at++;
-        e[0] = make_float4(P.x, P.y, P.z, N.x);
-        e[1] = make_float4(N.y, N.z, F.x, F.y);
-        e[2] = make_float4(F.z, 0.0f, 0.0f, 0.0f);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const auto neighbour = [&](int c) { return ((c / 9 - 1) * (long long)gy + (c / 3) % 3 - 1) * gx + c % 3 - 1; };
+  for (long long base = ((long long)blockIdx.x * 2 + w) * 32; base < total; base += (long long)gridDim.x * 64) {
+    const long long i = base + lane;
+    int n = 0, at = -1;
+    if (i < total) {
+      const int x = (int)(i % gx), y = (int)((i / gx) % gy), z = (int)(i / ((long long)gx * gy));
+      if (!(x < 1 || y < 1 || z < 1 || x > gx - 2 || y > gy - 2 || z > gz - 2)) {  // outside a gather is zero without a lookup
+        for (int c = 0; c < 27; c++) {
+          const int u = __ldg(pm.runs + i + neighbour(c));
+          if (u >= 0) n += __ldg(pm.span + u).y;
+        }
+        at = n > kLongRun ? -1 : 0;
+        if (n > 0 && at == 0) {
+          at = atomicAdd(&grid->used, n);
+          if (at < 0 || at > cap - n) at = -1;
+        }
       }
+      list[i] = make_int2(at, n);
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, at >= 0 && n > 0); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const int entries = __shfl_sync(0xffffffffu, n, l);
+      float4* out = lent + 3 * (size_t)__shfl_sync(0xffffffffu, at, l);
+      const int u = lane < 27 ? __ldg(pm.runs + base + l + neighbour(lane)) : -1;
+      const int2 sp = u >= 0 ? __ldg(pm.span + u) : make_int2(0, 0);
+      int upto = sp.y;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (lane < 27) {
+        first[w][lane + 1] = upto;
+        from[w][lane] = sp.x;
+      }
+      if (lane == 0) first[w][0] = 0;
+      __syncwarp();
+      for (int j = lane; j < entries; j += 32) {
+        int lo = 0, hi = 26;  // the last run that starts at or before entry j
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (first[w][mid] <= j) lo = mid;
+          else hi = mid - 1;
+        }
+        const int k = from[w][lo] + j - first[w][lo];
+        const float4 P = __ldg(pm.pos + k), N = __ldg(pm.nrm + k), F = __ldg(pm.flux + k);
+        out[3 * (size_t)j] = make_float4(P.x, P.y, P.z, N.x);
+        out[3 * (size_t)j + 1] = make_float4(N.y, N.z, F.x, F.y);
+        out[3 * (size_t)j + 2] = make_float4(F.z, 0.0f, 0.0f, 0.0f);
+      }
+      __syncwarp();
     }
   }
 }
@@ -457,8 +482,8 @@ static cudaError_t trace_pass(bc_context* ctx, const PhotonTraceArgs& a) {
 // Neighbour lists cost a launch, 1.5 KB of memory a photon and 8 bytes a cell. A level-1
 // map (512 photons: 27 run lookups find little to read) gets them for a render of
 // kListPaths paths or more, or once the map is used again; others get them for their
-// first render. Level 1, a new map every frame, without / with lists: 96 x 54, 1 sample 414
-// / 421 us, 384 x 216, 2 samples 439 / 462, 640 x 360, 4 samples 558 / 598, 960 x 540, 8
+// first render. Level 1, a new map every frame, without / with lists: 96 x 54, 1 sample 404
+// / 421 us, 384 x 216, 2 samples 436 / 462, 640 x 360, 4 samples 600 / 598, 960 x 540, 8
 // samples 1,467 / 1,337; level 2: 555 / 445, 588 / 525, 702 / 675, 1,719 / 1,436.
 constexpr long long kListPaths = 1 << 20;
 static bool wants_lists(int level, long long paths) { return level > 1 || paths >= kListPaths; }

@@ -65,13 +65,18 @@ __device__ __forceinline__ int photon_cell_lookup(const PhotonView& pm, unsigned
 }
 
 // One candidate of a gather (renderer.go:1745-1752): counted when it is within
-// the radius of p and faces n; true once kGatherMax photons are counted.
-__device__ __forceinline__ bool gather_photon(float r2, float3 P, float3 N, float3 F, float3 p, float3 n, float3& sum,
-                                              int& count) {
+// the radius of p and faces n (then *nd is its cosine).
+__device__ __forceinline__ bool photon_counts(float r2, float3 P, float3 N, float3 p, float3 n, float* nd) {
   const float3 d = P - p;
   if (dot3(d, d) > r2) return false;
-  const float nd = dot3(N, n);
-  if (nd <= 0.05f) return false;
+  *nd = dot3(N, n);
+  return !(*nd <= 0.05f);
+}
+// The same with its flux; true once kGatherMax photons are counted.
+__device__ __forceinline__ bool gather_photon(float r2, float3 P, float3 N, float3 F, float3 p, float3 n, float3& sum,
+                                              int& count) {
+  float nd;
+  if (!photon_counts(r2, P, N, p, n, &nd)) return false;
   sum = fma3(F, nd, sum);
   return ++count >= kGatherMax;
 }
@@ -81,8 +86,14 @@ __device__ __forceinline__ bool gather_photon(float r2, float3 P, float3 N, floa
 // of the cells is visited twice, as the reference's map lookups do.
 // A cell's neighbour list holds exactly those photons in exactly that order, so
 // a gather is one lookup (gather_run) and one contiguous run (gather_sum) whose
-// loads do not depend on what the candidates before them gave. Without lists the cells'
-// runs are read in their box (27 loads), and looked up in the hash outside of it.
+// loads do not depend on what the candidates before them gave. A cell without a list is
+// gathered from the 27 runs, found with 27 loads in the lists' box and in the hash outside
+// of it: in a map without lists, or with more than kLongRun candidates around it. Thousands
+// lie around a few cells where a scene is much larger than its lit part; most of them are
+// turned down for their normals, and the copies would not fit. Analytic spheres on a ground
+// sphere of radius 1,000 (the gathers of 155 x 495, 3 samples, 14 bounces; 8,192 photons): 25.0
+// ms from lists, where they found room, 12.7 ms from runs; 2,048 photons: 3.7 ms and 4.5.
+constexpr int kLongRun = 2048;
 
 // The run of p's cell: (first entry, entries), entries 0 where the gather is
 // zero; first < 0: no list, the cells' runs serve. A point more than one cell outside
@@ -101,10 +112,56 @@ __device__ __forceinline__ int2 gather_run(const PhotonView& pm, float3 p) {
   return pm.list ? __ldg(pm.list + (lz * gy + ly) * (long long)gx + lx) : make_int2(-1, 0);
 }
 
+// The candidates of p's 27 cells from their runs, or from hash lookups outside of the
+// runs' box: kAhead candidates' positions and normals in flight, flux for those that count.
+// Bound by the latency of these loads: the scene above 23.1 ms with one, 16.7 with two, 12.7
+// with four. Out of line: its registers stay out of gather_sum's loop.
+constexpr int kAhead = 4;
+static __device__ __noinline__ float3 gather_cells(const PhotonView& pm, float3 p, float3 n, int& count) {
+  const long long cx = (long long)floorf(p.x / pm.cell);
+  const long long cy = (long long)floorf(p.y / pm.cell);
+  const long long cz = (long long)floorf(p.z / pm.cell);
+  // gather_run has found the cell at least one inside the box
+  const PhotonGrid* G = pm.grid;
+  const int gx = G ? __ldg(&G->dim[0]) : 0, gy = gx ? __ldg(&G->dim[1]) : 0;
+  const int* runs = nullptr;
+  if (gx) runs = pm.runs + ((cz - __ldg(&G->g0[2])) * gy + cy - __ldg(&G->g0[1])) * (long long)gx + cx - __ldg(&G->g0[0]);
+  const float r2 = pm.r2;
+  float3 sum = f3(0.0f, 0.0f, 0.0f);
+  for (int dz = -1; dz <= 1; dz++)
+    for (int dy = -1; dy <= 1; dy++)
+      for (int dx = -1; dx <= 1; dx++) {
+        const int u = runs ? __ldg(runs + (dz * gy + dy) * (long long)gx + dx)
+                           : photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
+        if (u < 0) continue;
+        const int2 sp = __ldg(pm.span + u);
+        const int end = sp.x + sp.y;
+        for (int i = sp.x; i < end; i += kAhead) {
+          float4 P[kAhead], N[kAhead];
+#pragma unroll
+          for (int k = 0; k < kAhead; k++) {
+            P[k] = __ldg(pm.pos + min(i + k, end - 1));
+            N[k] = __ldg(pm.nrm + min(i + k, end - 1));
+          }
+#pragma unroll
+          for (int k = 0; k < kAhead; k++) {
+            float nd;
+            if (i + k >= end || !photon_counts(r2, f3(P[k].x, P[k].y, P[k].z), f3(N[k].x, N[k].y, N[k].z), p, n, &nd)) continue;
+            const float4 F = __ldg(pm.flux + i + k);
+            sum = fma3(f3(F.x, F.y, F.z), nd, sum);
+            if (++count >= kGatherMax) return sum;
+          }
+        }
+      }
+  return sum;
+}
+
 __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, float3 p, float3 n) {
   float3 sum = f3(0.0f, 0.0f, 0.0f);
   int count = 0;
-  if (run.x >= 0) {
+  if (run.x < 0) {
+    sum = gather_cells(pm, p, n, count);
+  } else {
     const float4* e = pm.lent + 3 * (size_t)run.x;
     for (int i = 0; i < run.y; i += 2) {  // two candidates in flight; the last pair may read the last entry twice
       const float4* e1 = e + 3 * (size_t)min(i + 1, run.y - 1);
@@ -115,28 +172,6 @@ __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, flo
           gather_photon(pm.r2, f3(b0.x, b0.y, b0.z), f3(b0.w, b1.x, b1.y), f3(b1.z, b1.w, b2.x), p, n, sum, count))
         break;
     }
-  } else {
-    const long long cx = (long long)floorf(p.x / pm.cell);
-    const long long cy = (long long)floorf(p.y / pm.cell);
-    const long long cz = (long long)floorf(p.z / pm.cell);
-    // gather_run has found the cell at least one inside the box
-    const PhotonGrid* G = pm.grid;
-    const int gx = G ? __ldg(&G->dim[0]) : 0, gy = gx ? __ldg(&G->dim[1]) : 0;
-    const int* runs = nullptr;
-    if (gx) runs = pm.runs + ((cz - __ldg(&G->g0[2])) * gy + cy - __ldg(&G->g0[1])) * (long long)gx + cx - __ldg(&G->g0[0]);
-    bool full = false;
-    for (int dz = -1; dz <= 1 && !full; dz++)
-      for (int dy = -1; dy <= 1 && !full; dy++)
-        for (int dx = -1; dx <= 1 && !full; dx++) {
-          const int u = runs ? __ldg(runs + (dz * gy + dy) * (long long)gx + dx)
-                             : photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
-          if (u < 0) continue;
-          const int2 sp = __ldg(pm.span + u);
-          for (int i = sp.x; i < sp.x + sp.y && !full; i++) {
-            const float4 P = __ldg(pm.pos + i), N = __ldg(pm.nrm + i), F = __ldg(pm.flux + i);
-            full = gather_photon(pm.r2, f3(P.x, P.y, P.z), f3(N.x, N.y, N.z), f3(F.x, F.y, F.z), p, n, sum, count);
-          }
-        }
   }
   if (count == 0) return f3(0.0f, 0.0f, 0.0f);
   return sum * (1.0f / (pm.pir2 * (float)count));

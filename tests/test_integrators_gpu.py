@@ -312,3 +312,20 @@ def test_photon_gathers_agree_with_and_without_lists(native_lib, level):
     for k in range(0, 9, 3):
         for a in (*with_lists[k:k + 3], *without[k:k + 3]):
             assert np.array_equal(a, with_lists[k])
+
+
+@pytest.mark.parametrize("level", [2, 3, 4])
+def test_photon_gathers_in_a_scene_larger_than_its_lit_part(gpu_ctx, level):
+    """The showcase's ground sphere is 2,000 wide: all photons lie in a few cells about the
+    origin, whose keys collide with those of cells mirrored there, and cells have thousands
+    of candidates. Lists, runs and hash lookups give the same image."""
+    spec, cam = scenes.showcase_scene()
+    gpu_ctx.upload(scenes.to_scene(spec))
+    st = _settings(PHOTON, w=72, h=40, spp=2, bounces=4, level=level, seed=70 + level)
+    a = gpu_ctx.render_frame(cam, st, want_guides=False, want_rgba=False)["linear"]
+    gpu_ctx.set_option("photon_grid", 0)
+    try:
+        b = gpu_ctx.render_frame(cam, st, want_guides=False, want_rgba=False)["linear"]
+    finally:
+        gpu_ctx.set_option("photon_grid", 1)
+    assert np.array_equal(a, b) and a.max() > 0
