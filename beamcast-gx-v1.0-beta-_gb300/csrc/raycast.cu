@@ -393,7 +393,7 @@ __device__ __forceinline__ double tri_t64(const double* __restrict__ q, D3 o, D3
 // contender need only its distance, the others the full tests (4,194,304 rays
 // against 1,000,000 triangles: 0.74 -> 0.45 ms);
 // each kind is settled 32 at a time. That a certain hit passes its fp64 test is checked
-// on the first 32 distances of every warp and on 32 of each 256 after them; on all of them it
+// on one group of 32 in sixteen (in each warp from another one on); on all of them it
 // costs the ray cast 2% (5.95 -> 6.07 ms).
 __global__ void __launch_bounds__(128) k_exact_settle(SceneView sv, const float4* __restrict__ rays, int64_t n,
                                                       ExactRecords rec, float* __restrict__ t_out,
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(128) k_exact_settle(SceneView sv, const float4
   const int64_t warps = (int64_t)gridDim.x * 4, per = ((n + warps - 1) / warps + 31) / 32 * 32;
   const int64_t first = ((int64_t)blockIdx.x * 4 + w) * per, last = min((int64_t)n, first + per);
   int len[2] = {0, 0};  // warp-uniform
-  unsigned distances = 0;  // groups of 32 settled by their distance
+  unsigned distances = blockIdx.x * 4 + w;  // groups of 32 settled by their distance, from a start of the warp's own
   for (int64_t base = first; base < last || len[0] > 0 || len[1] > 0; base += 32) {
     if (base < last) {
       const int64_t i = base + lane;
@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(128) k_exact_settle(SceneView sv, const float4
         const double tmin = (double)a.w, tmax = (double)b.w;
         double t;
         bool hit = true;
-        if (distances % 8 == 0) hit = tri_hit64(q, o, d, tmin, tmax, &t);
-        if (distances % 8 != 0 || !hit) t = tri_t64(q, o, d);
+        if (distances % 16 == 0) hit = tri_hit64(q, o, d, tmin, tmax, &t);
+        if (distances % 16 != 0 || !hit) t = tri_t64(q, o, d);
         if (!(hit && t >= tmin && t <= tmax)) atomicOr(status, kStatusBound);
         t_out[i] = __double2float_rn(t);
         prim_out[i] = __ldg(sv.slot_prim + slot);
