@@ -1177,7 +1177,7 @@ __global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_bod
 // 7 of 32 lanes, each on its own candidates. Here the vertices are listed,
 // counting-sorted by their run (k_gather_count, k_gather_scan, k_gather_scatter)
 // and gathered with the lanes of a warp on the same run (26 of 32 lanes active; bound by
-// the latency of the candidates' loads, issue 36%, L1 50%).
+// the latency of the candidates' loads: issue 36%, L1 50% at ten blocks an SM).
 __global__ void __launch_bounds__(256) k_gather_count(GatherSoA ga, const WaveCounters* cnt) {
   const int n = cnt->gather;
   const int lane = threadIdx.x & 31;
@@ -1244,7 +1244,13 @@ __global__ void __launch_bounds__(256) k_gather_scatter(GatherSoA ga, const Wave
   }
 }
 
-__global__ void __launch_bounds__(128) k_gather(const ViewGPU* __restrict__ views, PathState ps, GatherSoA ga,
+// Sorted waves take twelve blocks an SM (40 registers, of which the call of gather_cells
+// spills some), smaller ones eight (64): 1280 x 720, 16 samples, 8,192 photons, twelve against
+// eight: frame 4.25 / 4.59 ms; 640 x 360, 4 samples, 512 photons 700 / 598 us; 155 x 495, 3
+// samples of a scene whose gathers are long (see gather_cells) 17.7 / 12.8 ms.
+constexpr int kGatherBlocksSorted = 12, kGatherBlocks = 8;
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB) k_gather(const ViewGPU* __restrict__ views, PathState ps, GatherSoA ga,
                                                 const WaveCounters* cnt, const int32_t* __restrict__ order) {
   const int n = cnt->gather;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -2080,8 +2086,8 @@ static cudaError_t enqueue_wave(bc_context* ctx, const WaveShape& w, const Shade
         k_gather_scan<<<kGatherBins / kGatherScan, kGatherScan / 4, 0, st>>>(rb->ga);
         k_gather_scatter<<<w.acc_grid * 2, 256, 0, st>>>(rb->ga, c);
       }
-      k_gather<<<w.acc_grid * 4, 128, 0, st>>>(rb->views, rb->ps, rb->ga, c,
-                                                  w.gather_sort ? rb->ga.perm : rb->ga.list);
+      const auto gather = w.gather_sort ? k_gather<kGatherBlocksSorted> : k_gather<kGatherBlocks>;
+      gather<<<w.acc_grid * 4, 128, 0, st>>>(rb->views, rb->ps, rb->ga, c, w.gather_sort ? rb->ga.perm : rb->ga.list);
     }
     if (w.lights) rb->mark(st, kTimeConnect);
     if (w.lights && w.flat)
