@@ -113,11 +113,11 @@ __device__ __forceinline__ int2 gather_run(const PhotonView& pm, float3 p) {
 }
 
 // The candidates of p's 27 cells from their runs, or from hash lookups outside of the
-// runs' box: kAhead candidates' positions and normals in flight, flux for those that count.
+// runs' box: AHEAD candidates' positions and normals in flight, flux for those that count.
 // Bound by the latency of these loads: the scene above 23.1 ms with one, 16.7 with two, 12.7
-// with four. Out of line: its registers stay out of gather_sum's loop.
-constexpr int kAhead = 4;
-static __device__ __noinline__ float3 gather_cells(const PhotonView& pm, float3 p, float3 n, int& count) {
+// with four.
+template <int AHEAD>
+__device__ __forceinline__ float3 cells_sum(const PhotonView& pm, float3 p, float3 n, int& count) {
   const long long cx = (long long)floorf(p.x / pm.cell);
   const long long cy = (long long)floorf(p.y / pm.cell);
   const long long cz = (long long)floorf(p.z / pm.cell);
@@ -128,23 +128,26 @@ static __device__ __noinline__ float3 gather_cells(const PhotonView& pm, float3 
   if (gx) runs = pm.runs + ((cz - __ldg(&G->g0[2])) * gy + cy - __ldg(&G->g0[1])) * (long long)gx + cx - __ldg(&G->g0[0]);
   const float r2 = pm.r2;
   float3 sum = f3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1  // 27 copies of the body would not stay in the instruction cache
   for (int dz = -1; dz <= 1; dz++)
+#pragma unroll 1
     for (int dy = -1; dy <= 1; dy++)
+#pragma unroll 1
       for (int dx = -1; dx <= 1; dx++) {
         const int u = runs ? __ldg(runs + (dz * gy + dy) * (long long)gx + dx)
                            : photon_cell_lookup(pm, photon_cell_key(cx + dx, cy + dy, cz + dz));
         if (u < 0) continue;
         const int2 sp = __ldg(pm.span + u);
         const int end = sp.x + sp.y;
-        for (int i = sp.x; i < end; i += kAhead) {
-          float4 P[kAhead], N[kAhead];
+        for (int i = sp.x; i < end; i += AHEAD) {
+          float4 P[AHEAD], N[AHEAD];
 #pragma unroll
-          for (int k = 0; k < kAhead; k++) {
+          for (int k = 0; k < AHEAD; k++) {
             P[k] = __ldg(pm.pos + min(i + k, end - 1));
             N[k] = __ldg(pm.nrm + min(i + k, end - 1));
           }
 #pragma unroll
-          for (int k = 0; k < kAhead; k++) {
+          for (int k = 0; k < AHEAD; k++) {
             float nd;
             if (i + k >= end || !photon_counts(r2, f3(P[k].x, P[k].y, P[k].z), f3(N[k].x, N[k].y, N[k].z), p, n, &nd)) continue;
             const float4 F = __ldg(pm.flux + i + k);
@@ -156,11 +159,18 @@ static __device__ __noinline__ float3 gather_cells(const PhotonView& pm, float3 
   return sum;
 }
 
+// Out of line: its registers stay out of gather_sum's loop.
+static __device__ __noinline__ float3 gather_cells(const PhotonView& pm, float3 p, float3 n, int& count) {
+  return cells_sum<4>(pm, p, n, count);
+}
+
+// INLINE: without a call (the one-kernel form, which would keep its whole state across it).
+template <bool INLINE>
 __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, float3 p, float3 n) {
   float3 sum = f3(0.0f, 0.0f, 0.0f);
   int count = 0;
   if (run.x < 0) {
-    sum = gather_cells(pm, p, n, count);
+    sum = INLINE ? cells_sum<2>(pm, p, n, count) : gather_cells(pm, p, n, count);
   } else {
     const float4* e = pm.lent + 3 * (size_t)run.x;
     for (int i = 0; i < run.y; i += 2) {  // two candidates in flight; the last pair may read the last entry twice
@@ -180,7 +190,7 @@ __device__ __forceinline__ float3 gather_sum(const PhotonView& pm, int2 run, flo
 __device__ __forceinline__ float3 photon_gather(const PhotonView& pm, float3 p, float3 n) {
   const int2 run = gather_run(pm, p);
   if (run.x >= 0 && run.y == 0) return f3(0.0f, 0.0f, 0.0f);
-  return gather_sum(pm, run, p, n);
+  return gather_sum<true>(pm, run, p, n);
 }
 
 // Hit point and facing normal of a closest hit at fp32 distance t: the

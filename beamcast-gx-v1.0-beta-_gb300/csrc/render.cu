@@ -1258,7 +1258,7 @@ __global__ void __launch_bounds__(128, MINB) k_gather(const ViewGPU* __restrict_
     const float4 P = ga.p[i], N = ga.n[i], W = ga.w[i];
     const int path = __float_as_int(W.w);
     const PhotonView& pm = views[__float_as_uint(ps.ray[2 * (size_t)path].w)].pm;
-    const float3 g = gather_sum(pm, make_int2(__float_as_int(P.w), __float_as_int(N.w)), f3(P.x, P.y, P.z),
+    const float3 g = gather_sum<false>(pm, make_int2(__float_as_int(P.w), __float_as_int(N.w)), f3(P.x, P.y, P.z),
                                 f3(N.x, N.y, N.z));
     const float4 L = ps.L[path];
     ps.L[path] = with_bits(fma3(f3(W.x, W.y, W.z), g, f3(L.x, L.y, L.z)), 0u);
