@@ -920,8 +920,13 @@ bc_status build_sah_device(bc_context* ctx, int32_t n, const double* prim_box, c
   // Levels are launched without waiting while a balanced tree would still have
   // tasks, then two at a time: a level without tasks costs four empty launches,
   // a look at the counters a round trip to the host.
-  int cur = 0, levels = 0, look = 1;
-  while ((N >> look) > (size_t)kSmall) look++;
+  // Where the first centroids are all one point the tree may be a leaf: looked at at once
+  // (100,000 equal centroids: 12 empty levels took 85 of 415 us).
+  int cur = 0, levels = 0, balanced = 1;
+  while ((N >> balanced) > (size_t)kSmall) balanced++;
+  bool one_point = true;
+  for (size_t i = 3; i < 3 * std::min<size_t>(N, 64) && one_point; i++) one_point = centroid[i] == centroid[i % 3];
+  int look = one_point ? 1 : balanced;
   for (;;) {
     for (; levels < look; levels++) {
       // chunks of this level: known only on the device; the kernels stride
@@ -942,7 +947,7 @@ bc_status build_sah_device(bc_context* ctx, int32_t n, const double* prim_box, c
     if (e) return cuda_status(ctx, e, "BVH build");
     if (hdr[2 * cur] == 0) break;
     if (levels >= 4096) return set_error(ctx, BC_ERR_CAPACITY, "BVH deeper than 4096 levels: build on the host");
-    look = levels + 2;
+    look = std::max(levels + 2, balanced);
   }
   k_small<<<sms * 8, kThreads, 0, st>>>(a);
   k_sizes<<<sms * 4, 256, 0, st>>>(a);
