@@ -1177,7 +1177,7 @@ __global__ void __launch_bounds__(128, 8) k_shade_128(BC_SHADE_ARGS) { shade_bod
 // 7 of 32 lanes, each on its own candidates. Here the vertices are listed,
 // counting-sorted by their run (k_gather_count, k_gather_scan, k_gather_scatter)
 // and gathered with the lanes of a warp on the same run (26 of 32 lanes active; bound by
-// the latency of the candidates' loads: issue 36%, L1 50% at ten blocks an SM).
+// the latency of the candidates' loads: issue 51%, L1 73%).
 __global__ void __launch_bounds__(256) k_gather_count(GatherSoA ga, const WaveCounters* cnt) {
   const int n = cnt->gather;
   const int lane = threadIdx.x & 31;
