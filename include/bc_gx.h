@@ -455,7 +455,8 @@ bc_status bc_post_process_noalloc(int32_t width, int32_t height, const float* d_
  *                        bc_backward traces the paths again.
  *   "photon_grid"        1 (default): a photon gather reads its cell's neighbour
  *                        list, or (a level-1 map's first render of fewer than 2^20
- *                        paths) the runs of its 27 cells; 0: 27 hash lookups.
+ *                        paths, cells with more than 2,048 candidates) the runs of its
+ *                        27 cells; 0: 27 hash lookups.
  *                        All give the same photons in the same order.
  *   "raycast_chunk"      rays per chunk of bc_raycast (host buffers),
  *                        65,536 .. 2^28 (default 2^21): chunks alternate
